@@ -69,8 +69,9 @@ enum {
     KBWG_FLAG_EXACT_ORDER = 1u << 2, /* fuse without reordering commuting gates: amplitudes then
                                         equal the reference's bit for bit */
     KBWG_FLAG_NO_GRAPHS = 1u << 3,   /* do not replay repeated gate structures from CUDA graphs */
-    KBWG_FLAG_NO_FOLD = 1u << 4      /* do not fold runs of diagonal one-qubit gates on a qubit into one
-                                        (per-gate cost measurements) */
+    KBWG_FLAG_NO_FOLD = 1u << 4      /* apply every gate as given: do not fold runs of diagonal one-qubit gates on a
+                                        qubit into one, nor leave gates' uniform factors to one multiplication at
+                                        the end (per-gate cost measurements; float-float still leaves H's and RZ's) */
 };
 
 /* QuantumExecution::new (src/quantum_execution.rs:53; src/dense.rs:70-89).

@@ -542,8 +542,8 @@ __global__ void __launch_bounds__(AdjKernel<P, K, R>::kThreads, 2)
                     }
                 }
                 using B = typename pick_t<W, uint64_t, uint32_t>::type;
-                tile_gate<P, K, R, B>(g, vp, R0, F, (B)base);
-                tile_gate<P, K, R, B>(g, vl, R0, F, (B)base);
+                tile_gate<P, K, R, B, false>(g, vp, R0, F, (B)base);
+                tile_gate<P, K, R, B, false>(g, vl, R0, F, (B)base);
             }
             g0 = g1;
         }

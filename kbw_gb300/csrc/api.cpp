@@ -53,6 +53,7 @@ GateDesc make_gate_desc(int prec, uint32_t kind, uint32_t target, uint64_t ctrl,
     g.kind = kind;
     g.target = target;
     g.ctrl = ctrl;
+    g.angle = angle;
     if (prec) {  // Dense<f64>
         switch (kind) {
         case G_H: g.c[0] = 0.70710678118654752440; break;

@@ -312,7 +312,7 @@ __global__ void __launch_bounds__(BatchKernel<P, K, R>::kThreads, 2) k_batch_cir
                         for (int j = 0; j < NR; j++) v[j] = tile[F | ((uint32_t)j << R0)];
                     }
                     const uint32_t g1 = bs.stage_end[s];
-                    for (uint32_t gi = g0; gi < g1; gi++) tile_gate<P, K, R, uint64_t>(sg[gi], v, R0, F, base);
+                    for (uint32_t gi = g0; gi < g1; gi++) tile_gate<P, K, R, uint64_t, false>(sg[gi], v, R0, F, base);
                     g0 = g1;
                 }
                 if (in_tile) {

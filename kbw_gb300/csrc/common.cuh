@@ -71,12 +71,15 @@ struct GateDesc {
     uint32_t target; // qubit (global index) or, inside a tile, a local slot
     uint64_t ctrl;   // control mask on the global basis index
     double c[4];     // see make_gate_desc
+    double angle;    // the caller's angle (0 without one)
 };
 
 enum { G_X = 0, G_Y = 1, G_Z = 2, G_H = 3, G_P = 4, G_RX = 5, G_RY = 6, G_RZ = 7 };
-// Internal kinds of the complex128 float-float path (never seen at the ABI):
-// H without its 1/sqrt(2), |1> times i^q (c[0] = q), multiply every amplitude by c[0] + i c[1].
-enum { G_HN = 8, G_PI = 9, G_SCALE = 10 };
+// Internal kinds of the reordering paths (never seen at the ABI): H without its
+// 1/sqrt(2), |1> times i^q (c[0] = q), multiply every amplitude by c[0] + i c[1]
+// (G_SCALER: by the real c[0]), RX and RY without the larger of their
+// coefficients (c[0], c[1]: see pack_rot in sweep.h).
+enum { G_HN = 8, G_PI = 9, G_SCALE = 10, G_SCALER = 11, G_RXD = 12, G_RYD = 13 };
 
 #if defined(__CUDACC__)
 // ---- rounding-exact arithmetic -------------------------------------------
@@ -198,7 +201,8 @@ __device__ __forceinline__ void apply_pair(uint32_t kind, const GateK<T> &k, cx<
 
 // Diagonal gates: each amplitude only picks up a phase.
 __host__ __device__ __forceinline__ bool is_diag_kind(uint32_t kind) {
-    return kind == G_Z || kind == G_P || kind == G_RZ || kind == G_PI || kind == G_SCALE;
+    return kind == G_Z || kind == G_P || kind == G_RZ || kind == G_PI || kind == G_SCALE ||
+           kind == G_SCALER;
 }
 
 // Gates that only change the |1> amplitude of the pair.

@@ -354,7 +354,7 @@ __global__ void __launch_bounds__(HeaKernel<P, K, R>::kThreads, (sizeof(typename
                         __syncthreads();
                     }
                     const uint32_t g1 = stage_end[s];
-                    for (uint32_t gi = g0; gi < g1; gi++) tile_gate<P, K, R>(sg[gi], v, R0, F, 0);
+                    for (uint32_t gi = g0; gi < g1; gi++) tile_gate<P, K, R, uint32_t, false>(sg[gi], v, R0, F, 0);
                     g0 = g1;
                 }
             }
@@ -459,7 +459,7 @@ __global__ void __launch_bounds__(HeaKernel<P, K, R>::kThreads, (sizeof(typename
                             for (int j = 0; j < NR; j++) v[j] = tile[F | ((uint32_t)j << R0)];
                         }
                         const uint32_t g1 = stage_end[s];
-                        for (uint32_t gi = g0; gi < g1; gi++) tile_gate<P, K, R>(sg[gi], v, R0, F, base);
+                        for (uint32_t gi = g0; gi < g1; gi++) tile_gate<P, K, R, uint32_t, false>(sg[gi], v, R0, F, base);
                         g0 = g1;
                     }
                     if (ps == npass - 2) {

@@ -313,7 +313,7 @@ std::string outer_cond(const TileGate &t, bool wide) {
 std::string gate_stmt(const TileGate &t, const char *v, const char *k, const std::string &outer) {
     char buf[512];
     const char *cls = kClassName[t.cls];
-    const int q = (t.cls == TG_PI) ? (int)t.c[0] : 0;
+    const int q = (t.cls == TG_PI) ? (int)t.c[0] : (t.cls == TG_SCALE ? (int)t.sub : 0);
     std::string cond;
     if (t.fneed) cond = fok_of(t);
     if (!outer.empty()) cond = cond.empty() ? outer : cond + " && " + outer;

@@ -21,10 +21,28 @@
 namespace kbwg {
 namespace jit {
 
+// RX/RY with a deferred factor on register bit B.
+template <class P, int R, int B, bool RYG, bool COT>
+__device__ __forceinline__ void rot(typename P::Amp (&v)[1 << R], const typename P::K4 &k) {
+#pragma unroll
+    for (int jj = 0; jj < (1 << (R - 1)); jj++) {
+        const int j0 = ((jj >> B) << (B + 1)) | (jj & ((1 << B) - 1));
+        const int j1 = j0 | (1 << B);
+        if constexpr (RYG) P::template ryd_pair<COT>(k, v[j0], v[j1]);
+        else P::template rxd_pair<COT>(k, v[j0], v[j1]);
+    }
+}
+
 // Non-diagonal gate whose target is register bit B; bit j of JM: register j
 // passes the gate's controls on register bits.
 template <class P, int R, int B, int CLS, uint32_t JM, int SUB>
 __device__ __forceinline__ void reg(typename P::Amp (&v)[1 << R], const typename P::K4 &k) {
+    if constexpr (SUB == 1 && (CLS == TG_RX || CLS == TG_RY)) {  // deferred factor, uncontrolled (pack_rot)
+        // (the form depends on the angle; the vote tells the compiler that the branch is uniform)
+        if (__any_sync(0xffffffffu, P::cot(k))) rot<P, R, B, CLS == TG_RY, true>(v, k);
+        else rot<P, R, B, CLS == TG_RY, false>(v, k);
+        return;
+    }
 #pragma unroll
     for (int jj = 0; jj < (1 << (R - 1)); jj++) {
         const int j0 = ((jj >> B) << (B + 1)) | (jj & ((1 << B) - 1));
@@ -74,6 +92,11 @@ __device__ __forceinline__ void cswap(typename P::Amp (&v)[1 << R], bool c) {
 // thread after the shuffle, so every lane still joins it.
 template <class P, int R, int TB, int CLS, uint32_t CREG, int SUB>
 __device__ __forceinline__ void lane(typename P::Amp (&v)[1 << R], const typename P::K4 &k, bool fok, uint32_t F) {
+    if constexpr (SUB == 1 && (CLS == TG_RX || CLS == TG_RY)) {
+        if (__any_sync(0xffffffffu, P::cot(k))) rot_lane<P, R, CLS == TG_RY, true>(v, k, TB, F);
+        else rot_lane<P, R, CLS == TG_RY, false>(v, k, TB, F);
+        return;
+    }
     const bool one = ((F >> TB) & 1u) != 0u;
 #pragma unroll
     for (int j = 0; j < (1 << R); j++) {
@@ -136,6 +159,8 @@ __device__ __forceinline__ void dfix(typename P::Amp (&v)[1 << R], const typenam
                 v[j] = sel(on, P::neg(v[j]), v[j]);
             } else if constexpr (CLS == TG_PI) {
                 v[j] = sel(on, P::pi_mul(v[j], Q), v[j]);
+            } else if constexpr (CLS == TG_SCALE && Q != 0) {  // real factor
+                v[j] = P::smul(v[j], k.c0);
             } else {  // P (|1> side only) and SCALE
                 v[j] = sel(on, P::cmul(v[j], k.c0, k.c1), v[j]);
             }

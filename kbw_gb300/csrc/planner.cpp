@@ -191,6 +191,9 @@ std::vector<PlannedSweep> plan_sweeps(uint32_t n, int K, int R, const GateDesc *
                 case G_P: t.cls = TG_P; break;
                 case G_RZ: t.cls = TG_RZ; break;
                 case G_PI: t.cls = TG_PI; break;
+                case G_RXD: t.cls = TG_RX; t.sub = 1; break;
+                case G_RYD: t.cls = TG_RY; t.sub = 1; break;
+                case G_SCALER: t.cls = TG_SCALE; t.sub = 1; break;
                 default: t.cls = TG_SCALE; break;
                 }
                 memcpy(t.c, x.c, sizeof t.c);

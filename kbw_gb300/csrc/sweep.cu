@@ -566,51 +566,132 @@ static cudaError_t run_fused_t(Sim &s, const GateDesc *gates, size_t count) {
     else return run_fused_p<Fast<T>, K, R>(s, gates, count);
 }
 
-// Complex128 float-float path: rewrite the queue so that uncontrolled H
-// drops its 1/sqrt(2) and uncontrolled RZ(t) becomes the phase gate
-// diag(1, e^{it}), collecting the dropped factors 2^{-1/2} and e^{-it/2} in
-// one complex scale g, applied as a final gate (and earlier if |g| would
-// leave float range).  P(+-pi/2) and P(pi) become exact multiplications by
-// i^q.  Everything else keeps the binary64 constants of Dense<f64>.
-static std::vector<GateDesc> ff_rewrite(const GateDesc *gates, size_t count) {
+// Rewrite of the queue before planning, in every arithmetic that need not keep
+// the reference's rounding (c64, binary64 and float-float; not in program-order
+// mode): a uniform factor of a gate is left to one final multiplication of
+// the state, collected in the complex scale g.
+//   * uncontrolled H drops its 1/sqrt(2);
+//   * uncontrolled RZ(t) becomes the phase gate diag(1, e^{it}), dropping
+//     e^{-it/2} (its |0> half then costs nothing);
+//   * uncontrolled RX/RY drop the larger of cos and sin of their half angle
+//     (pack_rot): one multiplication per real part instead of two, in
+//     float-float 15 packed operations instead of 19 per amplitude.
+// Each H, RX or RY grows the state by at most sqrt(2), so kDeferRun of them
+// stay inside float's range before g is applied (a structural count: the
+// plan must not depend on the angles).  P(+-pi/2) and P(pi) become exact
+// multiplications by i^q.
+// A SCALE costs about two deferred rotations' savings, so lists with fewer
+// than kDeferMin such gates keep the full forms (float-float always drops H's
+// and RZ's factors: its multiplications cost most).
+// Measured (one GB300, specialised kernels): 25q 8-layer brickwork in binary64
+// 28.6 -> 16.3 ms (FP64-bound: half the products), 28q 20-layer complex64 27.3
+// -> 25.3 ms, 30q float-float 424 -> 395 ms.  Error of a 13q 12-layer
+// brickwork against 80-bit arithmetic: binary64 1.1-1.8e-15 -> 4.9-7.5e-16,
+// float-float 1.4-1.8e-14 -> 1.2-1.4e-14, complex64 6.9-8.6e-7 -> 2.3-2.7e-7.
+// Constants are recomputed in binary64 from the angles, also for complex64
+// (whose program-order constants are rounded like Dense<f32>'s); the deferred
+// factor is that of the coefficient as rounded to the program's type, so
+// each gate with its share of g is a rotation to binary64 accuracy.
+constexpr int kDeferRun = 192, kDeferMin = 3;
+
+template <class T>
+static double packed_value(double x) {  // x as the program's constants hold it
+    if constexpr (std::is_same<T, float>::value) return (double)(float)x;
+    if constexpr (std::is_same<T, ff::f2>::value) {
+        const ff::f2 v = ff::split_constant(x);
+        return (double)v.h + (double)v.l;
+    }
+    return x;
+}
+
+// The collected factor as an unevaluated sum of two doubles per part: a product
+// of a few hundred factors rounded once, at the end (in plain binary64 its
+// own rounding would be larger than the gates').
+struct Dd {
+    double h = 0.0, l = 0.0;
+};
+static Dd dd_mul(Dd a, Dd b) {
+    const double p = a.h * b.h, e = fma(a.h, b.h, -p) + (a.h * b.l + a.l * b.h), s = p + e;
+    return Dd{s, e - (s - p)};
+}
+static Dd dd_add(Dd a, Dd b) {
+    const double s = a.h + b.h, bb = s - a.h, e = ((a.h - (s - bb)) + (b.h - bb)) + (a.l + b.l), r = s + e;
+    return Dd{r, e - (r - s)};
+}
+// 1 / sqrt(1 + w^2) for |w| <= 1: the rounded value and one Newton step's correction
+static Dd dd_unit(double w) {
+    const double w2 = w * w, w2e = fma(w, w, -w2), sh = 1.0 + w2, sl = (w2 - (sh - 1.0)) + w2e;
+    const double r = 1.0 / sqrt(sh), r2 = r * r, r2e = fma(r, r, -r2);
+    const double e = fma(-r2, sh, 1.0) - (r2 * sl + r2e * sh);
+    return Dd{r, 0.5 * r * e};
+}
+
+template <class T>
+static std::vector<GateDesc> defer_scale(const GateDesc *gates, size_t count, bool rotations) {
+    constexpr bool kFF = std::is_same<T, ff::f2>::value;
     std::vector<GateDesc> out;
     out.reserve(count + 2);
-    double gr = 1.0, gi = 0.0;
+    size_t rots = 0, any = 0;
+    for (size_t i = 0; i < count; i++) {
+        if (gates[i].ctrl) continue;
+        if (gates[i].kind == G_RX || gates[i].kind == G_RY) rots++;
+        if (gates[i].kind == G_H || gates[i].kind == G_RZ) any++;
+    }
+    const bool defer = kFF || rots + any >= (size_t)kDeferMin;  // H and RZ
+    const bool drot = rotations && (rots >= (size_t)kDeferMin || (defer && any > 0));
+    Dd gr{1.0, 0.0}, gi;
+    bool complex_g = false, pending = false;
     int unscaled = 0;
+    auto scale_by = [&](Dd f) {
+        gr = dd_mul(gr, f);
+        gi = dd_mul(gi, f);
+        pending = true;
+    };
     auto emit_scale = [&]() {
         GateDesc sc;
         memset(&sc, 0, sizeof sc);
-        sc.kind = G_SCALE;
+        sc.kind = complex_g ? G_SCALE : G_SCALER;
         sc.target = 0;
-        sc.c[0] = gr;
-        sc.c[1] = gi;
+        sc.c[0] = gr.h;
+        sc.c[1] = gi.h;
         out.push_back(sc);
-        gr = 1.0;
-        gi = 0.0;
+        gr = Dd{1.0, 0.0};
+        gi = Dd();
+        complex_g = pending = false;
         unscaled = 0;
     };
     for (size_t i = 0; i < count; i++) {
         GateDesc x = gates[i];
-        if (x.kind == G_H && x.ctrl == 0) {
+        bool grew = false;
+        if (defer && x.kind == G_H && x.ctrl == 0) {
             x.kind = G_HN;
-            gr *= 0.70710678118654752440;
-            gi *= 0.70710678118654752440;
-            if (++unscaled >= 100) {
-                out.push_back(x);
-                emit_scale();
-                continue;
-            }
-        } else if (x.kind == G_RZ && x.ctrl == 0) {
+            scale_by(dd_unit(1.0));
+            grew = true;
+        } else if (defer && x.kind == G_RZ && x.ctrl == 0) {
             // diag(u0, u1) = u0 diag(1, u1 conj(u0)) for unit u0 (for RZ(t):
             // u1 conj(u0) = e^{it}; also a folded general diagonal)
-            const double c = x.c[2] * x.c[0] + x.c[3] * x.c[1], sn = x.c[3] * x.c[0] - x.c[2] * x.c[1];
-            const double nr = gr * x.c[0] - gi * x.c[1], ni = gr * x.c[1] + gi * x.c[0];
+            const Dd ur{x.c[0], 0.0}, ui{x.c[1], 0.0}, nui{-x.c[1], 0.0}, vr{x.c[2], 0.0}, vi{x.c[3], 0.0};
+            const double c = dd_add(dd_mul(vr, ur), dd_mul(vi, ui)).h, sn = dd_add(dd_mul(vi, ur), dd_mul(vr, nui)).h;
+            const Dd nr = dd_add(dd_mul(gr, ur), dd_mul(gi, nui));
+            gi = dd_add(dd_mul(gr, ui), dd_mul(gi, ur));
             gr = nr;
-            gi = ni;
+            complex_g = pending = true;
             x.kind = G_P;
             x.c[0] = c;
             x.c[1] = sn;
             x.c[2] = x.c[3] = 0.0;
+        } else if (drot && (x.kind == G_RX || x.kind == G_RY) && x.ctrl == 0) {
+            const double c = x.c[0], sn = x.c[1];
+            const bool cot = !(fabs(c) >= fabs(sn));
+            const double w = packed_value<T>(cot ? c / sn : sn / c);
+            // the factor that makes (1, w) a unit vector, with the dropped coefficient's sign
+            Dd f = dd_unit(w);
+            if ((cot ? sn : c) < 0.0) f = Dd{-f.h, -f.l};
+            scale_by(f);
+            x.kind = x.kind == G_RX ? G_RXD : G_RYD;
+            x.c[0] = w;
+            x.c[1] = cot ? 1.0 : 0.0;
+            grew = true;
         }
         if (x.kind == G_P) {
             const double c = x.c[0], sn = x.c[1], t = 1e-15;
@@ -625,9 +706,30 @@ static std::vector<GateDesc> ff_rewrite(const GateDesc *gates, size_t count) {
             }
         }
         out.push_back(x);
+        if (grew && ++unscaled >= kDeferRun) emit_scale();
     }
-    if (gr != 1.0 || gi != 0.0) emit_scale();
+    if (pending) emit_scale();
     return out;
+}
+
+// The gate list as the fused sweeps of a handle run it (folded, factors
+// deferred); the handle's state is at least one tile.
+static std::vector<GateDesc> rewritten(const Sim &s, const GateDesc *gates, size_t count) {
+    if (s.flags & KBWG_FLAG_EXACT_ORDER) return std::vector<GateDesc>(gates, gates + count);
+    if (s.flags & KBWG_FLAG_NO_FOLD) {  // every gate applied as given, but for float-float's H and RZ
+        if (ff_capable(s)) return defer_scale<ff::f2>(gates, count, false);
+        return std::vector<GateDesc>(gates, gates + count);
+    }
+    std::vector<GateDesc> r;
+    if (!s.prec) {  // complex64: constants in binary64 from the angles
+        r.assign(gates, gates + count);
+        for (GateDesc &x : r)
+            if (x.kind <= G_RZ) x = make_gate_desc(1, x.kind, x.target, x.ctrl, x.angle);
+        gates = r.data();
+    }
+    const std::vector<GateDesc> f = fold_diagonals(gates, count);
+    if (ff_capable(s)) return defer_scale<ff::f2>(f.data(), f.size(), true);
+    return s.prec ? defer_scale<double>(f.data(), f.size(), true) : defer_scale<float>(f.data(), f.size(), true);
 }
 
 std::vector<const void *> specialised_kernels(Sim &s, const std::vector<std::string> &srcs, const char *entry,
@@ -738,27 +840,25 @@ static size_t check_t(const Sim &s, const GateDesc *gates, size_t count, size_t 
 }
 
 size_t jit_check(const Sim &s, const GateDesc *gates, size_t count, size_t &sweeps) {
-    std::vector<GateDesc> folded;
-    if (!(s.flags & (KBWG_FLAG_EXACT_ORDER | KBWG_FLAG_NO_FOLD))) {
-        folded = fold_diagonals(gates, count);
-        gates = folded.data();
-        count = folded.size();
-    }
+    const std::vector<GateDesc> g = rewritten(s, gates, count);
     if (ff_capable(s)) {
-        std::vector<GateDesc> g = ff_rewrite(gates, count);
         if (chosen_tile(s) == 12) return check_p<FF2, 12, 4>(s, g.data(), g.size(), sweeps);
         return check_p<FF2, TileCfgFF::K, TileCfgFF::R>(s, g.data(), g.size(), sweeps);
     }
-    return s.prec ? check_t<double>(s, gates, count, sweeps) : check_t<float>(s, gates, count, sweeps);
+    return s.prec ? check_t<double>(s, g.data(), g.size(), sweeps) : check_t<float>(s, g.data(), g.size(), sweeps);
 }
 
 cudaError_t run_fused(Sim &s, const GateDesc *gates, size_t count) {
-    std::vector<GateDesc> folded;
-    if (!(s.flags & (KBWG_FLAG_EXACT_ORDER | KBWG_FLAG_NO_FOLD))) {
-        folded = fold_diagonals(gates, count);
-        gates = folded.data();
-        count = folded.size();
+    if (effective_tile_k(s) == 0) {  // the state is smaller than every tile: one kernel per gate
+        std::vector<GateDesc> folded;
+        if (!(s.flags & (KBWG_FLAG_EXACT_ORDER | KBWG_FLAG_NO_FOLD))) {
+            folded = fold_diagonals(gates, count);
+            gates = folded.data();
+            count = folded.size();
+        }
+        return s.prec ? run_fused_t<double>(s, gates, count) : run_fused_t<float>(s, gates, count);
     }
+    const std::vector<GateDesc> g = rewritten(s, gates, count);
     if (ff_capable(s)) {
         // float-float sweeps read and write the float-float form; the state
         // stays in it until an operation needs binary64
@@ -767,12 +867,11 @@ cudaError_t run_fused(Sim &s, const GateDesc *gates, size_t count) {
             if (e != cudaSuccess) return e;
             s.ff_resident = true;
         }
-        std::vector<GateDesc> g = ff_rewrite(gates, count);
         if (s.n > 32) return run_fused_p<FF2, TileCfgFF::K, TileCfgFF::R, true>(s, g.data(), g.size());
         if (chosen_tile(s) == 12) return run_fused_p<FF2, 12, 4>(s, g.data(), g.size());
         return run_fused_p<FF2, TileCfgFF::K, TileCfgFF::R>(s, g.data(), g.size());
     }
-    return s.prec ? run_fused_t<double>(s, gates, count) : run_fused_t<float>(s, gates, count);
+    return s.prec ? run_fused_t<double>(s, g.data(), g.size()) : run_fused_t<float>(s, g.data(), g.size());
 }
 
 }  // namespace kbwg

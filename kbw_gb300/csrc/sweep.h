@@ -36,14 +36,14 @@ struct TileCfgFF {
 enum {
     TG_X = 0,      // swap
     TG_Y = 1,      // a0' = -i a1, a1' = i a0
-    TG_H = 2,      // (a0 +- a1) * c0 (sub 0); sub 1: without the factor (float-float path)
-    TG_RX = 3,     // c a - i s partner
-    TG_RY = 4,     // c a -+ s partner
+    TG_H = 2,      // (a0 +- a1) * c0 (sub 0); sub 1: without the factor (deferred)
+    TG_RX = 3,     // c a - i s partner (sub 1: the larger of c, s deferred, see pack_rot)
+    TG_RY = 4,     // c a -+ s partner (sub 1: likewise)
     TG_Z = 5,      // |1> negated (first diagonal class)
     TG_P = 6,      // |1> * (c0 + i c1)
     TG_RZ = 7,     // |0> * (c0 + i c1), |1> * (c2 + i c3)
-    TG_PI = 8,     // |1> * i^q, q = c0 (float-float path)
-    TG_SCALE = 9   // every amplitude * (c0 + i c1) (float-float path)
+    TG_PI = 8,     // |1> * i^q, q = c0
+    TG_SCALE = 9   // every amplitude * (c0 + i c1), the deferred factors (sub 1: * c0, real)
 };
 __host__ __device__ inline bool tg_diagonal(uint32_t cls) { return cls >= TG_Z; }
 constexpr uint8_t TG_OUTER = 0xFF;  // tb value: diagonal gate whose target lies outside the tile
@@ -53,7 +53,9 @@ enum {
     OP_LANE = 0,   // + class (X..RY): target on a lane bit, partner by warp shuffle
     OP_REG = 8,    // + class * 4 + register bit: target on a register bit, in-thread pairs
     OP_DREG = 32,  // + (class - TG_Z) * 4 + register bit: diagonal, target on a register bit
-    OP_DFIX = 48   // + (class - TG_Z): diagonal, side fixed per thread (lane/warp bit) or per tile
+    OP_DFIX = 48,  // + (class - TG_Z): diagonal, side fixed per thread (lane/warp bit) or per tile
+    OP_ROT = 64    // + form * 4 + register bit: RX/RY with a deferred factor (form: 0 RX by tangent, 1 RX by
+                   // cotangent, 2 and 3 RY), set when the constants are packed
 };
 
 // One gate as a tile sees it (64 bytes; staged in shared memory).  The
@@ -93,6 +95,18 @@ __host__ __device__ inline void tile_gate_dispatch(TileGate &g, int R0, int R) {
     if (!tg_diagonal(g.cls)) g.op = (g.tb < kLaneBits) ? OP_LANE + g.cls : OP_REG + g.cls * 4 + rb;
     else if (g.cls != TG_SCALE && reg_target) g.op = OP_DREG + (g.cls - TG_Z) * 4 + rb;
     else g.op = OP_DFIX + (g.cls - TG_Z);
+}
+
+// A rotation with a deferred factor keeps one of its two coefficients: with
+// c = cos, s = sin of half the angle, |c| >= |s| leaves t = s / c and the
+// factor c ("tangent": a0 - t a1, a1 + t a0 for RY), else u = c / s and the
+// factor s ("cotangent": u a0 - a1, u a1 + a0).  c[0] holds t or u (at most 1
+// in size, so a gate grows the state by at most sqrt(2)), c[1] is 1 for the
+// cotangent.  The form follows from the angle: the interpreted kernel finds it
+// in `op`, set here; the specialised ones branch on c[1].
+__host__ __device__ inline void pack_rot(TileGate &g) {
+    if (g.sub != 1 || (g.cls != TG_RX && g.cls != TG_RY)) return;
+    if (g.op >= OP_REG) g.op = (uint8_t)(OP_ROT + ((g.cls == TG_RY ? 2 : 0) + (g.c[1] != 0.0 ? 1 : 0)) * 4 + g.rb);
 }
 
 // Gradient types of the adjoint sweep: the generator of a differentiated

@@ -89,6 +89,7 @@ struct Exact {
     // float<->double conversion issues at the FP64 rate on this chip).
 #if !defined(__CUDACC_RTC__)
     static void pack_host(TileGate &g) {
+        pack_rot(g);
         T v[4];
         for (int i = 0; i < 4; i++) v[i] = (T)g.c[i];
         memset(g.c, 0, sizeof g.c);
@@ -152,7 +153,15 @@ struct Exact {
         return Amp{xadd(xmul(k.c0, self.re), xmul(ss, o.re)), xadd(xmul(k.c0, self.im), xmul(ss, o.im))};
     }
     static __device__ __forceinline__ Amp cmul(Amp a, T c, T s) { return cmul_exact(a, c, s); }
-    static __device__ __forceinline__ Amp pi_mul(Amp a, int) { return a; }  // float-float path only
+    // |1> * i^q and the deferred forms never run in program order
+    static constexpr bool kDefer = false;
+    static __device__ __forceinline__ int power_of_i(const K4 &k) { return (int)k.c0; }
+    static __device__ __forceinline__ Amp pi_mul(Amp a, int q) {
+        if (q == 1) return Amp{-a.im, a.re};
+        if (q == 2) return Amp{-a.re, -a.im};
+        return Amp{a.im, -a.re};
+    }
+    static __device__ __forceinline__ Amp smul(Amp a, T c) { return Amp{xmul(a.re, c), xmul(a.im, c)}; }
 };
 
 // Fast: the same gates with fused multiply-adds (RX/RY 8 FP operations per
@@ -165,14 +174,20 @@ struct Fast : Exact<T> {
     using K4 = typename Exact<T>::K4;
     // (the products are explicitly rounded: a plain product could be fused
     // with the next gate's sum once gates run as straight-line code)
-    static __device__ __forceinline__ void h_pair(int, const K4 &k, Amp &a0, Amp &a1) {
-        const Amp n0{xmul(a0.re + a1.re, k.c0), xmul(a0.im + a1.im, k.c0)};
-        const Amp n1{xmul(a0.re - a1.re, k.c0), xmul(a0.im - a1.im, k.c0)};
+    static __device__ __forceinline__ void h_pair(int sub, const K4 &k, Amp &a0, Amp &a1) {
+        Amp n0{xadd(a0.re, a1.re), xadd(a0.im, a1.im)};
+        Amp n1{xsub(a0.re, a1.re), xsub(a0.im, a1.im)};
+        if (sub == 0) {
+            n0 = Amp{xmul(n0.re, k.c0), xmul(n0.im, k.c0)};
+            n1 = Amp{xmul(n1.re, k.c0), xmul(n1.im, k.c0)};
+        }
         a0 = n0;
         a1 = n1;
     }
-    static __device__ __forceinline__ Amp h_half(int, const K4 &k, Amp self, Amp o, T sgn) {
-        return Amp{xmul(fma(sgn, self.re, o.re), k.c0), xmul(fma(sgn, self.im, o.im), k.c0)};
+    static __device__ __forceinline__ Amp h_half(int sub, const K4 &k, Amp self, Amp o, T sgn) {
+        const Amp n{fma(sgn, self.re, o.re), fma(sgn, self.im, o.im)};
+        if (sub != 0) return n;
+        return Amp{xmul(n.re, k.c0), xmul(n.im, k.c0)};
     }
     static __device__ __forceinline__ void rx_pair(const K4 &k, Amp &a0, Amp &a1) {
         const Amp n0{fma(k.c0, a0.re, k.c1 * a1.im), fma(k.c0, a0.im, -k.c1 * a1.re)};
@@ -194,6 +209,54 @@ struct Fast : Exact<T> {
     }
     static __device__ __forceinline__ Amp cmul(Amp a, T c, T s) {
         return Amp{fma(a.re, c, -a.im * s), fma(a.re, s, a.im * c)};
+    }
+    // RX/RY with a deferred factor (pack_rot): one FMA per real part where
+    // the full form takes a product and an FMA
+    static constexpr bool kDefer = true;
+    static __device__ __forceinline__ bool cot(const K4 &k) { return k.c1 != (T)0; }
+    template <bool COT>
+    static __device__ __forceinline__ void rxd_pair(const K4 &k, Amp &a0, Amp &a1) {
+        const T t = k.c0;
+        Amp n0, n1;
+        if constexpr (COT) {  // u a0 - i a1, u a1 - i a0
+            n0 = Amp{fma(t, a0.re, a1.im), fma(t, a0.im, -a1.re)};
+            n1 = Amp{fma(t, a1.re, a0.im), fma(t, a1.im, -a0.re)};
+        } else {  // a0 - i t a1, a1 - i t a0
+            n0 = Amp{fma(t, a1.im, a0.re), fma(-t, a1.re, a0.im)};
+            n1 = Amp{fma(t, a0.im, a1.re), fma(-t, a0.re, a1.im)};
+        }
+        a0 = n0;
+        a1 = n1;
+    }
+    template <bool COT>
+    static __device__ __forceinline__ void ryd_pair(const K4 &k, Amp &a0, Amp &a1) {
+        const T t = k.c0;
+        Amp n0, n1;
+        if constexpr (COT) {  // u a0 - a1, u a1 + a0
+            n0 = Amp{fma(t, a0.re, -a1.re), fma(t, a0.im, -a1.im)};
+            n1 = Amp{fma(t, a1.re, a0.re), fma(t, a1.im, a0.im)};
+        } else {  // a0 - t a1, a1 + t a0
+            n0 = Amp{fma(-t, a1.re, a0.re), fma(-t, a1.im, a0.im)};
+            n1 = Amp{fma(t, a0.re, a1.re), fma(t, a0.im, a1.im)};
+        }
+        a0 = n0;
+        a1 = n1;
+    }
+    template <bool COT>
+    static __device__ __forceinline__ Amp rxd_half(const K4 &k, Amp self, Amp o) {
+        if constexpr (COT) return Amp{fma(k.c0, self.re, o.im), fma(k.c0, self.im, -o.re)};
+        return Amp{fma(k.c0, o.im, self.re), fma(-k.c0, o.re, self.im)};
+    }
+    // w: one ? 1 : -1 (cotangent) or one ? t : -t (tangent)
+    template <bool COT>
+    static __device__ __forceinline__ T ryd_weight(const K4 &k, bool one) {
+        const T w = COT ? (T)1 : k.c0;
+        return one ? w : -w;
+    }
+    template <bool COT>
+    static __device__ __forceinline__ Amp ryd_half(const K4 &k, Amp self, Amp o, T w) {
+        if constexpr (COT) return Amp{fma(k.c0, self.re, w * o.re), fma(k.c0, self.im, w * o.im)};
+        return Amp{fma(w, o.re, self.re), fma(w, o.im, self.im)};
     }
 };
 
@@ -233,14 +296,18 @@ struct FastP {
     static __device__ __forceinline__ float2 mul_rn(float2 a, float c) {
         return make_float2(__fmul_rn(a.x, c), __fmul_rn(a.y, c));
     }
-    static __device__ __forceinline__ void h_pair(int, const K4 &k, Amp &a0, Amp &a1) {
-        const Amp n0 = mul_rn(__fadd2_rn(a0, a1), k.c0);
-        const Amp n1 = mul_rn(ff2::sub(a0, a1), k.c0);
+    static __device__ __forceinline__ void h_pair(int sub, const K4 &k, Amp &a0, Amp &a1) {
+        Amp n0 = __fadd2_rn(a0, a1), n1 = ff2::sub(a0, a1);
+        if (sub == 0) {
+            n0 = mul_rn(n0, k.c0);
+            n1 = mul_rn(n1, k.c0);
+        }
         a0 = n0;
         a1 = n1;
     }
-    static __device__ __forceinline__ Amp h_half(int, const K4 &k, Amp self, Amp o, float sgn) {
-        return mul_rn(__ffma2_rn(bc(sgn), self, o), k.c0);
+    static __device__ __forceinline__ Amp h_half(int sub, const K4 &k, Amp self, Amp o, float sgn) {
+        const Amp n = __ffma2_rn(bc(sgn), self, o);
+        return sub == 0 ? mul_rn(n, k.c0) : n;
     }
     static __device__ __forceinline__ void rx_pair(const K4 &k, Amp &a0, Amp &a1) {
         const float2 c = bc(k.c0), s = make_float2(k.c1, -k.c1);
@@ -267,7 +334,50 @@ struct FastP {
     static __device__ __forceinline__ Amp cmul(Amp a, float c, float s) {
         return __ffma2_rn(a, bc(c), __fmul2_rn(swp(a), make_float2(-s, s)));
     }
-    static __device__ __forceinline__ Amp pi_mul(Amp a, int) { return a; }  // float-float path only
+    static __device__ __forceinline__ Amp pi_mul(Amp a, int q) {
+        if (q == 1) return make_float2(-a.y, a.x);
+        if (q == 2) return make_float2(-a.x, -a.y);
+        return make_float2(a.y, -a.x);
+    }
+    static __device__ __forceinline__ int power_of_i(const K4 &k) { return (int)k.c0; }
+    static __device__ __forceinline__ Amp smul(Amp a, float c) { return mul_rn(a, c); }
+    // RX/RY with a deferred factor (pack_rot): one packed FMA per amplitude
+    static constexpr bool kDefer = true;
+    static __device__ __forceinline__ bool cot(const K4 &k) { return k.c1 != 0.f; }
+    template <bool COT>
+    static __device__ __forceinline__ Amp rxd_half(const K4 &k, Amp self, Amp o) {
+        if constexpr (COT) return __ffma2_rn(bc(k.c0), self, make_float2(o.y, -o.x));
+        return __ffma2_rn(make_float2(k.c0, -k.c0), swp(o), self);
+    }
+    template <bool COT>
+    static __device__ __forceinline__ void rxd_pair(const K4 &k, Amp &a0, Amp &a1) {
+        const Amp n0 = rxd_half<COT>(k, a0, a1), n1 = rxd_half<COT>(k, a1, a0);
+        a0 = n0;
+        a1 = n1;
+    }
+    template <bool COT>
+    static __device__ __forceinline__ void ryd_pair(const K4 &k, Amp &a0, Amp &a1) {
+        Amp n0, n1;
+        if constexpr (COT) {
+            n0 = __ffma2_rn(bc(k.c0), a0, make_float2(-a1.x, -a1.y));
+            n1 = __ffma2_rn(bc(k.c0), a1, a0);
+        } else {
+            n0 = __ffma2_rn(bc(-k.c0), a1, a0);
+            n1 = __ffma2_rn(bc(k.c0), a0, a1);
+        }
+        a0 = n0;
+        a1 = n1;
+    }
+    template <bool COT>
+    static __device__ __forceinline__ float ryd_weight(const K4 &k, bool one) {
+        const float w = COT ? 1.f : k.c0;
+        return one ? w : -w;
+    }
+    template <bool COT>
+    static __device__ __forceinline__ Amp ryd_half(const K4 &k, Amp self, Amp o, float w) {
+        if constexpr (COT) return __ffma2_rn(bc(k.c0), self, __fmul2_rn(bc(w), o));
+        return __ffma2_rn(bc(w), o, self);
+    }
 };
 
 // ---- float-float policy (complex128 fast path) ---------------------------------
@@ -291,6 +401,7 @@ struct FFPol {
     static __device__ __forceinline__ Mem to_mem(Amp a) { return Mem{ff::to_double(a.re), ff::to_double(a.im)}; }
 #if !defined(__CUDACC_RTC__)
     static void pack_host(TileGate &g) {
+        pack_rot(g);
         double c[4] = {g.c[0], g.c[1], g.c[2], g.c[3]};
         float f[8];
         for (int i = 0; i < 4; i++) {
@@ -365,6 +476,9 @@ struct FFPol {
     static __device__ __forceinline__ Amp cmul(Amp a, ff::f2 c, ff::f2 s) {
         return Amp{ff::dot2(c, a.re, ff::neg(s), a.im), ff::dot2(c, a.im, s, a.re)};
     }
+    static constexpr bool kDefer = false;
+    static __device__ __forceinline__ int power_of_i(const K4 &k) { return (int)k.c0.h; }
+    static __device__ __forceinline__ Amp smul(Amp a, ff::f2 c) { return Amp{ff::mul(a.re, c), ff::mul(a.im, c)}; }
     static __device__ __forceinline__ Amp pi_mul(Amp a, int q) {
         if (q == 1) return Amp{ff::neg(a.im), a.re};
         if (q == 2) return Amp{ff::neg(a.re), ff::neg(a.im)};
@@ -450,6 +564,50 @@ struct FF2 {
         if (q == 1) return ff2::mul_i(a);
         if (q == 2) return ff2::neg(a);
         return ff2::mul_minus_i(a);
+    }
+    static __device__ __forceinline__ int power_of_i(const K4 &k) { return (int)k.c0.h; }
+    static __device__ __forceinline__ Amp smul(Amp a, ff::f2 c) { return ff2::mul(a, ff2::konst(c)); }
+    // RX/RY with a deferred factor (pack_rot): 15 packed operations per
+    // amplitude (ff2::axpy) where the full form's dot product takes 19
+    static constexpr bool kDefer = true;
+    static __device__ __forceinline__ bool cot(const K4 &k) { return k.c1.h != 0.f; }
+    template <bool COT>
+    static __device__ __forceinline__ Amp rxd_half(const K4 &k, Amp self, Amp o) {
+        if constexpr (COT) return ff2::axpy(ff2::konst(k.c0), self, ff2::mul_minus_i(o));
+        return ff2::axpy(ff2::konst(k.c0, ff::neg(k.c0)), ff2::swap(o), self);
+    }
+    template <bool COT>
+    static __device__ __forceinline__ void rxd_pair(const K4 &k, Amp &a0, Amp &a1) {
+        const Amp n0 = rxd_half<COT>(k, a0, a1), n1 = rxd_half<COT>(k, a1, a0);
+        a0 = n0;
+        a1 = n1;
+    }
+    template <bool COT>
+    static __device__ __forceinline__ void ryd_pair(const K4 &k, Amp &a0, Amp &a1) {
+        const ff2::k2 t = ff2::konst(k.c0);
+        Amp n0, n1;
+        if constexpr (COT) {
+            n0 = ff2::axmy(t, a0, a1);
+            n1 = ff2::axpy(t, a1, a0);
+        } else {
+            n0 = ff2::axpy(ff2::konst(ff::neg(k.c0)), a1, a0);
+            n1 = ff2::axpy(t, a0, a1);
+        }
+        a0 = n0;
+        a1 = n1;
+    }
+    template <bool COT>
+    static __device__ __forceinline__ ff::f2 ryd_weight(const K4 &k, bool one) {
+        const ff::f2 w = COT ? ff::f2{1.f, 0.f} : k.c0;
+        return one ? w : ff::neg(w);
+    }
+    template <bool COT>
+    static __device__ __forceinline__ Amp ryd_half(const K4 &k, Amp self, Amp o, ff::f2 w) {
+        if constexpr (COT) {
+            const float2 s = make_float2(w.h, w.h);  // +-1, exact
+            return ff2::axpy(ff2::konst(k.c0), self, ff2::v2{ff2::mul(o.h, s), ff2::mul(o.l, s)});
+        }
+        return ff2::axpy(ff2::konst(w), o, self);
     }
 };
 
@@ -567,7 +725,7 @@ __device__ __forceinline__ void diag_reg(typename P::Amp (&v)[1 << R], const Til
             } else if constexpr (CLS == TG_RZ) {
                 v[j] = hi ? P::cmul(v[j], k.c2, k.c3) : P::cmul(v[j], k.c0, k.c1);
             } else {  // TG_PI
-                if (hi) v[j] = P::pi_mul(v[j], (int)reinterpret_cast<const float &>(k.c0));
+                if (hi) v[j] = P::pi_mul(v[j], P::power_of_i(k));
             }
         }
     }
@@ -586,7 +744,7 @@ __device__ __forceinline__ void diag_fixed(typename P::Amp (&v)[1 << R], const T
         for (int j = 0; j < NR; j++)
             if (KBWG_JM(j)) v[j] = P::neg(v[j]);
     } else if constexpr (CLS == TG_PI) {
-        const int q = (int)reinterpret_cast<const float &>(k.c0);
+        const int q = P::power_of_i(k);
 #pragma unroll
         for (int j = 0; j < NR; j++)
             if (KBWG_JM(j)) v[j] = P::pi_mul(v[j], q);
@@ -594,9 +752,45 @@ __device__ __forceinline__ void diag_fixed(typename P::Amp (&v)[1 << R], const T
         // P: |1> * (c0, c1); SCALE: all * (c0, c1); RZ: (c0, c1) or (c2, c3)
         const auto c = (CLS == TG_RZ && one) ? k.c2 : k.c0;
         const auto s = (CLS == TG_RZ && one) ? k.c3 : k.c1;
+        if (CLS == TG_SCALE && g.sub != 0) {  // real factor
+#pragma unroll
+            for (int j = 0; j < NR; j++) v[j] = P::smul(v[j], c);
+            return;
+        }
 #pragma unroll
         for (int j = 0; j < NR; j++)
             if (KBWG_JM(j)) v[j] = P::cmul(v[j], c, s);
+    }
+}
+
+// RX/RY with a deferred factor on register bit B (uncontrolled: every pair).
+template <class P, int R, int B, bool RYG, bool COT>
+__device__ __forceinline__ void rot_pairs(typename P::Amp (&v)[1 << R], const TileGate &g) {
+    if constexpr (B < R && P::kDefer) {
+        const typename P::K4 k = P::load(g);
+#pragma unroll
+        for (int jj = 0; jj < (1 << (R - 1)); jj++) {
+            const int j0 = ((jj >> B) << (B + 1)) | (jj & ((1 << B) - 1));
+            const int j1 = j0 | (1 << B);
+            if constexpr (RYG) P::template ryd_pair<COT>(k, v[j0], v[j1]);
+            else P::template rxd_pair<COT>(k, v[j0], v[j1]);
+        }
+    }
+}
+
+// The same on lane bit TB's partner (every lane takes part, all uncontrolled).
+template <class P, int R, bool RYG, bool COT>
+__device__ __forceinline__ void rot_lane(typename P::Amp (&v)[1 << R], const typename P::K4 &k, uint32_t tb, uint32_t F) {
+    if constexpr (P::kDefer) {
+        const bool one = ((F >> tb) & 1u) != 0;
+        const int m = 1 << tb;
+        const auto w = P::template ryd_weight<COT>(k, one);
+#pragma unroll
+        for (int j = 0; j < (1 << R); j++) {
+            const typename P::Amp o = P::shfl(v[j], m);
+            if constexpr (RYG) v[j] = P::template ryd_half<COT>(k, v[j], o, w);
+            else v[j] = P::template rxd_half<COT>(k, v[j], o);
+        }
     }
 }
 
@@ -608,8 +802,10 @@ template <bool W, class A, class C> struct pick_t { using type = A; };
 template <class A, class C> struct pick_t<false, A, C> { using type = C; };
 
 // B: type of the state index (32 bits up to 32 qubits, 64 bits above; not
-// deduced from the argument, so a caller names 64 bits explicitly).
-template <class P, int K, int R, class B = uint32_t>
+// deduced from the argument, so a caller names 64 bits explicitly).  ROT:
+// the program may hold rotations with deferred factors (their bodies cost
+// the adjoint's kernels, which never run them, registers).
+template <class P, int K, int R, class B = uint32_t, bool ROT = P::kDefer>
 __device__ __forceinline__ void tile_gate(const TileGate &g, typename P::Amp (&v)[1 << R], int /*R0*/, uint32_t F,
                                           typename ident<B>::type base) {
     static_assert(R >= 3 && R <= 4, "dispatch covers register bits 0..3");
@@ -623,7 +819,18 @@ __device__ __forceinline__ void tile_gate(const TileGate &g, typename P::Amp (&v
         if (op == OP_LANE + TG_X) lane_gate<P, R, TG_X>(v, g, fok, F);
         else if (op == OP_LANE + TG_Y) lane_gate<P, R, TG_Y>(v, g, fok, F);
         else if (op == OP_LANE + TG_H) lane_gate<P, R, TG_H>(v, g, fok, F);
-        else if (op == OP_LANE + TG_RX) lane_gate<P, R, TG_RX>(v, g, fok, F);
+        else if (ROT && g.sub != 0) {
+            if constexpr (ROT) {
+                const typename P::K4 k = P::load(g);
+                if (op == OP_LANE + TG_RX) {
+                    if (P::cot(k)) rot_lane<P, R, false, true>(v, k, g.tb, F);
+                    else rot_lane<P, R, false, false>(v, k, g.tb, F);
+                } else {
+                    if (P::cot(k)) rot_lane<P, R, true, true>(v, k, g.tb, F);
+                    else rot_lane<P, R, true, false>(v, k, g.tb, F);
+                }
+            }
+        } else if (op == OP_LANE + TG_RX) lane_gate<P, R, TG_RX>(v, g, fok, F);
         else lane_gate<P, R, TG_RY>(v, g, fok, F);
         return;
     }
@@ -646,10 +853,17 @@ __device__ __forceinline__ void tile_gate(const TileGate &g, typename P::Amp (&v
         diag_fixed<P, R, C>(v, g, jm, one);                                                                 \
         break;                                                                                              \
     }
+#define KBWG_ROT(F4, RYG, COT)                                                 \
+    case OP_ROT + F4 * 4 + 0: rot_pairs<P, R, ROT ? 0 : R, RYG, COT>(v, g); break; \
+    case OP_ROT + F4 * 4 + 1: rot_pairs<P, R, ROT ? 1 : R, RYG, COT>(v, g); break; \
+    case OP_ROT + F4 * 4 + 2: rot_pairs<P, R, ROT ? 2 : R, RYG, COT>(v, g); break; \
+    case OP_ROT + F4 * 4 + 3: rot_pairs<P, R, ROT ? 3 : R, RYG, COT>(v, g); break;
         KBWG_REG(TG_X) KBWG_REG(TG_Y) KBWG_REG(TG_H) KBWG_REG(TG_RX) KBWG_REG(TG_RY)
+        KBWG_ROT(0, false, false) KBWG_ROT(1, false, true) KBWG_ROT(2, true, false) KBWG_ROT(3, true, true)
         KBWG_DREG(TG_Z) KBWG_DREG(TG_P) KBWG_DREG(TG_RZ) KBWG_DREG(TG_PI)
         KBWG_DFIX(TG_Z) KBWG_DFIX(TG_P) KBWG_DFIX(TG_RZ) KBWG_DFIX(TG_PI) KBWG_DFIX(TG_SCALE)
 #undef KBWG_REG
+#undef KBWG_ROT
 #undef KBWG_DREG
 #undef KBWG_DFIX
     default: break;
