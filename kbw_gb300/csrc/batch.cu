@@ -5,14 +5,20 @@
 // fresh simulator that replays the gates and sums the strings
 // (kbw src/quantum_execution.rs:392-405, 109-158).  Here the host plans
 // every circuit with the sweep planner (planner.cpp) into the gate programs
-// the tile kernels run, and persistent CTAs take circuits from a queue
-// sorted by cost (largest first):
-//   * n <= K: the circuit runs on a K-qubit tile that never leaves the SM
-//     (qubits n..K-1 stay |0>), its sweeps applied to the tile in registers
-//     and shared memory;
-//   * n > K: the state lives in the CTA's slot of a global buffer; every
-//     planned sweep walks the slot tile by tile (TMA bulk loads, bounded
-//     waits, coalesced stores), as k_sweep walks a handle's state.
+// the tile kernels run, and cuts the work into items that persistent CTAs take
+// from one queue:
+//   * n <= K: one item, the whole circuit on a K-qubit tile that never leaves
+//     the SM (qubits n..K-1 stay |0>), its sweeps applied to the tile in
+//     registers and shared memory;
+//   * n > K: the state has its place in a global buffer, and an item is a few
+//     tiles of one planned sweep (TMA bulk loads one tile ahead, bounded waits,
+//     coalesced stores, as k_sweep walks a handle's state) or of one <H> pass.
+//     An item waits until its circuit's earlier sweeps are done (a counter per
+//     circuit).  The queue is ordered by sweep, so every item that another one
+//     waits for was taken before it: the first unfinished item never waits,
+//     whatever the number of resident CTAs.
+// One CTA per circuit would leave the largest circuits to single SMs: 1024
+// circuits of 8..20 qubits took 55 ms, the time of one 20-qubit circuit's CTA.
 // <H> = sum_k c_k <P_k> with P = i^{ny} X^x Z^z: the strings are grouped by
 // flip mask x, and for each group one loop over the amplitudes forms
 // conj(a_s) a_{s^x} once and adds every string's signed share, accumulated
@@ -47,6 +53,21 @@ struct BatchJob {
     uint32_t n, nsweeps, sweep_off, nterms;
     uint32_t term_off, id, pad;
     uint32_t pass_off, npasses;  // tiled <H> passes (registers larger than a tile)
+    uint32_t items, part_off, nparts;  // items of the circuit; its partial sums of <H>
+    uint64_t state_off;                // first amplitude of its state (n > K)
+};
+
+// What an item of the queue does: part `part` of task `task`.
+enum { BT_WHOLE = 0, BT_SWEEP = 1, BT_PASS = 2, BT_WIDE = 3 };
+struct BatchTask {
+    uint32_t job, kind;
+    uint32_t index;  // sweep or pass of the circuit
+    uint32_t need;   // items of the circuit that must be done first
+    uint32_t per;    // tiles per part (BT_WIDE: log2 of the amplitudes per part)
+    uint32_t slot;   // partial sum of part 0 (BT_PASS, BT_WIDE), within the circuit's
+};
+struct BatchItem {
+    uint32_t task, part;
 };
 
 struct BatchTerm {
@@ -74,16 +95,19 @@ struct BatchTileTerm {
 
 struct BatchArgs {
     const BatchJob *jobs;
-    uint32_t njobs;
+    const BatchTask *tasks;
+    const BatchItem *items;
+    uint32_t nitems;
     unsigned *next;
+    unsigned *done;      // finished items per job
+    double *partials;
     const BatchSweep *sweeps;
     const TileGate *prog;
     const BatchTerm *terms;
     const BatchPass *passes;
     const BatchTileTerm *tterms;
     double *energies;
-    void *slots;
-    uint64_t slot_elems;
+    void *states;
     int *err;
 };
 
@@ -92,9 +116,47 @@ struct BatchKernel {
     using Mem = typename P::Mem;
     static constexpr int kThreads = 32 << (K - kLaneBits - R);
     static constexpr size_t kTileBytes = sizeof(Mem) << K;
-    static constexpr size_t kSmem = kTileBytes + 256 * sizeof(uint64_t) + kMaxSweepGates * sizeof(TileGate) + 64 +
+    static constexpr size_t kSmem = 2 * kTileBytes + 256 * sizeof(uint64_t) + kMaxSweepGates * sizeof(TileGate) + 64 +
                                     32 * 8 + 64;
 };
+
+// Wait until `need` items of a circuit are done (polled by one thread, at
+// most ~10 s); false, with the error flag set, if they never are.  Then orders
+// the circuit's amplitudes, written by other CTAs through the generic proxy,
+// before this CTA's TMA loads.
+__device__ __forceinline__ bool batch_wait(const unsigned *done, uint32_t need, int *err) {
+    bool ok = true;
+    if (threadIdx.x == 0) {
+        ok = false;
+        for (uint32_t spin = 0; spin < (1u << 25); spin++) {
+            unsigned v;
+            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(done) : "memory");
+            if (v >= need) {
+                ok = true;
+                break;
+            }
+            if ((spin & 1023u) == 1023u && *(volatile int *)err) break;  // another wait ran out
+            __nanosleep(200);
+        }
+        if (!ok) atomicExch(err, 1);
+    }
+    if (__syncthreads_or(!ok)) return false;
+    __threadfence();
+    asm volatile("fence.proxy.async;" ::: "memory");
+    return true;
+}
+
+// Sum of v over the CTA (every thread must call it); valid in thread 0.
+__device__ __forceinline__ double batch_block_sum(double v, double *red) {
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+    __syncthreads();
+    double t = 0.0;
+    if (threadIdx.x == 0)
+        for (int w = 0; w < (int)(blockDim.x >> 5); w++) t += red[w];
+    __syncthreads();
+    return t;
+}
 
 // FP64-grade sum of float shares (short float runs, then widened) or of
 // double shares
@@ -121,84 +183,93 @@ __device__ __forceinline__ Mem batch_basis(bool one) {
     return m;
 }
 
-// <H> of a register larger than a tile, in tiled passes: each tile staged
-// once per pass (TMA), every string of the pass summed from shared memory.
-// (Its own function: the sweep loop keeps its register allocation.)
+// Part of one tiled <H> pass of a register larger than a tile: tiles [t0, t1),
+// each staged once (TMA, one tile ahead), every string of the pass summed from
+// shared memory.  (Its own function: the sweep loop keeps its register
+// allocation.)
 template <class P, int K, int R>
-__device__ __noinline__ bool batch_energy_passes(const BatchArgs &a, const BatchJob &job, typename P::Mem *slot,
-                                                 typename P::Mem *tile_mem, uint64_t *chunk_off, uint64_t *bar,
-                                                 uint32_t &phase, double &sum) {
+__device__ __noinline__ bool batch_energy_pass(const BatchArgs &a, const BatchPass &bp, uint32_t n,
+                                               typename P::Mem *state, uint64_t t0, uint64_t t1,
+                                               typename P::Mem *tiles_mem, uint64_t *chunk_off, uint64_t *bar,
+                                               uint32_t *phase, double &sum) {
     using Mem = typename P::Mem;
     using T = decltype(Mem{}.re);
     BatchAcc<T> acc;  // (local: the caller's accumulator would live in memory across the call)
     using BK = BatchKernel<P, K, R>;
     constexpr int NR = 1 << R;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const uint32_t n = job.n;
-    for (uint32_t pi = 0; pi < job.npasses; pi++) {
-        const BatchPass &bp = a.passes[job.pass_off + pi];
-        const uint32_t l = bp.l, m = bp.m;
-        const uint32_t chunk = 1u << l, nchunks = 1u << m;
-        for (uint32_t c = threadIdx.x; c < nchunks; c += blockDim.x) {
-            uint64_t off = 0;
-            for (uint32_t j = 0; j < m; j++) off |= (uint64_t)((c >> j) & 1u) << bp.hq[j];
-            chunk_off[c] = off;
+    const uint32_t l = bp.l, m = bp.m;
+    const uint32_t chunk = 1u << l, nchunks = 1u << m;
+    for (uint32_t c = threadIdx.x; c < nchunks; c += blockDim.x) {
+        uint64_t off = 0;
+        for (uint32_t j = 0; j < m; j++) off |= (uint64_t)((c >> j) & 1u) << bp.hq[j];
+        chunk_off[c] = off;
+    }
+    __syncthreads();
+    auto tile_base = [&](uint64_t t) {
+        uint64_t b = t << l;
+        for (uint32_t j = 0; j < m; j++) b = insert_zero_at(b, bp.hq[j]);
+        return b;
+    };
+    auto issue_load = [&](uint64_t t, uint32_t buf) {
+        if (warp == 0) {
+            const uint64_t b = tile_base(t);
+            if (lane == 0) mbar_expect_tx(bar + buf, (uint32_t)BK::kTileBytes);
+            __syncwarp();
+            for (uint32_t c = lane; c < nchunks; c += 32)
+                tma_load(tiles_mem + ((size_t)buf << K) + (size_t)c * chunk, state + b + chunk_off[c],
+                         chunk * (uint32_t)sizeof(Mem), bar + buf);
         }
-        __syncthreads();
-        const uint64_t tiles = 1ull << (n - K);
-        const BatchTileTerm *tt = a.tterms + bp.term_off;
-        for (uint64_t tau = 0; tau < tiles; tau++) {
-            uint64_t base = tau << l;
-            for (uint32_t j = 0; j < m; j++) base = insert_zero_at(base, bp.hq[j]);
-            if (warp == 0) {
-                if (lane == 0) mbar_expect_tx(bar, (uint32_t)BK::kTileBytes);
-                __syncwarp();
-                for (uint32_t c = lane; c < nchunks; c += 32)
-                    tma_load(tile_mem + (size_t)c * chunk, slot + base + chunk_off[c], chunk * (uint32_t)sizeof(Mem),
-                             bar);
-            }
-            if (!tile_wait(bar, phase & 1u, a.err)) return false;
-            phase++;
-            // each thread's NR amplitudes u = tid + i * threads in registers;
-            // strings outer (their fields read once per tile), signs counted
-            // per amplitude, the product formed once per run
-            T ar[NR], ai[NR];
-            int cnt[NR];
+    };
+    const BatchTileTerm *tt = a.tterms + bp.term_off;
+    issue_load(t0, 0);
+    if (t0 + 1 < t1) issue_load(t0 + 1, 1);
+    for (uint64_t tau = t0; tau < t1; tau++) {
+        const uint32_t buf = (uint32_t)(tau - t0) & 1u;
+        const Mem *tile_mem = tiles_mem + ((size_t)buf << K);
+        const uint64_t base = tile_base(tau);
+        if (!tile_wait(bar + buf, phase[buf] & 1u, a.err)) return false;
+        phase[buf]++;
+        // each thread's NR amplitudes u = tid + i * threads in registers;
+        // strings outer (their fields read once per tile), signs counted
+        // per amplitude, the product formed once per run
+        T ar[NR], ai[NR];
+        int cnt[NR];
+#pragma unroll
+        for (int i = 0; i < NR; i++) {
+            const Mem m2 = tile_mem[threadIdx.x + (uint32_t)i * BK::kThreads];
+            ar[i] = m2.re;
+            ai[i] = m2.im;
+            cnt[i] = 0;
+        }
+        for (uint32_t k = 0; k < bp.nterms; k++) {
+            const BatchTileTerm t = tt[k];
+            const uint32_t op = (uint32_t)__popcll(base & t.zo) & 1u;
 #pragma unroll
             for (int i = 0; i < NR; i++) {
-                const Mem m2 = tile_mem[threadIdx.x + (uint32_t)i * BK::kThreads];
-                ar[i] = m2.re;
-                ai[i] = m2.im;
-                cnt[i] = 0;
+                const uint32_t u = threadIdx.x + (uint32_t)i * BK::kThreads;
+                cnt[i] += (((uint32_t)__popc((u ^ t.xl) & t.zl) + op) & 1u) ? -1 : 1;
             }
-            for (uint32_t k = 0; k < bp.nterms; k++) {
-                const BatchTileTerm t = tt[k];
-                const uint32_t op = (uint32_t)__popcll(base & t.zo) & 1u;
+            if (t.last) {  // (uniform)
 #pragma unroll
                 for (int i = 0; i < NR; i++) {
                     const uint32_t u = threadIdx.x + (uint32_t)i * BK::kThreads;
-                    cnt[i] += (((uint32_t)__popc((u ^ t.xl) & t.zl) + op) & 1u) ? -1 : 1;
-                }
-                if (t.last) {  // (uniform)
-#pragma unroll
-                    for (int i = 0; i < NR; i++) {
-                        const uint32_t u = threadIdx.x + (uint32_t)i * BK::kThreads;
-                        T pr, pim;  // conj(a_u) a_{u^x}
-                        if (t.xl == 0u) {
-                            pr = ar[i] * ar[i] + ai[i] * ai[i];
-                            pim = (T)0;
-                        } else {
-                            const Mem ax = tile_mem[u ^ t.xl];
-                            pr = ar[i] * ax.re + ai[i] * ax.im;
-                            pim = ar[i] * ax.im - ai[i] * ax.re;
-                        }
-                        acc.add((T)cnt[i] * ((T)t.cr * pr - (T)t.ci * pim));
-                        cnt[i] = 0;
+                    T pr, pim;  // conj(a_u) a_{u^x}
+                    if (t.xl == 0u) {
+                        pr = ar[i] * ar[i] + ai[i] * ai[i];
+                        pim = (T)0;
+                    } else {
+                        const Mem ax = tile_mem[u ^ t.xl];
+                        pr = ar[i] * ax.re + ai[i] * ax.im;
+                        pim = ar[i] * ax.im - ai[i] * ax.re;
                     }
+                    acc.add((T)cnt[i] * ((T)t.cr * pr - (T)t.ci * pim));
+                    cnt[i] = 0;
                 }
             }
-            __syncthreads();  // the tile is read no more: the next load may land
         }
+        __syncthreads();  // the tile is read no more: a load may land in its buffer
+        if (tau + 2 < t1) issue_load(tau + 2, buf);
     }
     sum = acc.value();
     return true;
@@ -210,11 +281,12 @@ __global__ void __launch_bounds__(BatchKernel<P, K, R>::kThreads, 2) k_batch_cir
     using Mem = typename P::Mem;
     using T = decltype(Mem{}.re);
     using BK = BatchKernel<P, K, R>;
+    static_assert(sizeof(Amp) == sizeof(Mem), "register and memory amplitudes share the tile buffers");
     constexpr int NR = 1 << R;
     extern __shared__ __align__(128) unsigned char smem_raw[];
-    Amp *tile = reinterpret_cast<Amp *>(smem_raw);
+    Amp *tile = reinterpret_cast<Amp *>(smem_raw);  // two tile buffers
     Mem *tile_mem = reinterpret_cast<Mem *>(smem_raw);
-    unsigned char *q = smem_raw + BK::kTileBytes;
+    unsigned char *q = smem_raw + 2 * BK::kTileBytes;
     uint64_t *chunk_off = reinterpret_cast<uint64_t *>(q);
     q += 256 * sizeof(uint64_t);
     TileGate *sg = reinterpret_cast<TileGate *>(q);
@@ -223,161 +295,197 @@ __global__ void __launch_bounds__(BatchKernel<P, K, R>::kThreads, 2) k_batch_cir
     q += 64;
     double *red = reinterpret_cast<double *>(q);
     q += 32 * 8;
-    uint64_t *bar = reinterpret_cast<uint64_t *>(q);
+    uint64_t *bar = reinterpret_cast<uint64_t *>(q);  // one per tile buffer
 
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t FA = (uint32_t)lane | ((uint32_t)warp << (kLaneBits + R));
     const uint32_t FB = (uint32_t)lane | ((uint32_t)warp << kLaneBits);
-    Mem *slot = reinterpret_cast<Mem *>(a.slots) + (size_t)blockIdx.x * a.slot_elems;
     if (threadIdx.x == 0) {
         mbar_init(bar, 1);
+        mbar_init(bar + 1, 1);
         fence_mbar_init();
     }
-    uint32_t phase = 0;
+    uint32_t phase[2] = {0, 0};
     for (;;) {
         __syncthreads();
         if (threadIdx.x == 0) meta[0] = atomicAdd(a.next, 1u);
         __syncthreads();
-        const uint32_t jix = meta[0];
-        if (jix >= a.njobs) break;
-        const BatchJob job = a.jobs[jix];
+        const uint32_t ix = meta[0];
+        if (ix >= a.nitems) break;
+        const BatchItem item = a.items[ix];
+        const BatchTask task = a.tasks[item.task];
+        const BatchJob &job = a.jobs[task.job];
         const uint32_t n = job.n;
-        const bool in_tile = n <= (uint32_t)K;
-        // ---- |0...0> ----
-        if (in_tile) {
-            for (uint32_t u = threadIdx.x; u < (1u << K); u += blockDim.x) tile[u] = P::from_mem(batch_basis<Mem>(u == 0));
-        } else {
-            for (uint64_t s = threadIdx.x; s < (1ull << n); s += blockDim.x) slot[s] = batch_basis<Mem>(s == 0);
-            asm volatile("fence.proxy.async;" ::: "memory");  // generic stores before the sweeps' TMA reads
-        }
-        __syncthreads();
-        // ---- the planned sweeps ----
-        for (uint32_t sw = 0; sw < job.nsweeps; sw++) {
-            const BatchSweep &bs = a.sweeps[job.sweep_off + sw];
-            const uint32_t l = bs.l, m = bs.m, nst = bs.nstages;
-            for (uint32_t i = threadIdx.x; i < bs.gate_count; i += blockDim.x) sg[i] = a.prog[bs.gate_off + i];
-            for (uint32_t c = threadIdx.x; c < (1u << m); c += blockDim.x) {
-                uint64_t off = 0;
-                for (uint32_t j = 0; j < m; j++) off |= (uint64_t)((c >> j) & 1u) << bs.hq[j];
-                chunk_off[c] = off;
-            }
-            __syncthreads();
-            const uint64_t tiles = in_tile ? 1ull : (1ull << (n - K));
-            const uint32_t chunk = 1u << l, nchunks = 1u << m;
-            const uint64_t lowmask = chunk - 1;
-            auto tile_base = [&](uint64_t t) {
-                uint64_t b = t << l;
-                for (uint32_t j = 0; j < m; j++) b = insert_zero_at(b, bs.hq[j]);
-                return b;
-            };
-            // the slot's tiles: tile tau + 1's load is issued before tile tau's
-            // stores (the tiles of a sweep are disjoint)
-            auto issue_load = [&](uint64_t t) {
-                if (warp == 0) {
-                    const uint64_t b = tile_base(t);
-                    if (lane == 0) mbar_expect_tx(bar, (uint32_t)BK::kTileBytes);
-                    __syncwarp();
-                    for (uint32_t c = lane; c < nchunks; c += 32)
-                        tma_load(tile_mem + (size_t)c * chunk, slot + b + chunk_off[c], chunk * (uint32_t)sizeof(Mem),
-                                 bar);
+        Mem *state = reinterpret_cast<Mem *>(a.states) + job.state_off;
+        if (task.need && !batch_wait(a.done + task.job, task.need, a.err)) return;
+        double energy = 0.0;  // this thread's share of <H>
+        if (task.kind == BT_WHOLE || task.kind == BT_SWEEP) {
+            const bool whole = task.kind == BT_WHOLE;
+            const uint32_t s0 = whole ? 0u : task.index, s1 = whole ? job.nsweeps : task.index + 1;
+            const uint64_t ntiles = whole ? 1ull : (1ull << (n - K));
+            const uint64_t t0 = whole ? 0 : (uint64_t)item.part * task.per;
+            const uint64_t t1 = whole ? 1 : min(ntiles, t0 + task.per);
+            if (whole)  // |0...0>
+                for (uint32_t u = threadIdx.x; u < (1u << K); u += blockDim.x) tile[u] = P::from_mem(batch_basis<Mem>(u == 0));
+            for (uint32_t sw = s0; sw < s1; sw++) {
+                const BatchSweep &bs = a.sweeps[job.sweep_off + sw];
+                const uint32_t l = bs.l, m = bs.m, nst = bs.nstages;
+                for (uint32_t i = threadIdx.x; i < bs.gate_count; i += blockDim.x) sg[i] = a.prog[bs.gate_off + i];
+                for (uint32_t c = threadIdx.x; c < (1u << m); c += blockDim.x) {
+                    uint64_t off = 0;
+                    for (uint32_t j = 0; j < m; j++) off |= (uint64_t)((c >> j) & 1u) << bs.hq[j];
+                    chunk_off[c] = off;
                 }
-            };
-            if (!in_tile) issue_load(0);
-            for (uint64_t tau = 0; tau < tiles; tau++) {
-                const uint64_t base = tile_base(tau);
-                int layout = bs.stage_layout[0];
-                int R0 = (layout == LAYOUT_A) ? kLaneBits : (K - R);
-                uint32_t F = (layout == LAYOUT_A) ? FA : FB;
-                Amp v[NR];
-                if (in_tile) {
-#pragma unroll
-                    for (int j = 0; j < NR; j++) v[j] = tile[F | ((uint32_t)j << R0)];
-                } else {
-                    if (!tile_wait(bar, phase & 1u, a.err)) return;
-                    phase++;
-#pragma unroll
-                    for (int j = 0; j < NR; j++) v[j] = P::from_mem(tile_mem[F | ((uint32_t)j << R0)]);
+                __syncthreads();
+                const uint32_t chunk = 1u << l, nchunks = 1u << m;
+                const uint64_t lowmask = chunk - 1;
+                auto tile_base = [&](uint64_t t) {
+                    uint64_t b = t << l;
+                    for (uint32_t j = 0; j < m; j++) b = insert_zero_at(b, bs.hq[j]);
+                    return b;
+                };
+                auto issue_load = [&](uint64_t t, uint32_t buf) {
+                    if (warp == 0) {
+                        const uint64_t b = tile_base(t);
+                        if (lane == 0) mbar_expect_tx(bar + buf, (uint32_t)BK::kTileBytes);
+                        __syncwarp();
+                        for (uint32_t c = lane; c < nchunks; c += 32)
+                            tma_load(tile_mem + ((size_t)buf << K) + (size_t)c * chunk, state + b + chunk_off[c],
+                                     chunk * (uint32_t)sizeof(Mem), bar + buf);
+                    }
+                };
+                // the first sweep starts from |0...0>: nothing is read
+                const bool load = !whole && sw > 0;
+                if (load) {
+                    issue_load(t0, 0);
+                    if (t0 + 1 < t1) issue_load(t0 + 1, 1);
                 }
-                uint32_t g0 = 0;
-                for (uint32_t s = 0; s < nst; s++) {
-                    const int nl = bs.stage_layout[s];
-                    if (nl != layout) {
+                for (uint64_t tau = t0; tau < t1; tau++) {
+                    const uint32_t buf = whole ? 0u : (uint32_t)(tau - t0) & 1u;
+                    Amp *tb = tile + ((size_t)buf << K);
+                    const uint64_t base = tile_base(tau);
+                    int layout = bs.stage_layout[0];
+                    int R0 = (layout == LAYOUT_A) ? kLaneBits : (K - R);
+                    uint32_t F = (layout == LAYOUT_A) ? FA : FB;
+                    Amp v[NR];
+                    if (whole) {
 #pragma unroll
-                        for (int j = 0; j < NR; j++) tile[F | ((uint32_t)j << R0)] = v[j];
+                        for (int j = 0; j < NR; j++) v[j] = tb[F | ((uint32_t)j << R0)];
+                    } else if (load) {
+                        if (!tile_wait(bar + buf, phase[buf] & 1u, a.err)) return;
+                        phase[buf]++;
+                        const Mem *tm = tile_mem + ((size_t)buf << K);
+#pragma unroll
+                        for (int j = 0; j < NR; j++) v[j] = P::from_mem(tm[F | ((uint32_t)j << R0)]);
+                    } else {
+#pragma unroll
+                        for (int j = 0; j < NR; j++) v[j] = P::from_mem(batch_basis<Mem>(base == 0 && F == 0 && j == 0));
+                    }
+                    uint32_t g0 = 0;
+                    for (uint32_t s = 0; s < nst; s++) {
+                        const int nl = bs.stage_layout[s];
+                        if (nl != layout) {
+#pragma unroll
+                            for (int j = 0; j < NR; j++) tb[F | ((uint32_t)j << R0)] = v[j];
+                            __syncthreads();
+                            layout = nl;
+                            R0 = (layout == LAYOUT_A) ? kLaneBits : (K - R);
+                            F = (layout == LAYOUT_A) ? FA : FB;
+#pragma unroll
+                            for (int j = 0; j < NR; j++) v[j] = tb[F | ((uint32_t)j << R0)];
+                        }
+                        const uint32_t g1 = bs.stage_end[s];
+                        for (uint32_t gi = g0; gi < g1; gi++) tile_gate<P, K, R, uint64_t>(sg[gi], v, R0, F, base);
+                        g0 = g1;
+                    }
+                    if (whole) {
+                        // every thread rewrites the positions it read in this layout
+#pragma unroll
+                        for (int j = 0; j < NR; j++) tb[F | ((uint32_t)j << R0)] = v[j];
+                    } else {
+                        // the tile buffer is read no more (the load after next) once all threads pass here
+                        fence_proxy_async();
                         __syncthreads();
-                        layout = nl;
-                        R0 = (layout == LAYOUT_A) ? kLaneBits : (K - R);
-                        F = (layout == LAYOUT_A) ? FA : FB;
+                        if (load && tau + 2 < t1) issue_load(tau + 2, buf);
 #pragma unroll
-                        for (int j = 0; j < NR; j++) v[j] = tile[F | ((uint32_t)j << R0)];
-                    }
-                    const uint32_t g1 = bs.stage_end[s];
-                    for (uint32_t gi = g0; gi < g1; gi++) tile_gate<P, K, R, uint64_t, false>(sg[gi], v, R0, F, base);
-                    g0 = g1;
-                }
-                if (in_tile) {
-                    // every thread rewrites the positions it read in this layout
-#pragma unroll
-                    for (int j = 0; j < NR; j++) tile[F | ((uint32_t)j << R0)] = v[j];
-                } else {
-                    // the tile buffer is read no more (next tile's load) once all threads pass here
-                    fence_proxy_async();
-                    __syncthreads();
-                    if (tau + 1 < tiles) issue_load(tau + 1);
-#pragma unroll
-                    for (int j = 0; j < NR; j++) {
-                        const uint32_t u = F | ((uint32_t)j << R0);
-                        slot[base + chunk_off[u >> l] + (u & lowmask)] = P::to_mem(v[j]);
+                        for (int j = 0; j < NR; j++) {
+                            const uint32_t u = F | ((uint32_t)j << R0);
+                            state[base + chunk_off[u >> l] + (u & lowmask)] = P::to_mem(v[j]);
+                        }
                     }
                 }
+                __syncthreads();
             }
-            if (!in_tile) asm volatile("fence.proxy.async;" ::: "memory");  // this sweep's stores before the next's loads
-            __syncthreads();
+        } else if (task.kind == BT_PASS) {
+            const uint64_t t0 = (uint64_t)item.part * task.per, t1 = min(1ull << (n - K), (unsigned long long)(t0 + task.per));
+            if (!batch_energy_pass<P, K, R>(a, a.passes[job.pass_off + task.index], n, state, t0, t1, tile_mem, chunk_off,
+                                            bar, phase, energy))
+                return;
         }
-        // ---- <H> ----
-        BatchAcc<T> acc;
-        // tiled passes (registers larger than a tile)
-        double tiled = 0.0;
-        if (job.npasses && !batch_energy_passes<P, K, R>(a, job, slot, tile_mem, chunk_off, bar, phase, tiled)) return;
-        const uint64_t ns = 1ull << n;
-        for (uint32_t t0 = 0; t0 < job.nterms;) {
-            const uint64_t x = a.terms[job.term_off + t0].x;
-            uint32_t t1 = t0 + 1;
-            while (t1 < job.nterms && a.terms[job.term_off + t1].x == x) t1++;
-            for (uint64_t s = threadIdx.x; s < ns; s += blockDim.x) {
-                Mem as, ax;
-                if (in_tile) {
-                    as = P::to_mem(tile[s]);
-                    ax = P::to_mem(tile[s ^ x]);
-                } else {
-                    as = slot[s];
-                    ax = slot[s ^ x];
+        if (task.kind == BT_WHOLE || task.kind == BT_WIDE) {
+            // <H> string by string: a register held on the tile, or flip masks too wide for any tile
+            const bool whole = task.kind == BT_WHOLE;
+            const uint64_t a0 = whole ? 0 : (uint64_t)item.part << task.per;
+            const uint64_t a1 = whole ? (1ull << n) : min(1ull << n, (unsigned long long)(a0 + (1ull << task.per)));
+            BatchAcc<T> acc;
+            for (uint32_t t0 = 0; t0 < job.nterms;) {
+                const uint64_t x = a.terms[job.term_off + t0].x;
+                uint32_t t1 = t0 + 1;
+                while (t1 < job.nterms && a.terms[job.term_off + t1].x == x) t1++;
+                for (uint64_t s = a0 + threadIdx.x; s < a1; s += blockDim.x) {
+                    Mem as, ax;
+                    if (whole) {
+                        as = P::to_mem(tile[s]);
+                        ax = P::to_mem(tile[s ^ x]);
+                    } else {
+                        as = state[s];
+                        ax = state[s ^ x];
+                    }
+                    // conj(a_s) a_{s^x}
+                    const T pr = as.re * ax.re + as.im * ax.im, pi = as.re * ax.im - as.im * ax.re;
+                    T share = (T)0;
+                    for (uint32_t k = t0; k < t1; k++) {
+                        const BatchTerm &tk = a.terms[job.term_off + k];
+                        const T w = (T)tk.cr * pr - (T)tk.ci * pi;
+                        share += (__popcll((s ^ x) & tk.z) & 1) ? -w : w;
+                    }
+                    acc.add(share);
                 }
-                // conj(a_s) a_{s^x}
-                const T pr = as.re * ax.re + as.im * ax.im, pi = as.re * ax.im - as.im * ax.re;
-                T share = (T)0;
-                for (uint32_t k = t0; k < t1; k++) {
-                    const BatchTerm &tk = a.terms[job.term_off + k];
-                    const T w = (T)tk.cr * pr - (T)tk.ci * pi;
-                    share += (__popcll((s ^ x) & tk.z) & 1) ? -w : w;
-                }
-                acc.add(share);
+                t0 = t1;
             }
-            t0 = t1;
+            energy = acc.value();
         }
-        double e = acc.value() + tiled;
-        for (int o = 16; o > 0; o >>= 1) e += __shfl_xor_sync(0xffffffffu, e, o);
-        if (lane == 0) red[warp] = e;
+        if (task.kind != BT_SWEEP) {
+            const double e = batch_block_sum(energy, red);
+            if (threadIdx.x == 0) {
+                if (task.kind == BT_WHOLE) a.energies[job.id] = e;
+                else a.partials[job.part_off + task.slot + item.part] = e;
+            }
+        }
+        if (task.kind == BT_WHOLE) continue;
+        // the item is done: its stores before the counter, for the generic
+        // reads and the TMA loads of the items that wait for it; the circuit's
+        // last item adds up its partial sums, in their order
+        __threadfence();
+        asm volatile("fence.proxy.async;" ::: "memory");
         __syncthreads();
         if (threadIdx.x == 0) {
-            double t = 0.0;
-            for (int w2 = 0; w2 < (int)(blockDim.x >> 5); w2++) t += red[w2];
-            a.energies[job.id] = t;
+            unsigned old;
+            asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(old) : "l"(a.done + task.job) : "memory");
+            if (old + 1 == job.items) {
+                double t = 0.0;
+                for (uint32_t k = 0; k < job.nparts; k++) t += __ldcg(a.partials + job.part_off + k);
+                a.energies[job.id] = t;
+            }
         }
     }
 }
 
 // ---- host side -----------------------------------------------------------------------
+// Room for the states of circuits larger than a tile in one launch (more
+// circuits run in further launches on the same buffer).
+constexpr uint64_t kBatchStateBytes = 16ull << 30;
+
 struct BatchCircuitIn {
     uint32_t n;
     std::vector<GateDesc> gates;
@@ -422,7 +530,7 @@ static void batch_parallel_for(size_t n, F &&fn) {
 }
 
 template <class P, int K, int R>
-static int32_t batch_run(int prec, std::vector<BatchCircuitIn> &circs, double *energies) {
+static int32_t batch_run(int arith, std::vector<BatchCircuitIn> &circs, double *energies) {
     using BK = BatchKernel<P, K, R>;
     using Mem = typename P::Mem;
     auto fail = [](cudaError_t e, const char *what) {
@@ -431,11 +539,11 @@ static int32_t batch_run(int prec, std::vector<BatchCircuitIn> &circs, double *e
                   std::string("batch circuits: ") + what + ": " + cudaGetErrorString(e));
         return e == cudaErrorMemoryAllocation ? (int32_t)KBWG_ENOMEM : (int32_t)KBWG_ECUDA;
     };
-    (void)prec;
     // plan every circuit (in parallel: the circuits are independent)
     batch_parallel_for(circs.size(), [&](size_t c) {
         BatchCircuitIn &ci = circs[c];
         const uint32_t nplan = std::max<uint32_t>(ci.n, (uint32_t)K);  // small registers padded with |0> qubits
+        ci.gates = defer_factors(arith, ci.gates.data(), ci.gates.size());
         const std::vector<PlannedSweep> plan =
             plan_sweeps(nplan, K, R, ci.gates.data(), ci.gates.size(), false, kMaxSweepGates);
         size_t placed = 0;
@@ -460,6 +568,14 @@ static int32_t batch_run(int prec, std::vector<BatchCircuitIn> &circs, double *e
             ci.sweeps.push_back(b);
         }
         ci.placed = placed == ci.gates.size();
+        if (ci.sweeps.empty() && ci.n > (uint32_t)K) {  // no gates: a sweep that writes |0...0>
+            BatchSweep b;
+            memset(&b, 0, sizeof b);
+            b.l = (uint32_t)K;
+            b.nstages = 1;
+            b.stage_layout[0] = LAYOUT_A;
+            ci.sweeps.push_back(b);
+        }
         if (ci.n > (uint32_t)K && !ci.terms.empty()) {
             std::vector<uint64_t> xm;
             for (const BatchTerm &t : ci.terms) xm.push_back(t.x);
@@ -564,10 +680,13 @@ static int32_t batch_run(int prec, std::vector<BatchCircuitIn> &circs, double *e
         if (!ci.tterms.empty())
             memcpy(&tterms[tt_off[c]], ci.tterms.data(), ci.tterms.size() * sizeof(BatchTileTerm));
     });
-    // largest first: the persistent CTAs then finish together
-    std::stable_sort(jobs.begin(), jobs.end(), [&](const BatchJob &x, const BatchJob &y) {
-        const double cx = (double)(1ull << x.n) * (1.0 + x.nsweeps + 0.25 * x.nterms);
-        const double cy = (double)(1ull << y.n) * (1.0 + y.nsweeps + 0.25 * y.nterms);
+    // largest first (the queue's order within a sweep)
+    std::vector<uint32_t> order(jobs.size());
+    for (size_t k = 0; k < order.size(); k++) order[k] = (uint32_t)k;
+    std::stable_sort(order.begin(), order.end(), [&](uint32_t x, uint32_t y) {
+        const BatchJob &jx = jobs[x], &jy = jobs[y];
+        const double cx = (double)(1ull << jx.n) * (1.0 + jx.nsweeps + 0.25 * jx.nterms);
+        const double cy = (double)(1ull << jy.n) * (1.0 + jy.nsweeps + 0.25 * jy.nterms);
         return cx > cy;
     });
     int dev = 0, sms = 0;
@@ -578,22 +697,104 @@ static int32_t batch_run(int prec, std::vector<BatchCircuitIn> &circs, double *e
     int occ = 0;
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_batch_circuits<P, K, R>, BK::kThreads, BK::kSmem);
     if (e != cudaSuccess) return fail(e, "occupancy");
-    const uint32_t grid = (uint32_t)std::min<size_t>(jobs.size(), (size_t)sms * std::max(occ, 1));
-    const uint64_t slot_elems = nmax > (uint32_t)K ? (1ull << nmax) : 0;
+    const size_t max_grid = (size_t)sms * std::max(occ, 1);
+    // Rounds: the circuits whose states are in memory together.  A round
+    // takes circuits until their states reach the room (at least one).
+    const uint64_t slot = nmax > (uint32_t)K ? (1ull << nmax) : 0;
+    size_t free_b = 0, total_b = 0;
+    e = cudaMemGetInfo(&free_b, &total_b);
+    if (e != cudaSuccess) return fail(e, "memory query");
+    const uint64_t room =
+        std::max<uint64_t>(slot, std::min<uint64_t>(kBatchStateBytes, free_b / 10 * 8) / sizeof(Mem));
+    std::vector<size_t> round_end;
+    uint64_t state_elems = 0;
+    {
+        uint64_t used = 0;
+        for (size_t k = 0; k < order.size(); k++) {
+            BatchJob &j = jobs[order[k]];
+            if (j.n <= (uint32_t)K) continue;
+            if (used + (1ull << j.n) > room) {
+                round_end.push_back(k);
+                used = 0;
+            }
+            j.state_off = used;
+            used += 1ull << j.n;
+            state_elems = std::max(state_elems, used);
+        }
+        round_end.push_back(order.size());
+    }
+    // the queue: per round, sweep by sweep over its large circuits, then their
+    // <H> parts, then the circuits that stay on one SM
+    std::vector<BatchTask> tasks;
+    std::vector<BatchItem> items;
+    std::vector<size_t> round_items;
+    uint64_t nparts = 0;
+    {
+        size_t k0 = 0;
+        for (size_t ke : round_end) {
+            std::vector<uint32_t> large, small;
+            for (size_t k = k0; k < ke; k++) (jobs[order[k]].n > (uint32_t)K ? large : small).push_back(order[k]);
+            k0 = ke;
+            auto add = [&](uint32_t jx, uint32_t kind, uint32_t index, uint32_t per, uint32_t parts, uint32_t sl) {
+                BatchJob &j = jobs[jx];
+                tasks.push_back(BatchTask{jx, kind, index, 0, per, sl});
+                for (uint32_t p = 0; p < parts; p++) items.push_back(BatchItem{(uint32_t)tasks.size() - 1, p});
+                j.items += parts;
+            };
+            uint32_t deepest = 0;
+            for (uint32_t jx : large) deepest = std::max(deepest, jobs[jx].nsweeps);
+            for (uint32_t sw = 0; sw < deepest; sw++)
+                for (uint32_t jx : large) {
+                    BatchJob &j = jobs[jx];
+                    if (sw >= j.nsweeps) continue;
+                    const uint32_t tiles = 1u << (j.n - K), per = std::min(8u, std::max(1u, tiles / 32u));
+                    const uint32_t need = j.items;
+                    add(jx, BT_SWEEP, sw, per, (tiles + per - 1) / per, 0);
+                    tasks.back().need = need;
+                }
+            for (uint32_t jx : large) {
+                BatchJob &j = jobs[jx];
+                const uint32_t need = j.items, tiles = 1u << (j.n - K), per = std::min(8u, std::max(1u, tiles / 32u));
+                j.part_off = (uint32_t)nparts;
+                for (uint32_t p = 0; p < j.npasses; p++) {
+                    const uint32_t parts = (tiles + per - 1) / per;
+                    add(jx, BT_PASS, p, per, parts, j.nparts);
+                    tasks.back().need = need;
+                    j.nparts += parts;
+                }
+                if (j.nterms) {  // strings too wide for a tile: 2^K amplitudes per part
+                    add(jx, BT_WIDE, 0, (uint32_t)K, tiles, j.nparts);
+                    tasks.back().need = need;
+                    j.nparts += tiles;
+                }
+                nparts += j.nparts;
+            }
+            for (uint32_t jx : small) add(jx, BT_WHOLE, 0, 0, 1, 0);
+            round_items.push_back(items.size());
+        }
+    }
+    if (items.size() > UINT32_MAX || nparts > UINT32_MAX) {
+        set_error(KBWG_EINVAL, "batch circuits: more than 2^32 work items");
+        return KBWG_EINVAL;
+    }
     auto up = [](size_t b) { return (b + 255) & ~(size_t)255; };
     const size_t jb = jobs.size() * sizeof(BatchJob), swb = std::max<size_t>(nsweeps, 1) * sizeof(BatchSweep),
                  pb = std::max<size_t>(nprog, 1) * sizeof(TileGate),
                  tb = std::max<size_t>(nterms, 1) * sizeof(BatchTerm), eb = circs.size() * sizeof(double),
                  pab = std::max<size_t>(npass, 1) * sizeof(BatchPass),
                  ttb = std::max<size_t>(ntt, 1) * sizeof(BatchTileTerm),
-                 sb = (size_t)grid * slot_elems * sizeof(Mem);
+                 tkb = std::max<size_t>(tasks.size(), 1) * sizeof(BatchTask),
+                 itb = std::max<size_t>(items.size(), 1) * sizeof(BatchItem),
+                 ptb = std::max<size_t>((size_t)nparts, 1) * sizeof(double),
+                 cb = (jobs.size() + round_items.size()) * sizeof(unsigned);
     const size_t o_sw = up(jb), o_p = o_sw + up(swb), o_t = o_p + up(pb), o_pa = o_t + up(tb), o_tt = o_pa + up(pab),
-                 o_e = o_tt + up(ttb), o_c = o_e + up(eb), o_err = o_c + 256, o_s = o_err + 256;
+                 o_tk = o_tt + up(ttb), o_it = o_tk + up(tkb), o_pt = o_it + up(itb), o_e = o_pt + up(ptb),
+                 o_c = o_e + up(eb), o_err = o_c + up(cb), o_s = o_err + 256;
     cudaStream_t st = nullptr;
     e = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
     if (e != cudaSuccess) return fail(e, "stream");
     char *dbuf = nullptr;
-    e = cudaMalloc(&dbuf, o_s + sb);
+    e = cudaMalloc(&dbuf, o_s + (size_t)state_elems * sizeof(Mem));
     if (e != cudaSuccess) {
         cudaStreamDestroy(st);
         return fail(e, "buffers");
@@ -601,14 +802,14 @@ static int32_t batch_run(int prec, std::vector<BatchCircuitIn> &circs, double *e
     BatchArgs a;
     memset(&a, 0, sizeof a);
     a.jobs = (const BatchJob *)dbuf;
-    a.njobs = (uint32_t)jobs.size();
-    a.next = (unsigned *)(dbuf + o_c);
+    a.tasks = (const BatchTask *)(dbuf + o_tk);
+    a.done = (unsigned *)(dbuf + o_c);
+    a.partials = (double *)(dbuf + o_pt);
     a.sweeps = (const BatchSweep *)(dbuf + o_sw);
     a.prog = (const TileGate *)(dbuf + o_p);
     a.terms = (const BatchTerm *)(dbuf + o_t);
     a.energies = (double *)(dbuf + o_e);
-    a.slots = dbuf + o_s;
-    a.slot_elems = slot_elems;
+    a.states = dbuf + o_s;
     a.err = (int *)(dbuf + o_err);
     a.passes = (const BatchPass *)(dbuf + o_pa);
     a.tterms = (const BatchTileTerm *)(dbuf + o_tt);
@@ -624,8 +825,17 @@ static int32_t batch_run(int prec, std::vector<BatchCircuitIn> &circs, double *e
         e = copy_async(dbuf + o_pa, passes.get(), npass * sizeof(BatchPass), cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess && ntt)
         e = copy_async(dbuf + o_tt, tterms.get(), ntt * sizeof(BatchTileTerm), cudaMemcpyHostToDevice, st);
-    if (e == cudaSuccess) e = cudaMemsetAsync(dbuf + o_c, 0, 512, st);
-    if (e == cudaSuccess) {
+    if (e == cudaSuccess) e = copy_async(dbuf + o_tk, tasks.data(), tasks.size() * sizeof(BatchTask), cudaMemcpyHostToDevice, st);
+    if (e == cudaSuccess) e = copy_async(dbuf + o_it, items.data(), items.size() * sizeof(BatchItem), cudaMemcpyHostToDevice, st);
+    if (e == cudaSuccess) e = cudaMemsetAsync(dbuf + o_c, 0, up(cb) + 256, st);
+    size_t i0 = 0;
+    for (size_t r = 0; r < round_items.size() && e == cudaSuccess; r++) {
+        a.items = (const BatchItem *)(dbuf + o_it) + i0;
+        a.nitems = (uint32_t)(round_items[r] - i0);
+        a.next = a.done + jobs.size() + r;
+        i0 = round_items[r];
+        if (a.nitems == 0) continue;
+        const uint32_t grid = (uint32_t)std::min<size_t>(a.nitems, max_grid);
         k_batch_circuits<P, K, R><<<grid, BK::kThreads, BK::kSmem, st>>>(a);
         count_launch();
         e = cudaGetLastError();
@@ -697,9 +907,9 @@ int32_t batch_circuits(int precision, uint32_t flags, size_t ncirc, const uint32
             return ci.status;
         }
     if (ncirc == 0) return KBWG_OK;
-    if (precision == KBWG_C64) return batch_run<FastP, 12, 4>(precision, circs, energies);
-    if (flags & KBWG_FLAG_FAST_C128) return batch_run<FF2B, 11, 3>(precision, circs, energies);
-    return batch_run<Fast<double>, 11, 3>(precision, circs, energies);
+    if (precision == KBWG_C64) return batch_run<FastP, 12, 4>(ARITH_C64, circs, energies);
+    if (flags & KBWG_FLAG_FAST_C128) return batch_run<FF2B, 11, 3>(ARITH_FF, circs, energies);
+    return batch_run<Fast<double>, 11, 3>(ARITH_F64, circs, energies);
 }
 
 }  // namespace kbwg

@@ -712,6 +712,20 @@ static std::vector<GateDesc> defer_scale(const GateDesc *gates, size_t count, bo
     return out;
 }
 
+std::vector<GateDesc> defer_factors(int arith, const GateDesc *gates, size_t count) {
+    std::vector<GateDesc> r;
+    if (arith == ARITH_C64) {  // constants in binary64 from the angles
+        r.assign(gates, gates + count);
+        for (GateDesc &x : r)
+            if (x.kind <= G_RZ) x = make_gate_desc(1, x.kind, x.target, x.ctrl, x.angle);
+        gates = r.data();
+    }
+    const std::vector<GateDesc> f = fold_diagonals(gates, count);
+    if (arith == ARITH_FF) return defer_scale<ff::f2>(f.data(), f.size(), true);
+    return arith == ARITH_F64 ? defer_scale<double>(f.data(), f.size(), true)
+                              : defer_scale<float>(f.data(), f.size(), true);
+}
+
 // The gate list as the fused sweeps of a handle run it (folded, factors
 // deferred); the handle's state is at least one tile.
 static std::vector<GateDesc> rewritten(const Sim &s, const GateDesc *gates, size_t count) {
@@ -720,16 +734,7 @@ static std::vector<GateDesc> rewritten(const Sim &s, const GateDesc *gates, size
         if (ff_capable(s)) return defer_scale<ff::f2>(gates, count, false);
         return std::vector<GateDesc>(gates, gates + count);
     }
-    std::vector<GateDesc> r;
-    if (!s.prec) {  // complex64: constants in binary64 from the angles
-        r.assign(gates, gates + count);
-        for (GateDesc &x : r)
-            if (x.kind <= G_RZ) x = make_gate_desc(1, x.kind, x.target, x.ctrl, x.angle);
-        gates = r.data();
-    }
-    const std::vector<GateDesc> f = fold_diagonals(gates, count);
-    if (ff_capable(s)) return defer_scale<ff::f2>(f.data(), f.size(), true);
-    return s.prec ? defer_scale<double>(f.data(), f.size(), true) : defer_scale<float>(f.data(), f.size(), true);
+    return defer_factors(ff_capable(s) ? ARITH_FF : (s.prec ? ARITH_F64 : ARITH_C64), gates, count);
 }
 
 std::vector<const void *> specialised_kernels(Sim &s, const std::vector<std::string> &srcs, const char *entry,

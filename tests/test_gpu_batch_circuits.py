@@ -81,3 +81,24 @@ def test_batch_edge_cases():
     with pytest.raises(KbwgError) as e:
         batch_circuits_exp_value([(3, [], [(1.0, [(C.PAULI_Z, 1), (C.PAULI_X, 1)])])])
     assert e.value.code == N.EINVAL
+
+
+@pytest.mark.parametrize("prec,fast,tol", [("c128", True, 1e-10), ("c128", False, 1e-10), ("c64", False, 5e-5)])
+def test_parts_of_large_circuits(prec, fast, tol):
+    # registers one and two qubits above a tile, several parts per sweep, no
+    # gates, no strings, strings too wide for a tile, one circuit alone
+    rng = np.random.default_rng(11)
+    circs = []
+    for n in (11, 12, 13, 14, 17, 18):
+        wide = [(0.4, [(C.PAULI_X, q) for q in range(n)]), (-0.7, [(C.PAULI_Y, q) for q in range(n)])]
+        circs.append((n, C.random_circuit(n, 12 * n, 60 + n, max_controls=2), C.tfim_ring(n) + wide))
+        circs.append((n, [], random_hamiltonian(n, rng) + wide))
+        circs.append((n, C.random_circuit(n, 30, 90 + n), []))
+    want = []
+    for n, g, h in circs:
+        o = oracle.OracleDense(n, "c128")
+        o.apply(g)
+        want.append(o.pauli_expect(h))
+    assert np.abs(batch_circuits_exp_value(circs, prec=prec, fast_c128=fast) - want).max() < tol
+    for i in (0, 12, 13, 15):
+        assert abs(batch_circuits_exp_value(circs[i: i + 1], prec=prec, fast_c128=fast)[0] - want[i]) < tol
