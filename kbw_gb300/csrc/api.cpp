@@ -639,8 +639,8 @@ static int32_t parse_hamiltonian(uint32_t n, const uint8_t *paulis, const uintpt
 // float-float resident form as is: the diagonal groups (x = 0) and the tiled
 // pair passes (no string too wide for a tile).
 static bool exp_reads_ff(const Sim &s, const std::vector<PauliString> &strs) {
-    const int K = pauli_tile_bits<double>();
-    if (s.n < (uint32_t)K) return false;
+    const int K = std::min<int>(pauli_tile_bits<double>(), (int)s.n);
+    if (K < kPauliMinBits) return false;
     std::vector<uint64_t> xm;
     for (const PauliString &t : strs)
         if (t.x != 0) xm.push_back(t.x);
@@ -658,7 +658,8 @@ static cudaError_t settle_for_exp(Sim &s, const std::vector<PauliString> &strs) 
     return cudaSuccess;
 }
 
-static int32_t exp_value_core(kbwg_sim *s, const std::vector<PauliString> &strs, double *out) {
+// <P_k> of every string, without its coefficient.
+static int32_t exp_strings(kbwg_sim *s, const std::vector<PauliString> &strs, std::vector<double> &vals) {
     const bool ff = s->ff_resident;  // (settle_for_exp left it so only when every kernel below reads that form)
     const size_t n_strings = strs.size();
     std::vector<size_t> order(n_strings);
@@ -676,8 +677,8 @@ static int32_t exp_value_core(kbwg_sim *s, const std::vector<PauliString> &strs,
     };
     // strings with a flip mask: tiled passes, each covering every string whose
     // flip mask fits one tile (ring TFIM, 30 qubits: 4 passes instead of 30)
-    const int K = s->prec ? pauli_tile_bits<double>() : pauli_tile_bits<float>();
-    const bool tiled = s->n >= (uint32_t)K;
+    const int K = std::min<int>(s->prec ? pauli_tile_bits<double>() : pauli_tile_bits<float>(), (int)s->n);
+    const bool tiled = K >= kPauliMinBits;
     std::vector<char> by_tile(n_strings, 0);
     if (tiled) {
         std::vector<size_t> pair_idx;
@@ -695,26 +696,61 @@ static int32_t exp_value_core(kbwg_sim *s, const std::vector<PauliString> &strs,
             pass.l = pp.l;
             pass.m = pp.m;
             memcpy(pass.hq, pp.hq, sizeof pass.hq);
+            // windows of three tile bits: the one that holds the most strings
+            // left, until no string fits one
+            std::vector<uint32_t> win(pp.members.size(), kPauliNoWindow);
+            for (;;) {
+                uint32_t best = 0, best_w = 0;
+                for (uint32_t w = 0; w + 3 <= (uint32_t)K; w++) {
+                    uint32_t c = 0;
+                    for (size_t j = 0; j < pp.members.size(); j++)
+                        if (win[j] == kPauliNoWindow && !(pp.local(strs[pair_idx[pp.members[j]]].x) & ~(7u << w))) c++;
+                    if (c > best) best = c, best_w = w;
+                }
+                if (!best) break;
+                for (size_t j = 0; j < pp.members.size(); j++)
+                    if (win[j] == kPauliNoWindow && !(pp.local(strs[pair_idx[pp.members[j]]].x) & ~(7u << best_w)))
+                        win[j] = best_w;
+            }
+            std::vector<size_t> ord(pp.members.size());
+            for (size_t j = 0; j < ord.size(); j++) ord[j] = j;
+            std::stable_sort(ord.begin(), ord.end(), [&](size_t a, size_t b) {
+                const PauliString &x = strs[pair_idx[pp.members[a]]], &y = strs[pair_idx[pp.members[b]]];
+                if (win[a] != win[b]) return win[a] < win[b];
+                const uint32_t u = pp.local(x.x), v = pp.local(y.x);
+                return u != v ? u < v : (x.ny & 1) < (y.ny & 1);
+            });
             std::vector<size_t> take;
-            for (size_t j = 0; j < pp.members.size(); j++) {
-                const size_t k = pair_idx[pp.members[j]];
+            for (size_t j = 0; j < ord.size(); j++) {
+                const size_t k = pair_idx[pp.members[ord[j]]];
                 const PauliString &t = strs[k];
                 PauliTileTerm &tt = pass.t[j];
                 tt.xl = pp.local(t.x);
                 tt.hb = 31 - __builtin_clz(tt.xl);
                 tt.zl = pp.local(t.z & pp.tile_mask);
                 tt.zo = t.z & ~pp.tile_mask;
+                tt.w = win[ord[j]];
                 pair_term(t, tt.factor, tt.im);
                 take.push_back(k);
                 by_tile[k] = 1;
             }
+            for (size_t j = take.size(); j-- > 0;) {
+                PauliTileTerm &tt = pass.t[j];
+                const bool last = j + 1 == take.size();
+                const bool same_w = !last && pass.t[j + 1].w == tt.w;
+                const bool same_g = same_w && pass.t[j + 1].xl == tt.xl && pass.t[j + 1].im == tt.im;
+                tt.window_end = same_w ? pass.t[j + 1].window_end : (uint32_t)j + 1;
+                tt.group_end = same_g ? pass.t[j + 1].group_end : (uint32_t)j + 1;
+                if (tt.w != kPauliNoWindow)
+                    tt.groups = (same_w ? pass.t[j + 1].groups : 0u) | (1u << (2 * (tt.xl >> tt.w) + tt.im));
+            }
             pass.nterms = (uint32_t)take.size();
+            ReduceScratch rs = s->rs;
+            rs.result = d_vals + slot_of.size();
             CUDA_TRY(dispatch(s, [&](auto *tp) {
                 using T = std::remove_pointer_t<decltype(tp)>;
-                return launch_pauli_tile<T>(s->state, s->n, ff, pass, s->rs, s->stream);
+                return launch_pauli_tile<T>(s->state, s->n, ff, pass, rs, s->d_err, s->stream);
             }));
-            CUDA_TRY(cudaMemcpyAsync(d_vals + slot_of.size(), s->rs.result, take.size() * 8,
-                                     cudaMemcpyDeviceToDevice, s->stream));
             slot_of.insert(slot_of.end(), take.begin(), take.end());
         }
     }
@@ -741,20 +777,29 @@ static int32_t exp_value_core(kbwg_sim *s, const std::vector<PauliString> &strs,
             i++;
         }
         g.nterms = (uint32_t)idx.size();
+        ReduceScratch rs = s->rs;
+        rs.result = d_vals + slot_of.size();
         CUDA_TRY(dispatch(s, [&](auto *tp) {
             using T = std::remove_pointer_t<decltype(tp)>;
-            return launch_pauli_group<T>(s->state, s->n, g, s->rs, s->stream, ff);
+            return launch_pauli_group<T>(s->state, s->n, g, rs, s->stream, ff);
         }));
-        CUDA_TRY(cudaMemcpyAsync(d_vals + slot_of.size(), s->rs.result, idx.size() * 8, cudaMemcpyDeviceToDevice,
-                                 s->stream));
         slot_of.insert(slot_of.end(), idx.begin(), idx.end());
     }
-    std::vector<double> grouped(n_strings + 1), vals(n_strings + 1);
+    std::vector<double> grouped(n_strings + 1);
+    vals.assign(n_strings, 0.0);
     if (n_strings) CUDA_TRY(copy_async(grouped.data(), d_vals, n_strings * 8, cudaMemcpyDeviceToHost, s->stream));
-    CUDA_TRY(cudaStreamSynchronize(s->stream));
+    const int32_t rc = check_device_error(s);  // (waits for the stream)
+    if (rc != KBWG_OK) return rc;
     for (size_t j = 0; j < n_strings; j++) vals[slot_of[j]] = grouped[j];
+    return KBWG_OK;
+}
+
+static int32_t exp_value_core(kbwg_sim *s, const std::vector<PauliString> &strs, double *out) {
+    std::vector<double> vals;
+    const int32_t rc = exp_strings(s, strs, vals);
+    if (rc != KBWG_OK) return rc;
     double total = 0.0;  // sum in string order, as the reference's zip/map/sum
-    for (size_t k = 0; k < n_strings; k++) total += vals[k] * strs[k].coef;
+    for (size_t k = 0; k < strs.size(); k++) total += vals[k] * strs[k].coef;
     *out = total;
     return KBWG_OK;
 }
@@ -1307,13 +1352,28 @@ int32_t kbwg_batch_exp_value(uintptr_t num_qubits, int32_t precision, uint32_t f
     int32_t rc = pool_get(num_qubits, precision, flags, &L.sim, &L.pooled);
     if (rc != KBWG_OK) return rc;
     rc = kbwg_apply_gates(L.sim, gates, n_gates);
-    for (uintptr_t k = 0; rc == KBWG_OK && k < n_hamiltonians; k++) {
-        const uintptr_t a = ham_offsets[k];
-        rc = kbwg_exp_value(L.sim, paulis, qubits, offsets ? offsets + a : nullptr,
-                            coefficients ? coefficients + a : nullptr, ham_offsets[k + 1] - a, &out[k]);
+    if (rc != KBWG_OK) return rc;
+    if (!n_hamiltonians) return kbwg_flush(L.sim);
+    // the strings of all Hamiltonians share the passes over the state and one
+    // read-back (a pass and a synchronisation per Hamiltonian took twice the
+    // circuit's own time on 14 qubits)
+    const uintptr_t a = ham_offsets[0], count = ham_offsets[n_hamiltonians] - a;
+    std::vector<PauliString> strs;
+    rc = parse_hamiltonian(L.sim->n, paulis, qubits, offsets ? offsets + a : nullptr,
+                           coefficients ? coefficients + a : nullptr, count, strs);
+    if (rc != KBWG_OK) return rc;
+    kbwg_sim *s = L.sim;
+    ENTER(s);
+    CUDA_TRY(settle_for_exp(*s, strs));
+    std::vector<double> vals;
+    rc = exp_strings(s, strs, vals);
+    if (rc != KBWG_OK) return rc;
+    for (uintptr_t k = 0; k < n_hamiltonians; k++) {
+        double total = 0.0;  // in string order
+        for (uintptr_t j = ham_offsets[k] - a; j < ham_offsets[k + 1] - a; j++) total += vals[j] * strs[j].coef;
+        out[k] = total;
     }
-    if (rc == KBWG_OK && !n_hamiltonians) rc = kbwg_flush(L.sim);
-    return rc;
+    return KBWG_OK;
     GUARD_END
 }
 

@@ -101,19 +101,25 @@ struct PauliTileTerm {
     uint64_t zo;    // phase mask on qubits outside the tile
     uint32_t hb;    // highest local bit of xl: each pair is visited with it clear
     uint32_t im;    // Im(conj(a_s) a_{s^x}) instead of Re
+    uint32_t w;           // first bit of the three-bit window that holds xl, or kPauliNoWindow
+    uint32_t group_end;   // end of the strings with this flip mask and part (and window)
+    uint32_t window_end;  // end of the window's strings
+    uint32_t groups;      // bit 2 x + im: the window has strings with flip mask x (of its bits) and that part
     double factor;  // +-2 (i^{nY} and (-1)^{|x & z|} folded in)
 };
+constexpr uint32_t kPauliNoWindow = 99;
 struct PauliTilePass {
     uint32_t K, l, m, nterms;
     uint8_t hq[16];
-    PauliTileTerm t[kMaxTerms];
+    PauliTileTerm t[kMaxTerms];  // window by window, then the rest; by flip mask and part (im)
 };
-// Tile size of the pass kernel (32 KiB of shared memory: several CTAs per SM
-// overlap one tile's loads with another's arithmetic).
+// Largest tile of the pass kernel: two buffers of 32 KiB, three CTAs per SM.
+// Registers down to kPauliMinBits qubits are one tile of their own size.
 template <class T> constexpr int pauli_tile_bits() { return sizeof(T) == 4 ? 12 : 11; }
+constexpr int kPauliMinBits = 9;
 template <class T>
 cudaError_t launch_pauli_tile(const void *st, uint32_t n, bool ff_resident, const PauliTilePass &p,
-                              const ReduceScratch &rs, cudaStream_t s);
+                              const ReduceScratch &rs, int *err, cudaStream_t s);
 
 // dump: support counts per block, then compaction.
 struct DumpSpec {

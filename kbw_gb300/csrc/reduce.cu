@@ -15,6 +15,7 @@
 #include "../../include/kbwg.h"
 #include "ff.cuh"
 #include "kernels.h"
+#include "sweep_dev.cuh"
 
 namespace kbwg {
 
@@ -120,6 +121,55 @@ __device__ double sum_partials(const double *partials, int nblocks, int stride, 
     double v = 0.0;
     for (int b = threadIdx.x; b < nblocks; b += blockDim.x) v += partials[(size_t)b * stride + k];
     return block_sum(v);
+}
+
+// Sums of up to 32 terms at once.  v[k]: this thread's share of term k; lane k
+// returns the warp's sum of term k.  Halving exchange: 31 float-float additions
+// instead of 5 per term, and no FP64 instruction: a double tree over 32 terms
+// took 19 us of a 25 us launch on GB300's FP64 pipe.
+__device__ __forceinline__ ff::f2 warp_sum_terms(ff::f2 (&v)[kMaxTerms]) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int w = 16; w > 0; w >>= 1) {
+        const bool up = (lane & w) != 0;
+#pragma unroll
+        for (int i = 0; i < w; i++) {
+            const ff::f2 keep = up ? v[i + w] : v[i], send = up ? v[i] : v[i + w];
+            const ff::f2 got{__shfl_xor_sync(0xffffffffu, send.h, w), __shfl_xor_sync(0xffffffffu, send.l, w)};
+            v[i] = ff::add(keep, got);
+        }
+    }
+    return v[0];
+}
+
+// The grid's sums of nt terms into rs.result: lane k of every warp holds its
+// warp's sum of term k.  Fixed order (warps, then blocks by warp of the last
+// block), so deterministic.  256 threads; every thread calls it.
+__device__ void finish_terms(double v, uint32_t nt, const ReduceScratch &rs) {
+    __shared__ double sh[kReduceThreads / 32][32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    __syncthreads();
+    sh[w][lane] = v;
+    __syncthreads();
+    if (w == 0 && lane < (int)nt) {
+        double t = 0.0;
+        for (int j = 0; j < kReduceThreads / 32; j++) t += sh[j][lane];
+        rs.partials[(size_t)blockIdx.x * kMaxTerms + lane] = t;
+    }
+    if (last_block(rs.ticket)) {
+        double t = 0.0;
+        if (lane < (int)nt)
+            for (unsigned b = (unsigned)w; b < gridDim.x; b += kReduceThreads / 32)
+                t += __ldcg(rs.partials + (size_t)b * kMaxTerms + lane);
+        sh[w][lane] = t;
+        __syncthreads();
+        if (w == 0 && lane < (int)nt) {
+            double r = 0.0;
+            for (int j = 0; j < kReduceThreads / 32; j++) r += sh[j][lane];
+            rs.result[lane] = r;
+        }
+        if (threadIdx.x == 0) *rs.ticket = 0;
+    }
 }
 
 __device__ __forceinline__ uint64_t insert_zero(uint64_t i, uint32_t m) {
@@ -670,20 +720,7 @@ __global__ void __launch_bounds__(kReduceThreads, 2)
         }
         __syncwarp();
     }
-#pragma unroll
-    for (int k = 0; k < kMaxTerms; k++) {
-        if (k < (int)nt) {
-            const double v = block_sum(A::to_d(acc[k]));
-            if (threadIdx.x == 0) rs.partials[(size_t)blockIdx.x * kMaxTerms + k] = v;
-        }
-    }
-    if (last_block(rs.ticket)) {
-        for (int k = 0; k < (int)nt; k++) {
-            const double t = sum_partials(rs.partials, gridDim.x, kMaxTerms, k);
-            if (threadIdx.x == 0) rs.result[k] = t;
-        }
-        if (threadIdx.x == 0) *rs.ticket = 0;
-    }
+    finish_terms(A::to_d(warp_sum_terms(acc)), nt, rs);
 }
 
 template <class T>
@@ -692,13 +729,16 @@ cudaError_t launch_pauli_group(const void *st, uint32_t n, const PauliGroup &g, 
     if (ff_resident && !(sizeof(T) == 8 && g.x == 0 && (1ull << n) >= (uint64_t)kDiagWarpSpan))
         return cudaErrorInvalidValue;  // (only the diagonal form reads the float-float resident state)
     if (g.x == 0 && (1ull << n) >= (uint64_t)kDiagWarpSpan) {
+        // no block without a run of amplitudes: their tails would only queue up
+        const uint64_t want = ((1ull << n) / kDiagWarpSpan + kReduceThreads / 32 - 1) / (kReduceThreads / 32);
+        const unsigned grid = (unsigned)std::min<uint64_t>(want, (uint64_t)kReduceBlocks);
         if constexpr (sizeof(T) == 8) {
             if (ff_resident)
-                k_pauli_diag<T, true><<<kReduceBlocks, kReduceThreads, 0, s>>>(st, n, g, rs);
+                k_pauli_diag<T, true><<<grid, kReduceThreads, 0, s>>>(st, n, g, rs);
             else
-                k_pauli_diag<T, false><<<kReduceBlocks, kReduceThreads, 0, s>>>(st, n, g, rs);
+                k_pauli_diag<T, false><<<grid, kReduceThreads, 0, s>>>(st, n, g, rs);
         } else {
-            k_pauli_diag<T, false><<<kReduceBlocks, kReduceThreads, 0, s>>>(st, n, g, rs);
+            k_pauli_diag<T, false><<<grid, kReduceThreads, 0, s>>>(st, n, g, rs);
         }
     } else {
         k_pauli_group<T><<<kReduceBlocks, kReduceThreads, 0, s>>>((const cx<T> *)st, n, g, rs);
@@ -708,151 +748,273 @@ cudaError_t launch_pauli_group(const void *st, uint32_t n, const PauliGroup &g, 
 }
 
 // ---- tiled pass over many pair-form strings ---------------------------------------
-// One tile of 2^K amplitudes per CTA iteration, staged in shared memory with
-// coalesced loads (chunks of 2^l contiguous amplitudes); every term then
-// visits its 2^(K-1) pairs inside the tile.  complex64: exact float products
-// summed in float-float (AccF) per thread.  complex128: the tile is held in
-// float-float form (binary64 split on load, or the float-float resident
-// form as is), each pair product is a float-float dot product, summed per
-// tile in float-float and added to a binary64 accumulator once per tile.
-template <class T> struct TileVal;
-template <> struct TileVal<float> {
-    using V = cx<float>;
-};
-template <> struct TileVal<double> {
-    struct V {
-        ff::f2 re, im;
-    };
-};
-
+// One tile of 2^K amplitudes (32 KiB, TMA) per CTA iteration, three CTAs per SM
+// that overlap one's load with the others' sums.  (Two buffers per CTA leave
+// the running sums too little L1: 5.7 -> 6.6 ms on the case below.)  An
+// amplitude's (re, im) is one packed operand: a pair's product is an f32x2
+// multiplication whose lanes (re re and im im, or re im and im re) are summed
+// apart until the end, so 12 packed instructions form and add one pair.
+// A product is its rounded high part plus the exact error and the cross terms
+// (complex128: the tile holds float-float amplitudes, binary64 split once per
+// tile); it is added without normalising (TwoSum of the high parts, errors
+// into the low one).
+// Strings whose flips lie within three neighbouring tile bits run in windows:
+// a thread holds the 8 amplitudes of its window in registers, read once for
+// all strings of the window, and a pair is two registers.  Lane l takes the
+// amplitudes in the order j ^ (l >> w) below bit 3, so the reads spread over
+// the banks; the flip mask still pairs j with j ^ x.  Other strings read both
+// amplitudes of every pair.  Strings with one flip mask and part (Re or Im)
+// form a group: the products are formed once and every string adds them with
+// its signs.
+// Tile sums gather in float-float and go to binary64 every kPauliFlush tiles:
+// a conversion per string and tile kept GB300's FP64 pipe busy half of the
+// time.
+// Measured, the 27 X strings of a ring TFIM on 27 qubits in float-float, four
+// passes: 5.8 -> 4.0 ms (a pass that only reads: 0.38 ms).
 __device__ __forceinline__ uint64_t tile_base_of(uint64_t tau, uint32_t l, uint32_t m, const uint8_t *hq) {
     uint64_t b = tau << l;
     for (uint32_t j = 0; j < m; j++) b = insert_zero(b, hq[j]);
     return b;
 }
 
+constexpr int kPauliThreads = kReduceThreads, kPauliFlush = 32;
+
+__device__ __forceinline__ float2 flip_signs(float2 v, uint32_t s) {
+    return make_float2(__uint_as_float(__float_as_uint(v.x) ^ s), __uint_as_float(__float_as_uint(v.y) ^ s));
+}
+template <bool FFV>
+__device__ __forceinline__ ff2::v2 pauli_amp(const void *tile, uint32_t u) {
+    ff2::v2 a{};
+    if constexpr (FFV) a = reinterpret_cast<const ff2::v2 *>(tile)[u];
+    else a.h = reinterpret_cast<const float2 *>(tile)[u];
+    return a;
+}
+// conj(a) b as h + l, lane by lane: Re = re re + im im, Im = re im - im re (the
+// lanes' difference; one scalar instruction per lane, no exchanged operands)
+template <bool FFV, bool IM>
+__device__ __forceinline__ ff2::v2 pauli_product(const ff2::v2 &a, const ff2::v2 &b) {
+    if constexpr (IM) {
+        const float2 p = make_float2(__fmul_rn(a.h.x, b.h.y), __fmul_rn(a.h.y, b.h.x));
+        float2 lo = make_float2(__fmaf_rn(a.h.x, b.h.y, -p.x), __fmaf_rn(a.h.y, b.h.x, -p.y));
+        if constexpr (FFV) {
+            lo = make_float2(__fmaf_rn(a.h.x, b.l.y, lo.x), __fmaf_rn(a.h.y, b.l.x, lo.y));
+            lo = make_float2(__fmaf_rn(a.l.x, b.h.y, lo.x), __fmaf_rn(a.l.y, b.h.x, lo.y));
+        }
+        return ff2::v2{p, lo};
+    }
+    const float2 p = ff2::mul(a.h, b.h);
+    float2 lo = ff2::fma(a.h, b.h, flip_signs(p, 0x80000000u));
+    if constexpr (FFV) lo = ff2::fma(a.l, b.h, ff2::fma(a.h, b.l, lo));
+    return ff2::v2{p, lo};
+}
+__device__ __forceinline__ void pauli_add(ff2::v2 &S, float2 p, float2 lo) {
+    const ff2::v2 t = ff2::two_sum(S.h, p);
+    S = ff2::v2{t.h, ff2::add(S.l, ff2::add(t.l, lo))};
+}
+// a thread's sum over the tile, its lanes joined, into the string's running sum (both unnormalised)
+template <bool IM>
+__device__ __forceinline__ void pauli_tail(const ff2::v2 &S, bool neg, ff::f2 &acc) {
+    const float sn = neg ? -1.f : 1.f, sy = IM ? -sn : sn;
+    const ff::f2 t = ff::two_sum(__fmul_rn(S.h.x, sn), __fmul_rn(S.h.y, sy)), r = ff::two_sum(acc.h, t.h);
+    const float l = __fmaf_rn(S.l.x, sn, __fmul_rn(S.l.y, sy));
+    acc = ff::f2{r.h, ff::add(acc.l, ff::add(ff::add(r.l, t.l), l))};
+}
+
+// The strings of one window with flip mask X and part IM: the four products,
+// then every string's signed sum.
+template <bool FFV, bool IM, int X>
+__device__ __forceinline__ void window_group(const PauliTilePass &p, const ff2::v2 (&a)[8], uint32_t &k, uint32_t w,
+                                             uint32_t F, uint32_t negs, uint32_t signs, ff::f2 *acc) {
+    constexpr int hb = X >= 4 ? 2 : (X >= 2 ? 1 : 0);
+    ff2::v2 c[4];
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const int j = ((i >> hb) << (hb + 1)) | (i & ((1 << hb) - 1));
+        c[i] = pauli_product<FFV, IM>(a[j], a[j ^ X]);
+    }
+    const uint32_t end = p.t[k].group_end;
+#pragma unroll 1
+    for (; k < end; k++) {
+        ff2::v2 S = c[0];
+        bool neg = ((negs >> k) & 1u) != 0;
+        if ((signs >> k) & 1u) {
+            const uint32_t zl = p.t[k].zl, zr = zl >> w;
+            neg ^= (__popc(F & zl) & 1) != 0;
+#pragma unroll
+            for (int i = 1; i < 4; i++) {  // (j = 0 has no sign of its own)
+                const uint32_t j = ((i >> hb) << (hb + 1)) | (i & ((1 << hb) - 1));
+                const uint32_t sg = (uint32_t)__popc(j & zr) << 31;
+                pauli_add(S, flip_signs(c[i].h, sg), flip_signs(c[i].l, sg));
+            }
+        } else {
+#pragma unroll
+            for (int i = 1; i < 4; i++) pauli_add(S, c[i].h, c[i].l);
+        }
+        pauli_tail<IM>(S, neg, acc[k]);
+    }
+}
+
+// Every string of one window, terms from k0.  Bit k of negs: the parity of
+// string k's phase mask on the tile's base; of signs: string k has phases
+// inside the tile.
+template <bool FFV>
+__device__ __forceinline__ void pauli_window(const PauliTilePass &p, const void *tile, uint32_t k0, uint32_t negs,
+                                             uint32_t signs, ff::f2 *acc) {
+    const uint32_t w = p.t[k0].w, low = (1u << w) - 1u, groups = p.t[k0].groups;
+    for (uint32_t q = threadIdx.x; q < (1u << (p.K - 3)); q += kPauliThreads) {
+        const uint32_t sw = w < 3 ? ((threadIdx.x & 31u) >> w) & 7u : 0u;
+        const uint32_t F = (q & low) | ((q & ~low) << 3) | (sw << w);
+        ff2::v2 a[8];
+#pragma unroll
+        for (int j = 0; j < 8; j++) a[j] = pauli_amp<FFV>(tile, F ^ ((uint32_t)j << w));
+        uint32_t k = k0;
+#define KBWG_WX(X)                                                                                    \
+    if (groups & (1u << (2 * X))) window_group<FFV, false, X>(p, a, k, w, F, negs, signs, acc); \
+    if (groups & (2u << (2 * X))) window_group<FFV, true, X>(p, a, k, w, F, negs, signs, acc);
+        KBWG_WX(1) KBWG_WX(2) KBWG_WX(3) KBWG_WX(4) KBWG_WX(5) KBWG_WX(6) KBWG_WX(7)
+#undef KBWG_WX
+    }
+}
+
+// C strings k0.. of one group over the tile, both amplitudes of a pair read.
+template <bool FFV, bool IM, int C>
+__device__ __forceinline__ void pauli_group_terms(const PauliTilePass &p, const void *tile, uint32_t k0, uint32_t negs,
+                                                  ff::f2 *acc) {
+    const uint32_t xl = p.t[k0].xl, pairs = 1u << (p.K - 1);
+    const uint32_t keep = (1u << p.t[k0].hb) - 1u;
+    ff2::v2 S[C];
+    uint32_t zl[C];
+#pragma unroll
+    for (int c = 0; c < C; c++) {
+        S[c] = ff2::v2{make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+        zl[c] = p.t[k0 + c].zl;
+    }
+#pragma unroll 4
+    for (uint32_t q = threadIdx.x; q < pairs; q += kPauliThreads) {
+        const uint32_t u = q + (q & ~keep);  // the highest flipped bit clear
+        const ff2::v2 w = pauli_product<FFV, IM>(pauli_amp<FFV>(tile, u), pauli_amp<FFV>(tile, u ^ xl));
+#pragma unroll
+        for (int c = 0; c < C; c++) {
+            const uint32_t sg = (uint32_t)__popc(u & zl[c]) << 31;
+            pauli_add(S[c], flip_signs(w.h, sg), flip_signs(w.l, sg));
+        }
+    }
+#pragma unroll
+    for (int c = 0; c < C; c++) pauli_tail<IM>(S[c], ((negs >> (k0 + c)) & 1u) != 0, acc[k0 + c]);
+}
+
+template <bool FFV, bool IM>
+__device__ __forceinline__ void pauli_group(const PauliTilePass &p, const void *tile, uint32_t k0, uint32_t k1,
+                                            uint32_t negs, ff::f2 *acc) {
+    for (; k0 + 2 <= k1; k0 += 2) pauli_group_terms<FFV, IM, 2>(p, tile, k0, negs, acc);
+    if (k0 < k1) pauli_group_terms<FFV, IM, 1>(p, tile, k0, negs, acc);
+}
+
 template <class T, bool kFF>
-__global__ void __launch_bounds__(256) k_pauli_tile(const void *__restrict__ st, uint32_t n,
-                                                    const __grid_constant__ PauliTilePass p, ReduceScratch rs) {
-    using V = typename TileVal<T>::V;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    V *tile = reinterpret_cast<V *>(smem_raw);
+__global__ void __launch_bounds__(kPauliThreads, 3) k_pauli_tile(const void *__restrict__ st, uint32_t n,
+                                                                 const __grid_constant__ PauliTilePass p,
+                                                                 ReduceScratch rs, int *err) {
+    constexpr bool FFV = sizeof(T) == 8;
+    constexpr uint32_t kElem = FFV ? 16 : 8;
+    extern __shared__ __align__(128) unsigned char smem_raw[];
     const uint32_t K = p.K, l = p.l, m = p.m, nt = p.nterms;
-    uint64_t *chunk_off = reinterpret_cast<uint64_t *>(smem_raw + (sizeof(V) << K));
+    const uint32_t N = 1u << K, tile_bytes = kElem << K;
+    uint64_t *chunk_off = reinterpret_cast<uint64_t *>(smem_raw + tile_bytes);
+    uint64_t *bar = chunk_off + (1u << m);
     for (uint32_t c = threadIdx.x; c < (1u << m); c += blockDim.x) {
         uint64_t off = 0;
         for (uint32_t j = 0; j < m; j++) off |= (uint64_t)((c >> j) & 1u) << p.hq[j];
         chunk_off[c] = off;
     }
+    if (threadIdx.x == 0) {
+        mbar_init(bar, 1);
+        fence_mbar_init();
+    }
     const uint64_t tiles = 1ull << (n - K);
-    const uint32_t lowmask = (1u << l) - 1u;
-    const uint32_t npairs = 1u << (K - 1);
-    typename AccOf<T>::type acc[kMaxTerms];
+    ff::f2 acc[kMaxTerms];  // (local memory, touched once per string and tile)
+    double wide[kMaxTerms];
+    bool flushed = false;
+    for (int k = 0; k < kMaxTerms; k++) acc[k] = ff::f2{0.f, 0.f};
     __syncthreads();
-    for (uint64_t tau = blockIdx.x; tau < tiles; tau += gridDim.x) {
+    auto issue_load = [&](uint64_t tau) {
+        if (threadIdx.x < 32) {
+            const uint64_t base = tile_base_of(tau, l, m, p.hq);
+            if (threadIdx.x == 0) mbar_expect_tx(bar, tile_bytes);
+            __syncwarp();
+            for (uint32_t c = threadIdx.x; c < (1u << m); c += 32)
+                tma_load(smem_raw + ((size_t)(c << l) * kElem), (const char *)st + (base + chunk_off[c]) * kElem,
+                         kElem << l, bar);
+        }
+    };
+    if (blockIdx.x < tiles) issue_load(blockIdx.x);
+    // lane k keeps string k's phase mask outside the tile
+    const uint32_t my = threadIdx.x & 31u;
+    const uint64_t my_zo = my < nt ? p.t[my].zo : 0ull;
+    const uint32_t signs = __ballot_sync(0xffffffffu, my < nt && p.t[my].zl != 0u);
+    uint32_t it = 0;
+    for (uint64_t tau = blockIdx.x; tau < tiles; tau += gridDim.x, it++) {
         const uint64_t base = tile_base_of(tau, l, m, p.hq);
-        for (uint32_t u = threadIdx.x; u < (1u << K); u += blockDim.x) {
-            const uint64_t gidx = base + chunk_off[u >> l] + (u & lowmask);
-            if constexpr (sizeof(T) == 4) {
-                tile[u] = reinterpret_cast<const cx<float> *>(st)[gidx];
-            } else if constexpr (kFF) {
-                const float4 f = reinterpret_cast<const float4 *>(st)[gidx];  // re.hi, im.hi, re.lo, im.lo
-                tile[u] = V{ff::f2{f.x, f.z}, ff::f2{f.y, f.w}};
-            } else {
-                const cx<double> a = reinterpret_cast<const cx<double> *>(st)[gidx];
-                tile[u] = V{ff::from_double(a.re), ff::from_double(a.im)};
+        void *tile = smem_raw;
+        const uint32_t negs = __ballot_sync(0xffffffffu, (__popcll(base & my_zo) & 1) != 0);
+        if (!tile_wait(bar, it & 1u, err)) break;  // (the sums are not valid; the ticket still counts)
+        if constexpr (FFV && !kFF) {
+            for (uint32_t u = threadIdx.x; u < N; u += kPauliThreads) {
+                const cx<double> a = reinterpret_cast<const cx<double> *>(tile)[u];
+                const ff::f2 r = ff::from_double(a.re), i = ff::from_double(a.im);
+                reinterpret_cast<ff2::v2 *>(tile)[u] = ff2::v2{make_float2(r.h, i.h), make_float2(r.l, i.l)};
             }
+            __syncthreads();
         }
-        __syncthreads();
-        // (not unrolled: one copy of the pair loop; acc[] lives in local
-        // memory, touched once per term and tile)
 #pragma unroll 1
-        for (int k = 0; k < (int)nt; k++) {
-            const PauliTileTerm &t = p.t[k];
-            const uint32_t tile_par = (uint32_t)__popcll(base & t.zo) & 1u;
-            // four independent partial sums per thread (the pair products are
-            // independent; one running sum would serialise its rounding chain)
-            constexpr int U = 4;
-            if constexpr (sizeof(T) == 4) {
-                AccF part[U];
-                for (uint32_t q0 = threadIdx.x; q0 < npairs; q0 += U * blockDim.x) {
-#pragma unroll
-                    for (int j = 0; j < U; j++) {
-                        const uint32_t q = q0 + j * blockDim.x;
-                        if (q >= npairs) break;
-                        const uint32_t u = (uint32_t)insert_zero(q, t.hb);
-                        const cx<float> a = tile[u], b = tile[u ^ t.xl];
-                        const bool neg = ((__popc(u & t.zl) & 1u) ^ tile_par) != 0;
-                        if (!t.im) {  // Re(conj(a) b) = a.re b.re + a.im b.im
-                            if (neg) {
-                                part[j].add_prod_neg(a.re, b.re);
-                                part[j].add_prod_neg(a.im, b.im);
-                            } else {
-                                part[j].add_prod(a.re, b.re);
-                                part[j].add_prod(a.im, b.im);
-                            }
-                        } else {  // Im(conj(a) b) = a.re b.im - a.im b.re
-                            if (neg) {
-                                part[j].add_prod_neg(a.re, b.im);
-                                part[j].add_prod(a.im, b.re);
-                            } else {
-                                part[j].add_prod(a.re, b.im);
-                                part[j].add_prod_neg(a.im, b.re);
-                            }
-                        }
-                    }
-                }
-#pragma unroll
-                for (int j = 0; j < U; j++) acc[k].add2(part[j].hi, part[j].lo);
+        for (uint32_t k0 = 0; k0 < nt;) {
+            if (p.t[k0].w < 32u) {
+                pauli_window<FFV>(p, tile, k0, negs, signs, acc);
+                k0 = p.t[k0].window_end;
             } else {
-                ff::f2 part[U];
-#pragma unroll
-                for (int j = 0; j < U; j++) part[j] = ff::f2{0.f, 0.f};
-                for (uint32_t q0 = threadIdx.x; q0 < npairs; q0 += U * blockDim.x) {
-#pragma unroll
-                    for (int j = 0; j < U; j++) {
-                        const uint32_t q = q0 + j * blockDim.x;
-                        if (q >= npairs) break;
-                        const uint32_t u = (uint32_t)insert_zero(q, t.hb);
-                        const V a = tile[u], b = tile[u ^ t.xl];
-                        const ff::f2 v =
-                            t.im ? ff::dot2(a.re, b.im, ff::neg(a.im), b.re) : ff::dot2(a.re, b.re, a.im, b.im);
-                        const bool neg = ((__popc(u & t.zl) & 1u) ^ tile_par) != 0;
-                        part[j] = neg ? ff::sub(part[j], v) : ff::add(part[j], v);
-                    }
-                }
-                const ff::f2 sum = ff::add(ff::add(part[0], part[1]), ff::add(part[2], part[3]));
-                acc[k].v += (double)sum.h + (double)sum.l;
+                const uint32_t k1 = p.t[k0].group_end;
+                if (p.t[k0].im) pauli_group<FFV, true>(p, tile, k0, k1, negs, acc);
+                else pauli_group<FFV, false>(p, tile, k0, k1, negs, acc);
+                k0 = k1;
             }
         }
+        fence_proxy_async();
         __syncthreads();
-    }
-    for (int k = 0; k < (int)nt; k++) {
-        {
-            const double v = block_sum(acc[k].value() * p.t[k].factor);
-            if (threadIdx.x == 0) rs.partials[(size_t)blockIdx.x * kMaxTerms + k] = v;
+        if (tau + gridDim.x < tiles) issue_load(tau + gridDim.x);
+        if ((it + 1) % (uint32_t)kPauliFlush == 0) {
+            for (int k = 0; k < (int)nt; k++) {
+                wide[k] = (flushed ? wide[k] : 0.0) + ((double)acc[k].h + (double)acc[k].l);
+                acc[k] = ff::f2{0.f, 0.f};
+            }
+            flushed = true;
         }
     }
-    if (last_block(rs.ticket)) {
+    const int lane = threadIdx.x & 31;
+    double mine = 0.0;
+    if (flushed)  // (uniform over the block)
         for (int k = 0; k < (int)nt; k++) {
-            const double tsum = sum_partials(rs.partials, gridDim.x, kMaxTerms, k);
-            if (threadIdx.x == 0) rs.result[k] = tsum;
+            const double v = warp_sum(wide[k]);
+            if (lane == k) mine = v;
         }
-        if (threadIdx.x == 0) *rs.ticket = 0;
-    }
+#pragma unroll 1
+    for (int k = 0; k < (int)nt; k++) acc[k] = ff::two_sum(acc[k].h, acc[k].l);
+    const ff::f2 r = warp_sum_terms(acc);
+    mine += (double)r.h + (double)r.l;
+    finish_terms(lane < (int)nt ? mine * p.t[lane].factor : 0.0, nt, rs);
 }
 
 template <class T>
 cudaError_t launch_pauli_tile(const void *st, uint32_t n, bool ff_resident, const PauliTilePass &p,
-                              const ReduceScratch &rs, cudaStream_t s) {
-    using V = typename TileVal<T>::V;
-    const size_t smem = (sizeof(V) << p.K) + (sizeof(uint64_t) << p.m);
+                              const ReduceScratch &rs, int *err, cudaStream_t s) {
+    auto bytes = [](uint32_t K, uint32_t m) -> size_t {
+        return ((size_t)(sizeof(T) == 8 ? 16 : 8) << K) + (sizeof(uint64_t) << m) + 16;
+    };
     auto kern = (sizeof(T) == 8 && ff_resident) ? k_pauli_tile<T, true> : k_pauli_tile<T, false>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    constexpr uint32_t kMax = pauli_tile_bits<T>();  // (the limit is set once per kernel, for its largest tile)
+    cudaError_t e = ensure_smem_limit((const void *)kern, bytes(kMax, kMax - 5));
     if (e != cudaSuccess) return e;
     const uint64_t tiles = 1ull << (n - p.K);
-    const unsigned grid = (unsigned)std::min<uint64_t>(tiles, (uint64_t)kReduceBlocks);
-    kern<<<grid, 256, smem, s>>>(st, n, p, rs);
+    const unsigned grid = (unsigned)std::min<uint64_t>(tiles, 152ull * 3);
+    kern<<<grid, kPauliThreads, bytes(p.K, p.m), s>>>(st, n, p, rs, err);
     count_launch();
     return cudaGetLastError();
 }
@@ -1196,7 +1358,7 @@ namespace kbwg {
     template cudaError_t launch_pauli_group<T>(const void *, uint32_t, const PauliGroup &, const ReduceScratch &, \
                                                cudaStream_t, bool);                                           \
     template cudaError_t launch_pauli_tile<T>(const void *, uint32_t, bool, const PauliTilePass &,               \
-                                              const ReduceScratch &, cudaStream_t);                           \
+                                              const ReduceScratch &, int *, cudaStream_t);                           \
     template cudaError_t launch_dump_count<T>(const void *, uint32_t, uint64_t *, cudaStream_t);               \
     template cudaError_t launch_dump_write<T>(const void *, uint32_t, const uint64_t *, const DumpSpec &,        \
                                               uint64_t *, double *, double *, cudaStream_t);                  \
