@@ -497,8 +497,24 @@ uint32_t tile_register_bits(const Sim &s, uint32_t k) {
     return k == 11 ? 3u : 4u;  // the 2^11 tiles hold 8 amplitudes per thread, the larger ones 16
 }
 
+// Default tile by register size: below ~152 tiles of the largest geometry the
+// chip has idle SMs, and a smaller tile spreads a gate over more of them at
+// the price of a few more sweeps.  Measured (interpreted sweeps, us per flush,
+// one GB300; HEA 4 layers / brickwork 8 layers):
+//   complex64  n = 16: K 13 153/161, 12 125/131, 11 117/120;  n = 19: 180/196,
+//   148/158, 145/150;  n = 20: 184/203, 173/189, 216/225;  n = 21: 261/291,
+//   282/315, 301/319
+//   binary64   n = 14: K 12 485/327, 11 278/201;  n = 19: 623/429, 620/401;
+//   specialised (from 20 qubits) K 12 is 3-5 % faster (n = 25: 46.5 against
+//   48.4 ms, HEA 6 layers)
+//   float-float: K 11 is the faster one up to 24 qubits.
 uint32_t default_tile_k(const Sim &s) {
     const std::vector<uint32_t> ks = compiled_tiles(s);
+    if (ks.size() > 1 && ks[0] <= s.n) {
+        if (!s.prec && s.n <= 19) return 11;
+        if (!s.prec && s.n == 20) return 12;
+        if (s.prec && !ff_capable(s) && s.n <= 19) return 11;
+    }
     if (ks[0] <= s.n) return ks[0];
     uint32_t fit = 0;
     for (uint32_t k : ks)
