@@ -542,8 +542,8 @@ __global__ void __launch_bounds__(AdjKernel<P, K, R>::kThreads, 2)
                     }
                 }
                 using B = typename pick_t<W, uint64_t, uint32_t>::type;
-                tile_gate<P, K, R, B, false>(g, vp, R0, F, (B)base);
-                tile_gate<P, K, R, B, false>(g, vl, R0, F, (B)base);
+                tile_gate<P, K, R, B>(g, vp, R0, F, (B)base);
+                tile_gate<P, K, R, B>(g, vl, R0, F, (B)base);
             }
             g0 = g1;
         }
@@ -645,15 +645,95 @@ static cudaError_t adj_grow(B *&p, size_t &cap, size_t want) {
     return e;
 }
 
-static GateDesc inverse_desc(int prec, const GateDesc &g, double angle) {
-    // X, Y, Z, H are their own inverses; P/RX/RY/RZ invert by negating the angle
+static GateDesc inverse_desc(const GateDesc &g, double angle) {
+    // X, Y, Z, H are their own inverses; P/RX/RY/RZ invert by negating the
+    // angle (constants in binary64 for every precision)
     switch (g.kind) {
     case G_P:
     case G_RX:
     case G_RY:
-    case G_RZ: return make_gate_desc(prec, g.kind, g.target, g.ctrl, -angle);
+    case G_RZ: return make_gate_desc(1, g.kind, g.target, g.ctrl, -angle);
+    case G_H: return make_gate_desc(1, G_H, g.target, g.ctrl, 0.0);
     default: return g;
     }
+}
+
+template <class P> constexpr int arith_of() {
+    return std::is_same<P, FastP>::value ? ARITH_C64 : (std::is_same<P, Fast<double>>::value ? ARITH_F64 : ARITH_FF);
+}
+
+// Uniform factors of a planned reverse sweep's gates left to one
+// multiplication of both states at its end (as the forward sweeps do it,
+// sweep.cu): H's 1/sqrt(2), RZ's phase on |0> and the larger coefficient of
+// an uncontrolled RX/RY.  With f the factor dropped so far, the states are
+// phi = f phi', lambda = f lambda', so a gradient term <lambda'|P|phi'> is
+// short of |f|^2: mult receives that factor per gate of the sweep.  At most
+// kAdjDeferRun gates that grow the states (each by sqrt(2)) are taken, so
+// products of two amplitudes stay inside float's range.  A phase alone is
+// carried to the segment's next sweep in `g`; the last one applies it.
+// With the fewer checkpoints of kDriftGates, measured on one GB300: 24 qubits,
+// 480 parameters, complex64 13.6 -> 9.2 ms (reverse sweeps 7.4 -> 5.9, forward
+// 2.7 -> 1.4, checkpoint copies 1.36 -> 0.17), 17 qubits, 170 parameters,
+// float-float 1.55 -> 1.10 ms (44 -> 8 sweeps).
+constexpr int kAdjDeferRun = 80, kAdjDeferMin = 3;
+template <class P, int R>
+static void defer_sweep(PlannedSweep &sw, bool last, DdFactor &g, std::vector<double> &mult) {
+    constexpr int arith = arith_of<P>();
+    mult.assign(sw.gates.size(), 1.0);
+    size_t count = 0;
+    for (const TileGate &t : sw.gates)
+        if (!t.cl && !t.co && (t.cls == TG_H || t.cls == TG_RX || t.cls == TG_RY || t.cls == TG_RZ)) count++;
+    const bool defer = count >= (size_t)kAdjDeferMin && sw.gates.size() < (size_t)kMaxSweepGates;
+    Dd mag{1.0, 0.0};  // |f|
+    int grown = 0;
+    for (size_t i = 0; i < sw.gates.size(); i++) {
+        TileGate &t = sw.gates[i];
+        mult[i] = mag.h * mag.h;
+        if (!defer || t.cl || t.co) continue;
+        if (t.cls == TG_RZ) {
+            const double u[4] = {t.c[0], t.c[1], t.c[2], t.c[3]};
+            defer_diagonal(u, t.c[0], t.c[1]);
+            t.c[2] = t.c[3] = 0.0;
+            g.times(u[0], u[1]);
+            t.cls = TG_P;
+            t.op = (uint8_t)(t.op - (TG_RZ - TG_P) * (t.op < OP_DFIX ? 4 : 1));
+        } else if (t.cls == TG_H && grown < kAdjDeferRun) {
+            t.sub = 1;
+            mag = dd_mul(mag, dd_unit(1.0));
+            g.times(dd_unit(1.0));
+            grown++;
+        } else if ((t.cls == TG_RX || t.cls == TG_RY) && grown < kAdjDeferRun) {
+            const DeferredRotation r = defer_rotation(arith, t.c[0], t.c[1]);
+            t.sub = 1;
+            t.c[0] = r.w;
+            t.c[1] = r.cot ? 1.0 : 0.0;
+            mag = dd_mul(mag, r.factor);
+            g.times(r.factor);
+            grown++;
+        }
+    }
+    if (sw.gates.size() >= (size_t)kMaxSweepGates || (last ? !g.used : !grown)) return;
+    // (the structure of a sweep does not depend on its angles: a last sweep
+    // always ends with the complex factor, the others with the real one)
+    TileGate t;
+    memset(&t, 0, sizeof t);
+    t.cls = TG_SCALE;
+    t.op = OP_DFIX + (TG_SCALE - TG_Z);
+    t.jm = (uint16_t)((1u << (1u << R)) - 1u);
+    if (last) {
+        t.c[0] = g.re.h;
+        t.c[1] = g.im.h;
+        g = DdFactor();
+    } else {
+        t.sub = 1;
+        t.c[0] = mag.h < 0.0 ? -mag.h : mag.h;
+        // the phase stays: g / |f|
+        const double inv = 1.0 / t.c[0], res = fma(-inv, t.c[0], 1.0);
+        g.times(Dd{inv, inv * res});
+    }
+    sw.gates.push_back(t);
+    sw.stage_end.back()++;
+    mult.push_back(1.0);
 }
 
 // One reverse sweep, planned: its parameters (program and gradient info
@@ -682,26 +762,31 @@ template <class P, int K, int R>
 static cudaError_t plan_segment(Sim &s, AdjScratch &sc, const std::vector<GateDesc> &fwd,
                                 const std::vector<double> &angles, const std::vector<int> &gtype, size_t lo, size_t hi,
                                 std::vector<unsigned char> &progs, std::vector<unsigned char> &infos,
-                                std::vector<RevSweep> &out) {
+                                std::vector<RevSweep> &out, std::vector<double> &gate_mult) {
     using AK = AdjKernel<P, K, R>;
     std::vector<GateDesc> rev;
     std::vector<size_t> rev_src;
     for (size_t j = hi; j-- > lo;) {
-        rev.push_back(inverse_desc(s.prec, fwd[j], angles[j]));
+        rev.push_back(inverse_desc(fwd[j], angles[j]));
         rev_src.push_back(j);
     }
-    const std::vector<PlannedSweep> plan = plan_sweeps(s.n, K, R, rev.data(), rev.size(), false);
+    // (one gate short of a full program: the deferred factor is the last one)
+    std::vector<PlannedSweep> plan = plan_sweeps(s.n, K, R, rev.data(), rev.size(), false, kMaxSweepGates - 1);
+    DdFactor g;
     // gradient info per sweep: type | slot << 4 per gate, then the gate of each slot
     std::vector<std::vector<uint32_t>> metas(plan.size());
     uint64_t key = fnv(1469598103934665603ull, AdjPolicyName<P>::s, strlen(AdjPolicyName<P>::s));
     const size_t first = out.size();
     for (size_t k = 0; k < plan.size(); k++) {
-        const PlannedSweep &sw = plan[k];
+        PlannedSweep &sw = plan[k];
+        std::vector<double> mult;
+        defer_sweep<P, R>(sw, k + 1 == plan.size(), g, mult);
         std::vector<uint32_t> &meta = metas[k];
         meta.assign(sw.gates.size(), 0);
         std::vector<uint32_t> gate_of_slot;
-        for (size_t i = 0; i < sw.gates.size(); i++) {
+        for (size_t i = 0; i < sw.src.size(); i++) {
             const size_t j = rev_src[sw.src[i]];
+            gate_mult[j] = mult[i];
             if (gtype[j] != GT_NONE) {
                 meta[i] = (uint32_t)gtype[j] | ((uint32_t)gate_of_slot.size() << 4);
                 gate_of_slot.push_back((uint32_t)j);
@@ -1024,6 +1109,9 @@ static std::vector<ApplyGroup> make_groups(const std::vector<PauliString> &H) {
     return groups;
 }
 
+constexpr size_t kDriftGates = 256;           // most gates uncomputed between two checkpoints
+constexpr size_t kSmallState = 64ull << 20;  // scratch of states up to this size stays with the handle unasked
+
 template <class P, class T, int K, int R>
 static int32_t adjoint_run(Sim &s, const std::vector<GateDesc> &fwd, const std::vector<double> &angles,
                            const std::vector<int> &gtype, const std::vector<PauliString> &H, double *energy,
@@ -1061,12 +1149,17 @@ static int32_t adjoint_run(Sim &s, const std::vector<GateDesc> &fwd, const std::
     e = adj_grow(sc.partials, sc.partials_cap, (size_t)num_sms * 8 * kMaxSweepGates * sizeof(double));
     if (e == cudaSuccess) e = adj_grow(sc.grads, sc.grads_cap, std::max<size_t>(M, 1) * sizeof(double));
     if (e != cudaSuccess) return fail_cuda(e, "scratch");
-    // checkpoints: at most max_ckpt, new ones only while they fit in 80% of
-    // the free memory
-    const size_t want = std::min<size_t>(max_ckpt, M > 1 ? M - 1 : 0);
+    // checkpoints: one per kDriftGates gates, at most max_ckpt, new ones only
+    // while they fit in 80% of the free memory.  (lambda is never reloaded, so
+    // its drift over the whole circuit bounds what closer checkpoints of phi
+    // could give, while every segment boundary costs sweeps: 24 qubits, 720
+    // gates, 17 segments 33 + 36 sweeps and 32 copies, 3 segments 10 + 12 and 4.)
+    const size_t want = std::min<size_t>(max_ckpt, M ? (M - 1) / kDriftGates : 0);
     size_t free_b = 0, total_b = 0;
-    e = cudaMemGetInfo(&free_b, &total_b);
-    if (e != cudaSuccess) return fail_cuda(e, "memory query");
+    if (sc.ckpt.size() < want || sb > kSmallState) {
+        e = cudaMemGetInfo(&free_b, &total_b);
+        if (e != cudaSuccess) return fail_cuda(e, "memory query");
+    }
     while (sc.ckpt.size() < want && sb <= (size_t)(0.8 * (double)free_b)) {
         void *c = nullptr;
         if (cudaMalloc(&c, sb) != cudaSuccess) {
@@ -1105,10 +1198,11 @@ static int32_t adjoint_run(Sim &s, const std::vector<GateDesc> &fwd, const std::
     // programs and gradient info go up in one copy from pinned memory
     std::vector<unsigned char> progs, infos;
     std::vector<RevSweep> sweeps;
+    std::vector<double> gate_mult(M, 1.0);  // what the deferred factors leave out of each gradient term
     std::vector<size_t> seg_first(S + 1, 0);
     for (size_t seg = S; seg-- > 0;) {
         seg_first[seg + 1] = sweeps.size();  // (segments run last first)
-        e = plan_segment<P, K, R>(s, sc, fwd, angles, gtype, b[seg], b[seg + 1], progs, infos, sweeps);
+        e = plan_segment<P, K, R>(s, sc, fwd, angles, gtype, b[seg], b[seg + 1], progs, infos, sweeps, gate_mult);
         if (e != cudaSuccess) return fail_cuda(e, "reverse plan");
     }
     const size_t up = progs.size() + infos.size();
@@ -1200,9 +1294,10 @@ static int32_t adjoint_run(Sim &s, const std::vector<GateDesc> &fwd, const std::
     if (e == cudaSuccess) e = cudaStreamSynchronize(s.stream);
     if (e != cudaSuccess) return fail_cuda(e, "finish");
     *energy = s.h_result[0];
+    for (size_t j = 0; j < M; j++) grad_per_gate[j] *= gate_mult[j];
     // lambda and the checkpoints stay for the next call while they are small
     // against the device (a sixteenth of its memory); larger ones go now
-    if (sb * (1 + sc.ckpt.size()) > total_b / 16) sc.release_states();
+    if (sb > kSmallState && sb * (1 + sc.ckpt.size()) > total_b / 16) sc.release_states();
     return KBWG_OK;
 }
 
@@ -1217,13 +1312,16 @@ static size_t check_adjoint_p(const Sim &s, const std::vector<GateDesc> &fwd, co
         rev.push_back(fwd[j]);  // (the structure of the inverse gate is the gate's)
         rev_src.push_back(j);
     }
-    const std::vector<PlannedSweep> plan = plan_sweeps(s.n, K, R, rev.data(), rev.size(), false);
+    std::vector<PlannedSweep> plan = plan_sweeps(s.n, K, R, rev.data(), rev.size(), false, kMaxSweepGates - 1);
+    DdFactor g;
     const JitGeometry geo{AdjPolicyName<P>::s, K, R, AK::kThreads, 2};
     std::vector<std::string> srcs;
-    for (const PlannedSweep &sw : plan) {
+    for (PlannedSweep &sw : plan) {
+        std::vector<double> mult;
+        defer_sweep<P, R>(sw, &sw == &plan.back(), g, mult);
         std::vector<uint32_t> meta(sw.gates.size(), 0);
         uint32_t nslots = 0;
-        for (size_t i = 0; i < sw.gates.size(); i++) {
+        for (size_t i = 0; i < sw.src.size(); i++) {
             const size_t j = rev_src[sw.src[i]];
             if (gtype[j] != GT_NONE) meta[i] = (uint32_t)gtype[j] | (nslots++ << 4);
         }

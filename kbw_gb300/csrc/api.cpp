@@ -866,7 +866,7 @@ int32_t kbwg_adjoint_gradient(kbwg_sim *s, const kbwg_gate *gates, uintptr_t n_g
     std::vector<int> gtype;
     r = parse_grad_circuit(s, gates, n_gates, param_index, n_params, fwd, angles, gtype);
     if (r) return r;
-    CUDA_TRY(settle(*s));
+    CUDA_TRY(flush_queue(*s));  // (the state itself starts anew, in whatever form it is)
     std::vector<double> per_gate;
     r = adjoint_gradient(*s, fwd, angles, gtype, strs, energy, per_gate, max_checkpoints);
     if (r) return r;

@@ -9,6 +9,7 @@
 
 #include "../../include/kbwg.h"
 #include "common.cuh"
+#include "dd.h"
 #include "kernels.h"
 #include "stdrng.h"
 
@@ -114,7 +115,6 @@ GateDesc make_gate_desc(int prec, uint32_t kind, uint32_t target, uint64_t ctrl,
 
 // Gates folded and their uniform factors left to one multiplication, as the
 // sweeps of a reordering handle run them (sweep.cu).
-enum { ARITH_C64 = 0, ARITH_F64 = 1, ARITH_FF = 2 };
 std::vector<GateDesc> defer_factors(int arith, const GateDesc *gates, size_t count);
 
 // Run every queued gate (fused sweeps unless KBWG_FLAG_NO_FUSION).

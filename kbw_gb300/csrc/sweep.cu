@@ -30,6 +30,7 @@
 #include <math.h>
 
 #include "../../include/kbwg.h"
+#include "dd.h"
 #include "jit.h"
 #include "kernels.h"
 #include "sim.h"
@@ -610,41 +611,7 @@ static cudaError_t run_fused_t(Sim &s, const GateDesc *gates, size_t count) {
 // each gate with its share of g is a rotation to binary64 accuracy.
 constexpr int kDeferRun = 192, kDeferMin = 3;
 
-template <class T>
-static double packed_value(double x) {  // x as the program's constants hold it
-    if constexpr (std::is_same<T, float>::value) return (double)(float)x;
-    if constexpr (std::is_same<T, ff::f2>::value) {
-        const ff::f2 v = ff::split_constant(x);
-        return (double)v.h + (double)v.l;
-    }
-    return x;
-}
-
-// The collected factor as an unevaluated sum of two doubles per part: a product
-// of a few hundred factors rounded once, at the end (in plain binary64 its
-// own rounding would be larger than the gates').
-struct Dd {
-    double h = 0.0, l = 0.0;
-};
-static Dd dd_mul(Dd a, Dd b) {
-    const double p = a.h * b.h, e = fma(a.h, b.h, -p) + (a.h * b.l + a.l * b.h), s = p + e;
-    return Dd{s, e - (s - p)};
-}
-static Dd dd_add(Dd a, Dd b) {
-    const double s = a.h + b.h, bb = s - a.h, e = ((a.h - (s - bb)) + (b.h - bb)) + (a.l + b.l), r = s + e;
-    return Dd{r, e - (r - s)};
-}
-// 1 / sqrt(1 + w^2) for |w| <= 1: the rounded value and one Newton step's correction
-static Dd dd_unit(double w) {
-    const double w2 = w * w, w2e = fma(w, w, -w2), sh = 1.0 + w2, sl = (w2 - (sh - 1.0)) + w2e;
-    const double r = 1.0 / sqrt(sh), r2 = r * r, r2e = fma(r, r, -r2);
-    const double e = fma(-r2, sh, 1.0) - (r2 * sl + r2e * sh);
-    return Dd{r, 0.5 * r * e};
-}
-
-template <class T>
-static std::vector<GateDesc> defer_scale(const GateDesc *gates, size_t count, bool rotations) {
-    constexpr bool kFF = std::is_same<T, ff::f2>::value;
+static std::vector<GateDesc> defer_scale(int arith, const GateDesc *gates, size_t count, bool rotations) {
     std::vector<GateDesc> out;
     out.reserve(count + 2);
     size_t rots = 0, any = 0;
@@ -653,26 +620,20 @@ static std::vector<GateDesc> defer_scale(const GateDesc *gates, size_t count, bo
         if (gates[i].kind == G_RX || gates[i].kind == G_RY) rots++;
         if (gates[i].kind == G_H || gates[i].kind == G_RZ) any++;
     }
-    const bool defer = kFF || rots + any >= (size_t)kDeferMin;  // H and RZ
+    const bool defer = arith == ARITH_FF || rots + any >= (size_t)kDeferMin;  // H and RZ
     const bool drot = rotations && (rots >= (size_t)kDeferMin || (defer && any > 0));
-    Dd gr{1.0, 0.0}, gi;
+    DdFactor g;
     bool complex_g = false, pending = false;
     int unscaled = 0;
-    auto scale_by = [&](Dd f) {
-        gr = dd_mul(gr, f);
-        gi = dd_mul(gi, f);
-        pending = true;
-    };
     auto emit_scale = [&]() {
         GateDesc sc;
         memset(&sc, 0, sizeof sc);
         sc.kind = complex_g ? G_SCALE : G_SCALER;
         sc.target = 0;
-        sc.c[0] = gr.h;
-        sc.c[1] = gi.h;
+        sc.c[0] = g.re.h;
+        sc.c[1] = g.im.h;
         out.push_back(sc);
-        gr = Dd{1.0, 0.0};
-        gi = Dd();
+        g = DdFactor();
         complex_g = pending = false;
         unscaled = 0;
     };
@@ -681,32 +642,24 @@ static std::vector<GateDesc> defer_scale(const GateDesc *gates, size_t count, bo
         bool grew = false;
         if (defer && x.kind == G_H && x.ctrl == 0) {
             x.kind = G_HN;
-            scale_by(dd_unit(1.0));
+            g.times(dd_unit(1.0));
             grew = true;
         } else if (defer && x.kind == G_RZ && x.ctrl == 0) {
-            // diag(u0, u1) = u0 diag(1, u1 conj(u0)) for unit u0 (for RZ(t):
-            // u1 conj(u0) = e^{it}; also a folded general diagonal)
-            const Dd ur{x.c[0], 0.0}, ui{x.c[1], 0.0}, nui{-x.c[1], 0.0}, vr{x.c[2], 0.0}, vi{x.c[3], 0.0};
-            const double c = dd_add(dd_mul(vr, ur), dd_mul(vi, ui)).h, sn = dd_add(dd_mul(vi, ur), dd_mul(vr, nui)).h;
-            const Dd nr = dd_add(dd_mul(gr, ur), dd_mul(gi, nui));
-            gi = dd_add(dd_mul(gr, ui), dd_mul(gi, ur));
-            gr = nr;
+            // u0 diag(1, u1 conj(u0)) (for RZ(t): u1 conj(u0) = e^{it}; also a folded general diagonal)
+            double c, sn;
+            defer_diagonal(x.c, c, sn);
+            g.times(x.c[0], x.c[1]);
             complex_g = pending = true;
             x.kind = G_P;
             x.c[0] = c;
             x.c[1] = sn;
             x.c[2] = x.c[3] = 0.0;
         } else if (drot && (x.kind == G_RX || x.kind == G_RY) && x.ctrl == 0) {
-            const double c = x.c[0], sn = x.c[1];
-            const bool cot = !(fabs(c) >= fabs(sn));
-            const double w = packed_value<T>(cot ? c / sn : sn / c);
-            // the factor that makes (1, w) a unit vector, with the dropped coefficient's sign
-            Dd f = dd_unit(w);
-            if ((cot ? sn : c) < 0.0) f = Dd{-f.h, -f.l};
-            scale_by(f);
+            const DeferredRotation r = defer_rotation(arith, x.c[0], x.c[1]);
+            g.times(r.factor);
             x.kind = x.kind == G_RX ? G_RXD : G_RYD;
-            x.c[0] = w;
-            x.c[1] = cot ? 1.0 : 0.0;
+            x.c[0] = r.w;
+            x.c[1] = r.cot ? 1.0 : 0.0;
             grew = true;
         }
         if (x.kind == G_P) {
@@ -722,6 +675,7 @@ static std::vector<GateDesc> defer_scale(const GateDesc *gates, size_t count, bo
             }
         }
         out.push_back(x);
+        pending = pending || grew;
         if (grew && ++unscaled >= kDeferRun) emit_scale();
     }
     if (pending) emit_scale();
@@ -737,9 +691,7 @@ std::vector<GateDesc> defer_factors(int arith, const GateDesc *gates, size_t cou
         gates = r.data();
     }
     const std::vector<GateDesc> f = fold_diagonals(gates, count);
-    if (arith == ARITH_FF) return defer_scale<ff::f2>(f.data(), f.size(), true);
-    return arith == ARITH_F64 ? defer_scale<double>(f.data(), f.size(), true)
-                              : defer_scale<float>(f.data(), f.size(), true);
+    return defer_scale(arith, f.data(), f.size(), true);
 }
 
 // The gate list as the fused sweeps of a handle run it (folded, factors
@@ -747,7 +699,7 @@ std::vector<GateDesc> defer_factors(int arith, const GateDesc *gates, size_t cou
 static std::vector<GateDesc> rewritten(const Sim &s, const GateDesc *gates, size_t count) {
     if (s.flags & KBWG_FLAG_EXACT_ORDER) return std::vector<GateDesc>(gates, gates + count);
     if (s.flags & KBWG_FLAG_NO_FOLD) {  // every gate applied as given, but for float-float's H and RZ
-        if (ff_capable(s)) return defer_scale<ff::f2>(gates, count, false);
+        if (ff_capable(s)) return defer_scale(ARITH_FF, gates, count, false);
         return std::vector<GateDesc>(gates, gates + count);
     }
     return defer_factors(ff_capable(s) ? ARITH_FF : (s.prec ? ARITH_F64 : ARITH_C64), gates, count);
