@@ -369,60 +369,79 @@ __global__ void __launch_bounds__(256) k_apply_tile_f32(const cx<float> *__restr
     }
 }
 
-// Re<a|b> of float-float states: per-thread float-float sums, then FP64.
-__global__ void __launch_bounds__(256) k_inner_re_ff(const ff2::v2 *__restrict__ a, const ff2::v2 *__restrict__ b,
-                                                     uint64_t ns, double *partials, unsigned *ticket, double *result) {
-    ff::f2 t{0.f, 0.f};
-    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    for (uint64_t s = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; s < ns; s += stride) {
-        const ff2::v2 x = a[s], y = b[s];
-        t = ff::add(t, ff::dot2(ff::f2{x.h.x, x.l.x}, ff::f2{y.h.x, y.l.x}, ff::f2{x.h.y, x.l.y}, ff::f2{y.h.y, y.l.y}));
-    }
-    double acc = (double)t.h + (double)t.l;
-    __shared__ double sh[8];
-    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = acc;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double tot = 0.0;
-        for (int w = 0; w < (int)(blockDim.x >> 5); w++) tot += sh[w];
-        partials[blockIdx.x] = tot;
-        __threadfence();
-        if (atomicAdd(ticket, 1u) == gridDim.x - 1) {
-            double all = 0.0;
-            for (unsigned b2 = 0; b2 < gridDim.x; b2++) all += partials[b2];
-            result[0] = all;
-            *ticket = 0;
-        }
-    }
+// Share of Re<a|b> of one amplitude pair: float-float (exact products of the
+// complex64 parts), or added in binary64 for binary64 states.
+__device__ __forceinline__ ff::f2 re_product(const ff2::v2 &x, const ff2::v2 &y) {
+    return ff::dot2(ff::f2{x.h.x, x.l.x}, ff::f2{y.h.x, y.l.x}, ff::f2{x.h.y, x.l.y}, ff::f2{y.h.y, y.l.y});
+}
+__device__ __forceinline__ ff::f2 re_product(const cx<float> &x, const cx<float> &y) {
+    const float p = __fmul_rn(x.re, y.re), q = __fmul_rn(x.im, y.im);
+    const ff::f2 t = ff::two_sum(p, q);
+    return ff::fast_two_sum(t.h, ff::add(t.l, ff::add(__fmaf_rn(x.re, y.re, -p), __fmaf_rn(x.im, y.im, -q))));
 }
 
-// Re<a|b> (FP64-grade) into result[0].
-template <class T>
-__global__ void __launch_bounds__(256) k_inner_re(const cx<T> *__restrict__ a, const cx<T> *__restrict__ b,
-                                                  uint64_t ns, double *partials, unsigned *ticket, double *result) {
-    double acc = 0.0;
+// Re<a|b> (FP64-grade) into result[0].  Four pairs in flight per thread; the
+// last block adds the partials with all its threads (one thread read 608 of
+// them in a row: most of a 35 us launch on 17 qubits), and complex64 products
+// stay off the FP64 pipe (24 qubits: 227 us there, 40 us of reads).
+template <class Mem>
+__global__ void __launch_bounds__(256) k_inner_re(const Mem *__restrict__ a, const Mem *__restrict__ b, uint64_t ns,
+                                                  double *partials, unsigned *ticket, double *result) {
+    constexpr bool kWide = std::is_same<Mem, cx<double>>::value;
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    for (uint64_t s = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; s < ns; s += stride) {
-        const cx<T> x = a[s], y = b[s];
-        acc = fma((double)x.re, (double)y.re, acc);
-        acc = fma((double)x.im, (double)y.im, acc);
+    uint64_t s = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    double acc = 0.0;
+    ff::f2 t0{0.f, 0.f}, t1{0.f, 0.f};
+    for (; s + 3 * stride < ns; s += 4 * stride) {
+        Mem x[4], y[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            x[u] = a[s + u * stride];
+            y[u] = b[s + u * stride];
+        }
+        if constexpr (kWide) {
+#pragma unroll
+            for (int u = 0; u < 4; u++) acc = fma(x[u].re, y[u].re, fma(x[u].im, y[u].im, acc));
+        } else {
+            t0 = ff::add(t0, ff::add(re_product(x[0], y[0]), re_product(x[1], y[1])));
+            t1 = ff::add(t1, ff::add(re_product(x[2], y[2]), re_product(x[3], y[3])));
+        }
+    }
+    for (; s < ns; s += stride) {
+        const Mem x = a[s], y = b[s];
+        if constexpr (kWide) acc = fma(x.re, y.re, fma(x.im, y.im, acc));
+        else t0 = ff::add(t0, re_product(x, y));
+    }
+    if constexpr (!kWide) {
+        t0 = ff::add(t0, t1);
+        acc = (double)t0.h + (double)t0.l;
     }
     __shared__ double sh[8];
-    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = acc;
-    __syncthreads();
-    if (threadIdx.x == 0) {
+    __shared__ bool is_last;
+    auto block_total = [&](double v) {  // valid in thread 0
+        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+        __syncthreads();
+        if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
+        __syncthreads();
         double t = 0.0;
-        for (int w = 0; w < (int)(blockDim.x >> 5); w++) t += sh[w];
-        partials[blockIdx.x] = t;
+        if (threadIdx.x == 0)
+            for (int w = 0; w < (int)(blockDim.x >> 5); w++) t += sh[w];
+        return t;
+    };
+    const double mine = block_total(acc);
+    if (threadIdx.x == 0) {
+        partials[blockIdx.x] = mine;
         __threadfence();
-        if (atomicAdd(ticket, 1u) == gridDim.x - 1) {
-            double tot = 0.0;
-            for (unsigned b2 = 0; b2 < gridDim.x; b2++) tot += partials[b2];
-            result[0] = tot;
-            *ticket = 0;
-        }
+        is_last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!is_last) return;
+    double v = 0.0;
+    for (unsigned k = threadIdx.x; k < gridDim.x; k += blockDim.x) v += __ldcg(partials + k);
+    const double tot = block_total(v);
+    if (threadIdx.x == 0) {
+        result[0] = tot;
+        *ticket = 0;
     }
 }
 
@@ -1057,21 +1076,13 @@ static cudaError_t apply_hamiltonian_ff(Sim &s, void *lam, const std::vector<App
     return cudaSuccess;
 }
 
-static cudaError_t inner_re_ff_async(Sim &s, const void *a, const void *b) {
-    k_inner_re_ff<<<kReduceBlocks, 256, 0, s.stream>>>((const ff2::v2 *)a, (const ff2::v2 *)b, s.ns, s.rs.partials,
-                                                        s.rs.ticket, s.rs.result);
-    count_launch();
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-    return copy_async(s.h_result, s.rs.result, sizeof(double), cudaMemcpyDeviceToHost, s.stream);
-}
-
 // Re<a|b> into the handle's pinned result slot; readable after the stream's
 // next synchronisation.
-template <class T>
+template <class Mem>
 static cudaError_t inner_re_async(Sim &s, const void *a, const void *b) {
-    k_inner_re<T><<<kReduceBlocks, 256, 0, s.stream>>>((const cx<T> *)a, (const cx<T> *)b, s.ns, s.rs.partials,
-                                                        s.rs.ticket, s.rs.result);
+    const unsigned grid = (unsigned)std::min<uint64_t>(kReduceBlocks, std::max<uint64_t>(1, s.ns / 1024));
+    k_inner_re<Mem><<<grid, 256, 0, s.stream>>>((const Mem *)a, (const Mem *)b, s.ns, s.rs.partials, s.rs.ticket,
+                                                s.rs.result);
     count_launch();
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
@@ -1270,7 +1281,7 @@ static int32_t adjoint_run(Sim &s, const std::vector<GateDesc> &fwd, const std::
         if (e == cudaSuccess && !tiled) e = apply_hamiltonian<T>(s, sc.lam, make_groups(H));
     }
     if (e != cudaSuccess) return fail_cuda(e, "H|phi>");
-    e = kFF ? inner_re_ff_async(s, s.state, sc.lam) : inner_re_async<T>(s, s.state, sc.lam);
+    e = kFF ? inner_re_async<ff2::v2>(s, s.state, sc.lam) : inner_re_async<cx<T>>(s, s.state, sc.lam);
     if (e != cudaSuccess) return fail_cuda(e, "energy");
     // 3. reverse, segment by segment
     e = cudaMemsetAsync(sc.grads, 0, std::max<size_t>(M, 1) * sizeof(double), s.stream);

@@ -440,16 +440,13 @@ int32_t kbwg_measure(kbwg_sim *s, const uintptr_t *qubits, uintptr_t n_qubits, c
     }
     CUDA_TRY(copy_async(s->d_ctl, &c, sizeof c, cudaMemcpyHostToDevice, s->stream));
     if (s->ff_resident) {
-        for (uint32_t k = 0; k < n_qubits; k++)
-            CUDA_TRY(launch_measure_step_ff(s->state, s->n, s->d_ctl, k, s->rs, s->stream));
+        CUDA_TRY(launch_measure_steps_ff(s->state, s->n, s->d_ctl, (uint32_t)n_qubits, s->rs, s->stream));
         CUDA_TRY(launch_collapse_ff(s->state, s->n, s->d_ctl, 0, 0, 0.0, s->stream));
     } else {
         CUDA_TRY(dispatch(s, [&](auto *tp) {
             using T = std::remove_pointer_t<decltype(tp)>;
-            for (uint32_t k = 0; k < n_qubits; k++) {
-                cudaError_t e = launch_measure_step<T>(s->state, s->n, s->d_ctl, k, s->rs, s->stream);
-                if (e != cudaSuccess) return e;
-            }
+            cudaError_t e = launch_measure_steps<T>(s->state, s->n, s->d_ctl, (uint32_t)n_qubits, s->rs, s->stream);
+            if (e != cudaSuccess) return e;
             return launch_collapse<T>(s->state, s->n, s->d_ctl, 0, 0, 0.0, s->stream);
         }));
     }
@@ -528,13 +525,14 @@ int32_t kbwg_sample(kbwg_sim *s, const uintptr_t *qubits, uintptr_t n_qubits, ui
         set_error(KBWG_ECAPACITY, "sample capacity too small");
         return KBWG_ECAPACITY;
     }
-    CUDA_TRY(settle(*s));
+    CUDA_TRY(flush_queue(*s));  // (a float-float resident state is sampled as is)
+    const bool ff = s->ff_resident;
     const int B = sample_blocks(s->n);
     CUDA_TRY(s->tmp0.ensure((size_t)B * 8));
     double *d_bs = (double *)s->tmp0.ptr;
     CUDA_TRY(dispatch(s, [&](auto *tp) {
         using T = std::remove_pointer_t<decltype(tp)>;
-        return launch_weight_blocksum<T>(s->state, s->n, d_bs, s->stream);
+        return launch_weight_blocksum<T>(s->state, s->n, ff, d_bs, s->stream);
     }));
     std::vector<double> bs(B), pre(B + 1);
     CUDA_TRY(copy_async(bs.data(), d_bs, (size_t)B * 8, cudaMemcpyDeviceToHost, s->stream));
@@ -577,7 +575,7 @@ int32_t kbwg_sample(kbwg_sim *s, const uintptr_t *qubits, uintptr_t n_qubits, ui
     CUDA_TRY(copy_async(d_blocks, blocks.data(), nb * 4, cudaMemcpyHostToDevice, s->stream));
     CUDA_TRY(dispatch(s, [&](auto *tp) {
         using T = std::remove_pointer_t<decltype(tp)>;
-        return launch_sample_pick<T>(s->state, s->n, d_blocks, (uint32_t)nb, d_begin, d_pre, d_chosen, d_pick,
+        return launch_sample_pick<T>(s->state, s->n, ff, d_blocks, (uint32_t)nb, d_begin, d_pre, d_chosen, d_pick,
                                      s->stream);
     }));
     std::vector<uint64_t> pick(shots);

@@ -54,11 +54,12 @@ cudaError_t launch_distance(const void *a, const void *b, uint32_t n, const Redu
 cudaError_t launch_overlap(const void *a, int prec_a, const void *b, int prec_b, uint32_t n, const ReduceScratch &rs,
                            cudaStream_t s);
 
-// One step of the sequential measurement: conditional p1 of ctl->qubit[step]
-// given the outcomes so far, then the WeightedIndex decision, all on device.
+// The first `steps` steps of the sequential measurement, each of a qubit of its
+// own: conditional p1 of ctl->qubit[step] given the outcomes so far, then the
+// WeightedIndex decision, all on device.
 template <class T>
-cudaError_t launch_measure_step(const void *st, uint32_t n, MeasureCtl *ctl, uint32_t step,
-                                const ReduceScratch &rs, cudaStream_t s);
+cudaError_t launch_measure_steps(const void *st, uint32_t n, MeasureCtl *ctl, uint32_t steps,
+                                 const ReduceScratch &rs, cudaStream_t s);
 
 // Keep amplitudes with (s & M) == V multiplied by F(p[0])*F(p[1])*... in
 // sequence, zero the others.  M, V, p come from ctl when ctl != nullptr,
@@ -80,11 +81,11 @@ struct PauliGroup {
 // ff_resident: the state is in the float-float resident form (complex128,
 // diagonal groups only).
 // Float-float resident complex128 state (sweeps leave it so): the masked
-// norm, one measurement step and the collapse read and write that form.
+// norm, the measurement steps and the collapse read and write that form.
 cudaError_t launch_masked_norm_ff(const void *st, uint32_t n, uint64_t M, uint64_t V, const ReduceScratch &rs,
                                   cudaStream_t s);
-cudaError_t launch_measure_step_ff(const void *st, uint32_t n, MeasureCtl *ctl, uint32_t step,
-                                   const ReduceScratch &rs, cudaStream_t s);
+cudaError_t launch_measure_steps_ff(const void *st, uint32_t n, MeasureCtl *ctl, uint32_t steps,
+                                    const ReduceScratch &rs, cudaStream_t s);
 cudaError_t launch_collapse_ff(void *st, uint32_t n, const MeasureCtl *ctl, uint64_t M, uint64_t V, double p,
                                cudaStream_t s);
 template <class T>
@@ -136,13 +137,13 @@ cudaError_t launch_dump_write(const void *st, uint32_t n, const uint64_t *offset
 // sampling: per-block weight sums, then per-block picks for sorted draws.
 int sample_blocks(uint32_t n);
 template <class T>
-cudaError_t launch_weight_blocksum(const void *st, uint32_t n, double *blocksum, cudaStream_t s);
+cudaError_t launch_weight_blocksum(const void *st, uint32_t n, bool ff_resident, double *blocksum, cudaStream_t s);
 // For every block b with shots: shots [shot_begin[b], shot_begin[b+1]) of the
 // sorted chosen[] array; prefix[b] = weight before the block.  Writes the
 // picked amplitude index per shot into pick[].
 template <class T>
-cudaError_t launch_sample_pick(const void *st, uint32_t n, const uint32_t *blocks, uint32_t nblocks_with_shots,
-                               const uint64_t *shot_begin, const double *prefix, const double *chosen,
+cudaError_t launch_sample_pick(const void *st, uint32_t n, bool ff_resident, const uint32_t *blocks,
+                               uint32_t nblocks_with_shots, const uint64_t *shot_begin, const double *prefix, const double *chosen,
                                uint64_t *pick, cudaStream_t s);
 
 }  // namespace kbwg

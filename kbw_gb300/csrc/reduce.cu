@@ -260,13 +260,24 @@ cudaError_t launch_masked_norm(const void *st, uint32_t n, uint64_t M, uint64_t 
 // product, summed per thread in float-float (FP32-pipe work), then in binary64.
 __device__ __forceinline__ double masked_norm_body_ff(const float4 *__restrict__ st, uint64_t count, uint64_t M,
                                                       uint64_t V) {
-    ff::f2 acc{0.f, 0.f};
+    // four loads in flight per thread and two independent sums: with one of
+    // each, a 24-qubit p1 (128 MiB read) took 41 us, two thirds of it waiting
+    ff::f2 acc{0.f, 0.f}, acc1{0.f, 0.f};
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < count; i += stride) {
-        const float4 f = st[insert_zeros(i, M) | V];
+    uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    auto prob = [](float4 f) {
         const ff::f2 re{f.x, f.z}, im{f.y, f.w};
-        acc = ff::add(acc, ff::dot2(re, re, im, im));
+        return ff::dot2(re, re, im, im);
+    };
+    for (; i + 3 * stride < count; i += 4 * stride) {
+        float4 f[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) f[u] = st[insert_zeros(i + u * stride, M) | V];
+        acc = ff::add(acc, ff::add(prob(f[0]), prob(f[1])));
+        acc1 = ff::add(acc1, ff::add(prob(f[2]), prob(f[3])));
     }
+    for (; i < count; i += stride) acc = ff::add(acc, prob(st[insert_zeros(i, M) | V]));
+    acc = ff::add(acc, acc1);
     return block_sum((double)acc.h + (double)acc.l);
 }
 
@@ -392,56 +403,95 @@ cudaError_t launch_overlap(const void *a, int prec_a, const void *b, int prec_b,
 }
 
 // ---- sequential measurement step ------------------------------------------
+// QubitManager::do_measure's decision for one qubit (src/quantum_execution.rs:278-287)
+// from s1, the weight of its |1> side among the outcomes so far; by one thread.
+template <class T>
+__device__ __forceinline__ void measure_decide(MeasureCtl *ctl, uint32_t step, uint64_t bit, double s1) {
+    const double p1 = __dmul_rn(s1, ctl->scale2);
+    double p0 = __dsub_rn(1.0, p1);
+    if (!(p0 > 0.0)) p0 = 0.0;
+    const double total = __dadd_rn(p0, p1);
+    const double chosen = __dmul_rn(ctl->draws[step], uniform_scale(total));
+    const int r = (p0 <= chosen) ? 1 : 0;
+    double prob = r ? p1 : p0;
+    if (!(prob > DBL_MIN)) prob = DBL_MIN;
+    const double p = 1.0 / sqrt(prob);
+    const double pf = (double)(T)p;
+    ctl->p[step] = p;
+    ctl->scale2 = __dmul_rn(__dmul_rn(ctl->scale2, pf), pf);
+    ctl->M = ctl->M | bit;
+    ctl->V = ctl->V | (r ? bit : 0ull);
+    ctl->result |= (uint64_t)r << step;
+    ctl->steps = step + 1;
+}
+
+template <class T, bool kFF>
+__device__ __forceinline__ double measure_norm(const void *__restrict__ st, uint32_t n, uint64_t M, uint64_t V) {
+    const uint64_t count = 1ull << (n - __popcll(M));
+    if constexpr (kFF) return masked_norm_body_ff((const float4 *)st, count, M, V);
+    else return masked_norm_body<T>((const cx<T> *)st, count, M, V);
+}
+
 template <class T, bool kFF = false>
 __global__ void __launch_bounds__(kReduceThreads)
     k_measure_step(const void *__restrict__ st, uint32_t n, MeasureCtl *ctl, uint32_t step, ReduceScratch rs) {
     const uint64_t bit = 1ull << ctl->qubit[step];
-    const uint64_t M = ctl->M | bit, V = ctl->V | bit;
-    const uint64_t count = 1ull << (n - __popcll(M));
-    double v;
-    if constexpr (kFF)
-        v = masked_norm_body_ff((const float4 *)st, count, M, V);
-    else
-        v = masked_norm_body<T>((const cx<T> *)st, count, M, V);
+    const double v = measure_norm<T, kFF>(st, n, ctl->M | bit, ctl->V | bit);
     if (threadIdx.x == 0) rs.partials[blockIdx.x] = v;
     if (last_block(rs.ticket)) {
         const double s1 = sum_partials(rs.partials, gridDim.x, 1, 0);
         if (threadIdx.x == 0) {
-            // QubitManager::do_measure decision (src/quantum_execution.rs:278-287)
-            const double p1 = __dmul_rn(s1, ctl->scale2);
-            double p0 = __dsub_rn(1.0, p1);
-            if (!(p0 > 0.0)) p0 = 0.0;
-            const double total = __dadd_rn(p0, p1);
-            const double chosen = __dmul_rn(ctl->draws[step], uniform_scale(total));
-            const int r = (p0 <= chosen) ? 1 : 0;
-            double prob = r ? p1 : p0;
-            if (!(prob > DBL_MIN)) prob = DBL_MIN;
-            const double p = 1.0 / sqrt(prob);
-            const double pf = (double)(T)p;
-            ctl->p[step] = p;
-            ctl->scale2 = __dmul_rn(__dmul_rn(ctl->scale2, pf), pf);
-            ctl->M = ctl->M | bit;
-            ctl->V = ctl->V | (r ? bit : 0ull);
-            ctl->result |= (uint64_t)r << step;
-            ctl->steps = step + 1;
+            measure_decide<T>(ctl, step, bit, s1);
             *rs.ticket = 0;
         }
     }
 }
 
-template <class T>
-cudaError_t launch_measure_step(const void *st, uint32_t n, MeasureCtl *ctl, uint32_t step,
-                                const ReduceScratch &rs, cudaStream_t s) {
-    k_measure_step<T><<<kReduceBlocks, kReduceThreads, 0, s>>>(st, n, ctl, step, rs);
-    count_launch();
-    return cudaGetLastError();
+// Steps [step, steps) by one block: once few amplitudes are left, a step is
+// shorter than its launch (24 qubits: 14 of 24 steps, 13 us each before).
+template <class T, bool kFF>
+__global__ void __launch_bounds__(kReduceThreads)
+    k_measure_tail(const void *__restrict__ st, uint32_t n, MeasureCtl *ctl, uint32_t step, uint32_t steps) {
+    for (; step < steps; step++) {
+        const uint64_t bit = 1ull << ctl->qubit[step];
+        const double s1 = measure_norm<T, kFF>(st, n, ctl->M | bit, ctl->V | bit);
+        __syncthreads();
+        if (threadIdx.x == 0) measure_decide<T>(ctl, step, bit, s1);
+        __syncthreads();
+    }
 }
 
-cudaError_t launch_measure_step_ff(const void *st, uint32_t n, MeasureCtl *ctl, uint32_t step,
-                                   const ReduceScratch &rs, cudaStream_t s) {
-    k_measure_step<double, true><<<kReduceBlocks, kReduceThreads, 0, s>>>(st, n, ctl, step, rs);
-    count_launch();
-    return cudaGetLastError();
+// Amplitudes a step reads below which one block takes the remaining steps.
+constexpr uint64_t kMeasureTail = 1ull << 12;
+
+template <class T, bool kFF>
+static cudaError_t measure_steps(const void *st, uint32_t n, MeasureCtl *ctl, uint32_t steps, const ReduceScratch &rs,
+                                 cudaStream_t s) {
+    for (uint32_t k = 0; k < steps; k++) {
+        const uint64_t count = 1ull << (n - (k + 1));  // the qubits are distinct
+        if (count <= kMeasureTail) {
+            k_measure_tail<T, kFF><<<1, kReduceThreads, 0, s>>>(st, n, ctl, k, steps);
+            count_launch();
+            return cudaGetLastError();
+        }
+        const unsigned grid = (unsigned)std::min<uint64_t>(kReduceBlocks, count / (4 * kReduceThreads));
+        k_measure_step<T, kFF><<<grid, kReduceThreads, 0, s>>>(st, n, ctl, k, rs);
+        count_launch();
+        const cudaError_t e = cudaGetLastError();
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
+}
+
+template <class T>
+cudaError_t launch_measure_steps(const void *st, uint32_t n, MeasureCtl *ctl, uint32_t steps, const ReduceScratch &rs,
+                                 cudaStream_t s) {
+    return measure_steps<T, false>(st, n, ctl, steps, rs, s);
+}
+
+cudaError_t launch_measure_steps_ff(const void *st, uint32_t n, MeasureCtl *ctl, uint32_t steps,
+                                    const ReduceScratch &rs, cudaStream_t s) {
+    return measure_steps<double, true>(st, n, ctl, steps, rs, s);
 }
 
 // ---- collapse -----------------------------------------------------------------
@@ -1046,6 +1096,28 @@ __device__ __forceinline__ double weight(cx<T> a) {
     return __fma_rn(r, r, __dmul_rn(i, i));
 }
 
+// The same for the float-float resident form; kept as a float-float value.
+__device__ __forceinline__ ff::f2 weight_ff(float4 f) {
+    const ff::f2 re{f.x, f.z}, im{f.y, f.w}, w = ff::dot2(re, re, im, im);
+    if (w.h > 1.00001e-30f) return w;
+    if (w.h < 0.99999e-30f || !((double)w.h + (double)w.l > 1e-30)) return ff::f2{0.f, 0.f};
+    return w;
+}
+__device__ __forceinline__ ff::f2 weight_ff(cx<float> a) {  // exact products, summed in float-float
+    if (!above_eps(a)) return ff::f2{0.f, 0.f};
+    return DiagArith<float>::prob(a);
+}
+// Weight of amplitude i of a state of either type or form.
+template <class T, bool kFF>
+__device__ __forceinline__ double weight_at(const void *st, uint64_t i) {
+    if constexpr (kFF) {
+        const ff::f2 w = weight_ff(reinterpret_cast<const float4 *>(st)[i]);
+        return (double)w.h + (double)w.l;
+    } else {
+        return weight(reinterpret_cast<const cx<T> *>(st)[i]);
+    }
+}
+
 int dump_blocks(uint32_t n) {
     const uint64_t ns = 1ull << n;
     uint64_t R = ns / 4096;
@@ -1128,24 +1200,30 @@ cudaError_t launch_dump_write(const void *st, uint32_t n, const uint64_t *offset
 // Both kernels walk a block's range in chunks of blockDim with the same scan,
 // so the in-block running sums of the pick kernel end exactly at the block
 // sums the host prefixes.
-template <class T>
-__global__ void __launch_bounds__(256) k_weight_blocksum(const cx<T> *__restrict__ st, uint64_t R, double *blocksum) {
+// (Sums only: the picks scan the few blocks that hold a shot.  Scanning every
+// block here too kept the FP64 pipe busy for 372 us on 24 qubits.)
+template <class T, bool kFF>
+__global__ void __launch_bounds__(256) k_weight_blocksum(const void *__restrict__ st, uint64_t R, double *blocksum) {
     const uint64_t base = (uint64_t)blockIdx.x * R;
-    double running = 0.0;
-    for (uint64_t c0 = 0; c0 < R; c0 += blockDim.x) {
-        const uint64_t i = c0 + threadIdx.x;
-        const double w = (i < R) ? weight(st[base + i]) : 0.0;
-        double total;
-        block_inclusive_scan(w, &total);
-        running = running + total;
-        __syncthreads();
+    double sum = 0.0;
+    if constexpr (sizeof(T) == 8 && !kFF) {
+#pragma unroll 4
+        for (uint64_t i = threadIdx.x; i < R; i += 256) sum += weight_at<T, kFF>(st, base + i);
+    } else {
+        using Mem = typename std::conditional<kFF, float4, cx<float>>::type;
+        ff::f2 acc{0.f, 0.f};
+#pragma unroll 4
+        for (uint64_t i = threadIdx.x; i < R; i += 256)
+            acc = ff::add(acc, weight_ff(reinterpret_cast<const Mem *>(st)[base + i]));
+        sum = (double)acc.h + (double)acc.l;
     }
-    if (threadIdx.x == 0) blocksum[blockIdx.x] = running;
+    const double t = block_sum(sum);
+    if (threadIdx.x == 0) blocksum[blockIdx.x] = t;
 }
 
-template <class T>
+template <class T, bool kFF>
 __global__ void __launch_bounds__(256)
-    k_sample_pick(const cx<T> *__restrict__ st, uint64_t R, const uint32_t *blocks, const uint64_t *shot_begin,
+    k_sample_pick(const void *__restrict__ st, uint64_t R, const uint32_t *blocks, const uint64_t *shot_begin,
                   const double *prefix, const double *chosen, uint64_t *pick) {
     __shared__ double pre[256];
     __shared__ uint64_t last_nz;
@@ -1159,7 +1237,7 @@ __global__ void __launch_bounds__(256)
     __syncthreads();
     for (uint64_t c0 = 0; c0 < R && sh < sh_end; c0 += blockDim.x) {
         const uint64_t i = c0 + threadIdx.x;
-        const double w = (i < R) ? weight(st[base + i]) : 0.0;
+        const double w = (i < R) ? weight_at<T, kFF>(st, base + i) : 0.0;
         double total;
         const double incl = block_inclusive_scan(w, &total);
         pre[threadIdx.x] = P + (running + incl);
@@ -1195,23 +1273,27 @@ __global__ void __launch_bounds__(256)
 }
 
 template <class T>
-cudaError_t launch_weight_blocksum(const void *st, uint32_t n, double *blocksum, cudaStream_t s) {
+cudaError_t launch_weight_blocksum(const void *st, uint32_t n, bool ff_resident, double *blocksum, cudaStream_t s) {
     const int B = sample_blocks(n);
     const uint64_t R = (1ull << n) / B;
-    k_weight_blocksum<T><<<B, 256, 0, s>>>((const cx<T> *)st, R, blocksum);
+    if (sizeof(T) == 8 && ff_resident) k_weight_blocksum<double, true><<<B, 256, 0, s>>>(st, R, blocksum);
+    else k_weight_blocksum<T, false><<<B, 256, 0, s>>>(st, R, blocksum);
     count_launch();
     return cudaGetLastError();
 }
 
 template <class T>
-cudaError_t launch_sample_pick(const void *st, uint32_t n, const uint32_t *blocks, uint32_t nblocks_with_shots,
+cudaError_t launch_sample_pick(const void *st, uint32_t n, bool ff_resident, const uint32_t *blocks,
+                               uint32_t nblocks_with_shots,
                                const uint64_t *shot_begin, const double *prefix, const double *chosen,
                                uint64_t *pick, cudaStream_t s) {
     const int B = sample_blocks(n);
     const uint64_t R = (1ull << n) / B;
     if (nblocks_with_shots == 0) return cudaSuccess;
-    k_sample_pick<T><<<nblocks_with_shots, 256, 0, s>>>((const cx<T> *)st, R, blocks, shot_begin, prefix, chosen,
-                                                          pick);
+    if (sizeof(T) == 8 && ff_resident)
+        k_sample_pick<double, true><<<nblocks_with_shots, 256, 0, s>>>(st, R, blocks, shot_begin, prefix, chosen, pick);
+    else
+        k_sample_pick<T, false><<<nblocks_with_shots, 256, 0, s>>>(st, R, blocks, shot_begin, prefix, chosen, pick);
     count_launch();
     return cudaGetLastError();
 }
@@ -1351,8 +1433,8 @@ namespace kbwg {
 #define INST(T)                                                                                               \
     template cudaError_t launch_masked_norm<T>(const void *, uint32_t, uint64_t, uint64_t, const ReduceScratch &, \
                                                cudaStream_t);                                                 \
-    template cudaError_t launch_measure_step<T>(const void *, uint32_t, MeasureCtl *, uint32_t,                \
-                                                const ReduceScratch &, cudaStream_t);                         \
+    template cudaError_t launch_measure_steps<T>(const void *, uint32_t, MeasureCtl *, uint32_t,               \
+                                                 const ReduceScratch &, cudaStream_t);                        \
     template cudaError_t launch_collapse<T>(void *, uint32_t, const MeasureCtl *, uint64_t, uint64_t, double,   \
                                             cudaStream_t);                                                    \
     template cudaError_t launch_pauli_group<T>(const void *, uint32_t, const PauliGroup &, const ReduceScratch &, \
@@ -1362,8 +1444,8 @@ namespace kbwg {
     template cudaError_t launch_dump_count<T>(const void *, uint32_t, uint64_t *, cudaStream_t);               \
     template cudaError_t launch_dump_write<T>(const void *, uint32_t, const uint64_t *, const DumpSpec &,        \
                                               uint64_t *, double *, double *, cudaStream_t);                  \
-    template cudaError_t launch_weight_blocksum<T>(const void *, uint32_t, double *, cudaStream_t);            \
-    template cudaError_t launch_sample_pick<T>(const void *, uint32_t, const uint32_t *, uint32_t,             \
+    template cudaError_t launch_weight_blocksum<T>(const void *, uint32_t, bool, double *, cudaStream_t);      \
+    template cudaError_t launch_sample_pick<T>(const void *, uint32_t, bool, const uint32_t *, uint32_t,       \
                                                const uint64_t *, const double *, const double *, uint64_t *,  \
                                                cudaStream_t);
 INST(float)
