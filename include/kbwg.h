@@ -251,7 +251,8 @@ int32_t kbwg_batch_gradient(uintptr_t num_qubits, int32_t precision, uint32_t fl
                             const double *coefficients, uintptr_t n_strings, uint32_t max_checkpoints,
                             double *energy, double *gradient);
 
-/* Free the pooled registers no call is using. */
+/* Free the pooled registers no call is using, and the buffer (up to 4 GiB)
+ * that kbwg_batch_circuits_exp_value keeps between calls. */
 int32_t kbwg_batch_release(void);
 
 /* Many BatchExecution::exp_value requests (src/quantum_execution.rs:392-405,

@@ -152,6 +152,58 @@ def load(path=None):
     return lib
 
 
+# Native packers of gate lists and Hamiltonians (native/pack.c); None where
+# they could not be built: the binding then packs in Python.
+_pack = None
+_pack_tried = False
+
+
+def _packer():
+    global _pack, _pack_tried
+    if not _pack_tried:
+        _pack_tried = True
+        path = os.path.join(os.path.dirname(LIB_PATH), "_kbwgpack.so")
+        if os.path.exists(path):
+            try:
+                lib = ctypes.PyDLL(path)  # the functions walk Python objects: the interpreter lock stays held
+            except OSError:
+                return None
+            obj, lng, ptr = ctypes.py_object, ctypes.c_long, ctypes.c_void_p
+            for fn, args in ((lib.kbwg_pack_gates, [obj, ptr, lng]), (lib.kbwg_count_terms, [obj, lng]),
+                             (lib.kbwg_pack_terms, [obj, lng, lng, ptr, ptr, ptr, ptr])):
+                fn.restype = lng
+                fn.argtypes = args
+            _pack = lib
+    return _pack
+
+
+def pack_gates(circuit, buf, n):
+    """Fill n kbwg_gate records of the numpy buffer; False: not plain lists of
+    numbers (or no packer), nothing promised about the buffer."""
+    lib = _packer()
+    return lib is not None and lib.kbwg_pack_gates(circuit, buf.ctypes.data, n) == 0
+
+
+def pack_terms(ham):
+    """(paulis, qubits, offsets, coefficients, strings) arrays of a
+    Hamiltonian, or None as pack_gates."""
+    import numpy as np
+    lib = _packer()
+    if lib is None or type(ham) not in (list, tuple):
+        return None
+    n = len(ham)
+    total = lib.kbwg_count_terms(ham, n)
+    if total < 0:
+        return None
+    pa = np.zeros(max(total, 1), np.uint8)
+    qa = np.zeros(max(total, 1), np.uintp)
+    oa = np.zeros(n + 1, np.uintp)
+    ca = np.zeros(max(n, 1), np.float64)
+    if lib.kbwg_pack_terms(ham, n, total, pa.ctypes.data, qa.ctypes.data, oa.ctypes.data, ca.ctypes.data) != 0:
+        return None
+    return pa, qa, oa, ca, n
+
+
 def check(code):
     if code != OK:
         msg = _lib.kbwg_last_error().decode(errors="replace") if _lib is not None else ""

@@ -10,6 +10,7 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(HERE)
@@ -68,6 +69,28 @@ def write_jit_sources():
             f.write(out)
 
 
+PACK_SRC = os.path.join(HERE, "native", "pack.c")
+PACK_LIB = os.path.join(HERE, "_kbwgpack.so")
+
+
+def build_pack():
+    """The Python binding's packers (host C, CPython API).  Where the Python
+    headers or a C compiler are missing the binding packs in Python."""
+    inc = sysconfig.get_paths()["include"]
+    cc = shutil.which("gcc") or shutil.which("cc")
+    if cc is None or not os.path.exists(os.path.join(inc, "Python.h")):
+        return None
+    if os.path.exists(PACK_LIB) and os.path.getmtime(PACK_LIB) >= os.path.getmtime(PACK_SRC):
+        return PACK_LIB
+    tmp = PACK_LIB + ".tmp%d" % os.getpid()
+    r = subprocess.run([cc, "-std=c11", "-O2", "-fPIC", "-shared", "-I", inc, PACK_SRC, "-o", tmp],
+                       capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError("building %s failed:\n%s" % (PACK_SRC, r.stderr))
+    os.replace(tmp, PACK_LIB)
+    return PACK_LIB
+
+
 def _compile(src, verbose):
     obj = os.path.join(OBJ, os.path.basename(src) + ".o")
     newest_dep = max(os.path.getmtime(p) for p in headers() + [src, __file__, JIT_INC])
@@ -106,6 +129,7 @@ def build(verbose=False, force=False):
         if r.returncode != 0:
             raise RuntimeError("link failed:\n%s\n%s" % (" ".join(cmd), r.stderr))
         os.replace(tmp, LIB)
+    build_pack()
     return LIB
 
 

@@ -624,6 +624,13 @@ struct AdjScratch {
         std::vector<const void *> f;
     };
     std::vector<Kernels> kernels;  // final entries only (compiled, loaded or failed)
+    // planned segments by structure (kinds, targets, controls): a loop over
+    // the same ansatz plans its reverse sweeps once
+    struct Plan {
+        std::vector<uint64_t> sig;
+        std::vector<PlannedSweep> sweeps;
+    };
+    std::vector<Plan> plans;
     void release_states() {
         if (lam) cudaFree(lam);
         lam = nullptr;
@@ -641,9 +648,11 @@ struct AdjScratch {
         dprog = hprog = nullptr;
         partials_cap = grads_cap = dprog_cap = hprog_cap = 0;
         kernels.clear();
+        plans.clear();
     }
 };
 constexpr size_t kAdjKernelEntries = 256;
+constexpr size_t kAdjPlanEntries = 32;
 
 void release_adjoint(Sim &s) {
     AdjScratch *a = (AdjScratch *)s.adj;
@@ -789,8 +798,23 @@ static cudaError_t plan_segment(Sim &s, AdjScratch &sc, const std::vector<GateDe
         rev.push_back(inverse_desc(fwd[j], angles[j]));
         rev_src.push_back(j);
     }
-    // (one gate short of a full program: the deferred factor is the last one)
-    std::vector<PlannedSweep> plan = plan_sweeps(s.n, K, R, rev.data(), rev.size(), false, kMaxSweepGates - 1);
+    std::vector<uint64_t> sig(2 * rev.size());
+    for (size_t i = 0; i < rev.size(); i++) {
+        sig[2 * i] = (uint64_t)rev[i].kind | ((uint64_t)rev[i].target << 8);
+        sig[2 * i + 1] = rev[i].ctrl;
+    }
+    const AdjScratch::Plan *known = nullptr;
+    for (const AdjScratch::Plan &pl : sc.plans)
+        if (pl.sig == sig) known = &pl;
+    if (!known) {
+        // (one gate short of a full program: the deferred factor is the last one)
+        if (sc.plans.size() >= kAdjPlanEntries) sc.plans.erase(sc.plans.begin());
+        sc.plans.push_back({sig, plan_sweeps(s.n, K, R, rev.data(), rev.size(), false, kMaxSweepGates - 1)});
+        known = &sc.plans.back();
+    }
+    std::vector<PlannedSweep> plan = known->sweeps;
+    for (PlannedSweep &sw : plan)
+        for (size_t i = 0; i < sw.gates.size(); i++) memcpy(sw.gates[i].c, rev[sw.src[i]].c, sizeof sw.gates[i].c);
     DdFactor g;
     // gradient info per sweep: type | slot << 4 per gate, then the gate of each slot
     std::vector<std::vector<uint32_t>> metas(plan.size());

@@ -1435,6 +1435,7 @@ int32_t kbwg_batch_release(void) {
             }
     }
     for (kbwg_sim *s : idle) kbwg_free(s);
+    batch_release_workspace();
     return KBWG_OK;
     GUARD_END
 }

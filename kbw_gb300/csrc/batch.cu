@@ -32,6 +32,7 @@
 #include <memory>
 #include <mutex>
 #include <thread>
+#include <unordered_map>
 #include <vector>
 
 #include "../../include/kbwg.h"
@@ -529,6 +530,70 @@ static void batch_parallel_for(size_t n, F &&fn) {
     if (first) std::rethrow_exception(first);
 }
 
+// Device buffer of a call, kept for the next one (the largest up to
+// kBatchKeepBytes, one per process): allocating and freeing a gigabyte costs
+// milliseconds of a call.  Calls that overlap take their own; a call's work
+// is finished when it gives its buffer back.  kbwg_batch_release frees it.
+constexpr size_t kBatchKeepBytes = 4ull << 30;
+static std::mutex g_batch_mu;
+static int g_batch_dev = -1;
+static void *g_batch_buf = nullptr;
+static size_t g_batch_cap = 0;
+
+static cudaError_t batch_take(int dev, size_t bytes, char **buf, size_t *cap) {
+    {
+        std::lock_guard<std::mutex> lk(g_batch_mu);
+        if (g_batch_buf && g_batch_dev == dev && g_batch_cap >= bytes) {
+            *buf = (char *)g_batch_buf;
+            *cap = g_batch_cap;
+            g_batch_buf = nullptr;
+            return cudaSuccess;
+        }
+    }
+    cudaError_t e = cudaMalloc((void **)buf, bytes);
+    if (e == cudaErrorMemoryAllocation) {  // the kept buffer may be what is missing
+        cudaGetLastError();
+        batch_release_workspace();
+        e = cudaMalloc((void **)buf, bytes);
+    }
+    *cap = bytes;
+    return e;
+}
+
+static void batch_give(int dev, char *buf, size_t cap) {
+    void *drop = buf;
+    int drop_dev = dev;
+    if (cap <= kBatchKeepBytes) {
+        std::lock_guard<std::mutex> lk(g_batch_mu);
+        if (!g_batch_buf || (g_batch_dev == dev && g_batch_cap < cap)) {
+            drop = g_batch_buf;
+            drop_dev = g_batch_dev;
+            g_batch_buf = buf;
+            g_batch_cap = cap;
+            g_batch_dev = dev;
+        }
+    }
+    (void)drop_dev;  // (the dropped buffer is on this device or null)
+    if (drop) cudaFree(drop);
+}
+
+void batch_release_workspace() {
+    void *buf = nullptr;
+    int dev = -1, cur = -1;
+    {
+        std::lock_guard<std::mutex> lk(g_batch_mu);
+        buf = g_batch_buf;
+        dev = g_batch_dev;
+        g_batch_buf = nullptr;
+        g_batch_cap = 0;
+    }
+    if (!buf) return;
+    cudaGetDevice(&cur);
+    if (cur != dev) cudaSetDevice(dev);
+    cudaFree(buf);
+    if (cur != dev && cur >= 0) cudaSetDevice(cur);
+}
+
 template <class P, int K, int R>
 static int32_t batch_run(int arith, std::vector<BatchCircuitIn> &circs, double *energies) {
     using BK = BatchKernel<P, K, R>;
@@ -539,13 +604,49 @@ static int32_t batch_run(int arith, std::vector<BatchCircuitIn> &circs, double *
                   std::string("batch circuits: ") + what + ": " + cudaGetErrorString(e));
         return e == cudaErrorMemoryAllocation ? (int32_t)KBWG_ENOMEM : (int32_t)KBWG_ECUDA;
     };
-    // plan every circuit (in parallel: the circuits are independent)
+    // plan every circuit (in parallel: the circuits are independent), those of
+    // one structure (register size, kinds, targets, controls) once
+    std::vector<std::vector<uint64_t>> sigs(circs.size());
     batch_parallel_for(circs.size(), [&](size_t c) {
         BatchCircuitIn &ci = circs[c];
-        const uint32_t nplan = std::max<uint32_t>(ci.n, (uint32_t)K);  // small registers padded with |0> qubits
         ci.gates = defer_factors(arith, ci.gates.data(), ci.gates.size());
-        const std::vector<PlannedSweep> plan =
-            plan_sweeps(nplan, K, R, ci.gates.data(), ci.gates.size(), false, kMaxSweepGates);
+        std::vector<uint64_t> &sig = sigs[c];
+        sig.reserve(2 * ci.gates.size() + 1);
+        sig.push_back(ci.n);
+        for (const GateDesc &g : ci.gates) {
+            sig.push_back((uint64_t)g.kind | ((uint64_t)g.target << 8));
+            sig.push_back(g.ctrl);
+        }
+    });
+    struct SigHash {
+        size_t operator()(const std::vector<uint64_t> *v) const {
+            uint64_t h = 1469598103934665603ull;  // FNV-1a over the words
+            for (uint64_t w : *v) {
+                h ^= w;
+                h *= 1099511628211ull;
+            }
+            return (size_t)h;
+        }
+    };
+    struct SigEqual {
+        bool operator()(const std::vector<uint64_t> *a, const std::vector<uint64_t> *b) const { return *a == *b; }
+    };
+    std::unordered_map<const std::vector<uint64_t> *, size_t, SigHash, SigEqual> known;
+    std::vector<size_t> plan_of(circs.size()), first;
+    for (size_t c = 0; c < circs.size(); c++) {
+        const auto ins = known.emplace(&sigs[c], first.size());
+        if (ins.second) first.push_back(c);
+        plan_of[c] = ins.first->second;
+    }
+    std::vector<std::vector<PlannedSweep>> plans(first.size());
+    batch_parallel_for(first.size(), [&](size_t k) {
+        const BatchCircuitIn &ci = circs[first[k]];
+        const uint32_t nplan = std::max<uint32_t>(ci.n, (uint32_t)K);  // small registers padded with |0> qubits
+        plans[k] = plan_sweeps(nplan, K, R, ci.gates.data(), ci.gates.size(), false, kMaxSweepGates);
+    });
+    batch_parallel_for(circs.size(), [&](size_t c) {
+        BatchCircuitIn &ci = circs[c];
+        const std::vector<PlannedSweep> &plan = plans[plan_of[c]];
         size_t placed = 0;
         for (const PlannedSweep &sw : plan) {
             BatchSweep b;
@@ -560,7 +661,9 @@ static int32_t batch_run(int arith, std::vector<BatchCircuitIn> &circs, double *
                 b.stage_layout[i] = sw.stage_layout[i];
                 b.stage_end[i] = sw.stage_end[i];
             }
-            for (TileGate t : sw.gates) {
+            for (size_t i = 0; i < sw.gates.size(); i++) {
+                TileGate t = sw.gates[i];
+                memcpy(t.c, ci.gates[sw.src[i]].c, sizeof t.c);
                 P::pack_host(t);
                 ci.prog.push_back(t);
             }
@@ -794,7 +897,8 @@ static int32_t batch_run(int arith, std::vector<BatchCircuitIn> &circs, double *
     e = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
     if (e != cudaSuccess) return fail(e, "stream");
     char *dbuf = nullptr;
-    e = cudaMalloc(&dbuf, o_s + (size_t)state_elems * sizeof(Mem));
+    size_t dcap = 0;
+    e = batch_take(dev, o_s + (size_t)state_elems * sizeof(Mem), &dbuf, &dcap);
     if (e != cudaSuccess) {
         cudaStreamDestroy(st);
         return fail(e, "buffers");
@@ -842,8 +946,10 @@ static int32_t batch_run(int arith, std::vector<BatchCircuitIn> &circs, double *
     }
     if (e == cudaSuccess) e = copy_async(energies, a.energies, eb, cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = copy_async(&err_flag, a.err, sizeof(int), cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-    cudaFree(dbuf);
+    const cudaError_t es = cudaStreamSynchronize(st);  // (also after a failure: the buffer goes back idle)
+    if (e == cudaSuccess) e = es;
+    if (e == cudaSuccess) batch_give(dev, dbuf, dcap);
+    else cudaFree(dbuf);
     cudaStreamDestroy(st);
     if (e != cudaSuccess) return fail(e, "run");
     if (err_flag) {

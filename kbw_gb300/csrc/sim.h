@@ -179,6 +179,9 @@ int32_t batch_circuits(int precision, uint32_t flags, size_t ncirc, const uint32
                        const uintptr_t *qubits, const uintptr_t *term_offsets, const double *coefficients,
                        const uintptr_t *ham_offsets, double *energies);
 
+// Free the buffer batch_circuits keeps between calls.
+void batch_release_workspace();
+
 // Adjoint gradient (adjoint.cu).  fwd: the circuit; angles: each gate's
 // angle; gtype: GT_* per gate (GT_NONE if not differentiated).  Writes E and
 // dE/dtheta per gate; the handle ends in |0...0>.  Returns 0 or a KBWG_* code.

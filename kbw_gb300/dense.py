@@ -26,7 +26,12 @@ def _sizes(seq):
 
 
 def _p(a, t):
-    return a.ctypes.data_as(ctypes.POINTER(t)) if a.size else None
+    """Pointer argument to a contiguous array's first element (keeps the array alive)."""
+    if not a.size:
+        return None
+    if not a.flags.writeable:
+        return a.ctypes.data_as(ctypes.POINTER(t))
+    return ctypes.byref(t.from_buffer(a))
 
 
 class DenseGB300:
@@ -156,20 +161,10 @@ class DenseGB300:
 
     def exp_value(self, hamiltonian):
         """hamiltonian: list of (coefficient, [(pauli_code, qubit), ...])."""
-        paulis, qubits, offsets, coefs = [], [], [0], []
-        for coef, terms in hamiltonian:
-            for p, q in terms:
-                paulis.append(int(p))
-                qubits.append(int(q))
-            offsets.append(len(paulis))
-            coefs.append(float(coef))
-        pa = np.ascontiguousarray(paulis if paulis else [0], dtype=np.uint8)
-        qa = np.ascontiguousarray(qubits if qubits else [0], dtype=np.uintp)
-        oa = np.ascontiguousarray(offsets, dtype=np.uintp)
-        ca = np.ascontiguousarray(coefs if coefs else [0.0], dtype=np.float64)
+        pa, qa, oa, ca, ns = _ham_arrays(hamiltonian)
         out = ctypes.c_double()
         N.check(self._lib.kbwg_exp_value(self._h, _p(pa, ctypes.c_uint8), _p(qa, ctypes.c_size_t),
-                                         _p(oa, ctypes.c_size_t), _p(ca, ctypes.c_double), len(coefs),
+                                         _p(oa, ctypes.c_size_t), _p(ca, ctypes.c_double), ns,
                                          ctypes.byref(out)))
         return out.value
 
@@ -457,10 +452,10 @@ def _mask(cs):
 
 def _gate_array(circuit):
     """kbwg_gate records of a (kind, target, controls, angle) list, as a
-    ctypes array over one numpy buffer (filled column by column)."""
+    ctypes array over one numpy buffer (filled natively, else column by column)."""
     n = len(circuit)
     buf = np.zeros(max(n, 1), _GATE_DT)
-    if n:
+    if n and not N.pack_gates(circuit, buf, n):
         kinds, targets, ctrls, angles = zip(*circuit)
         buf["kind"][:n] = kinds
         buf["target"][:n] = targets
@@ -470,6 +465,9 @@ def _gate_array(circuit):
 
 
 def _ham_arrays(hamiltonian):
+    packed = N.pack_terms(hamiltonian)
+    if packed is not None:
+        return packed
     paulis, qubits, offsets, coefs = [], [], [0], []
     for coef, terms in hamiltonian:
         for p, q in terms:
