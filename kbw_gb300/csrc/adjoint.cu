@@ -479,9 +479,9 @@ __global__ void __launch_bounds__(AdjKernel<P, K, R>::kThreads, 2)
     const uint32_t chunk_bytes = chunk * (uint32_t)sizeof(Mem);
     const uint64_t lowmask = chunk - 1;
 
-    for (uint32_t i = threadIdx.x; i < p.gate_count; i += blockDim.x) {
+    for (uint32_t i = threadIdx.x; i < p.gate_count + p.data_count; i += blockDim.x) {
         sg[i] = p.prog[i];
-        sinfo[i] = a.ginfo[i];
+        if (i < p.gate_count) sinfo[i] = a.ginfo[i];
     }
     for (uint32_t i = threadIdx.x; i < (uint32_t)AK::kWarps * kMaxSweepGates; i += blockDim.x) acc[i] = Wacc{};
     for (uint32_t c = threadIdx.x; c < nchunks; c += blockDim.x) {
@@ -551,6 +551,12 @@ __global__ void __launch_bounds__(AdjKernel<P, K, R>::kThreads, 2)
             for (uint32_t gi = g0; gi < g1; gi++) {
                 const TileGate &g = sg[gi];
                 if ((base & g.co) != g.co) continue;  // uniform over the tile
+                if (g.op == OP_SIGN) {
+                    const uint32_t S = sign_mask<P, K, R>(g, R0, F, base);
+                    flip_registers<P, R>(vp, S);
+                    flip_registers<P, R>(vl, S);
+                    continue;
+                }
                 const uint32_t info = sinfo[gi];
                 const int gt = (int)(info & 15u);
                 if (gt != GT_NONE) {
@@ -762,6 +768,16 @@ static void defer_sweep(PlannedSweep &sw, bool last, DdFactor &g, std::vector<do
     sw.gates.push_back(t);
     sw.stage_end.back()++;
     mult.push_back(1.0);
+    for (TileGate &x : sw.gates)  // (the rows of merged signs stand behind the gates)
+        if (x.cls == TG_SIGN) x.creg++;
+}
+
+// Merged Z and CZ gates of a reverse sweep, with room left for its factor.
+template <int K, int R>
+static void merge_reverse(PlannedSweep &sw) {
+    const PlannedSweep before = sw;
+    merge_signs(sw, K, R);
+    if (sw.gates.size() + sw.data.size() + 1 > (size_t)kMaxSweepGates) sw = before;
 }
 
 // One reverse sweep, planned: its parameters (program and gradient info
@@ -810,11 +826,13 @@ static cudaError_t plan_segment(Sim &s, AdjScratch &sc, const std::vector<GateDe
         // (one gate short of a full program: the deferred factor is the last one)
         if (sc.plans.size() >= kAdjPlanEntries) sc.plans.erase(sc.plans.begin());
         sc.plans.push_back({sig, plan_sweeps(s.n, K, R, rev.data(), rev.size(), false, kMaxSweepGates - 1)});
+        for (PlannedSweep &sw : sc.plans.back().sweeps) merge_reverse<K, R>(sw);
         known = &sc.plans.back();
     }
     std::vector<PlannedSweep> plan = known->sweeps;
     for (PlannedSweep &sw : plan)
-        for (size_t i = 0; i < sw.gates.size(); i++) memcpy(sw.gates[i].c, rev[sw.src[i]].c, sizeof sw.gates[i].c);
+        for (size_t i = 0; i < sw.src.size(); i++)
+            if (sw.src[i] != kNoSource) memcpy(sw.gates[i].c, rev[sw.src[i]].c, sizeof sw.gates[i].c);
     DdFactor g;
     // gradient info per sweep: type | slot << 4 per gate, then the gate of each slot
     std::vector<std::vector<uint32_t>> metas(plan.size());
@@ -828,6 +846,7 @@ static cudaError_t plan_segment(Sim &s, AdjScratch &sc, const std::vector<GateDe
         meta.assign(sw.gates.size(), 0);
         std::vector<uint32_t> gate_of_slot;
         for (size_t i = 0; i < sw.src.size(); i++) {
+            if (sw.src[i] == kNoSource) continue;
             const size_t j = rev_src[sw.src[i]];
             gate_mult[j] = mult[i];
             if (gtype[j] != GT_NONE) {
@@ -843,6 +862,7 @@ static cudaError_t plan_segment(Sim &s, AdjScratch &sc, const std::vector<GateDe
         memcpy(r.a.sw.hq, sw.hq, sizeof r.a.sw.hq);
         r.a.sw.nstages = (uint32_t)sw.stage_layout.size();
         r.a.sw.gate_count = (uint32_t)sw.gates.size();
+        r.a.sw.data_count = (uint32_t)sw.data.size();
         for (uint32_t i = 0; i < r.a.sw.nstages; i++) {
             r.a.sw.stage_layout[i] = sw.stage_layout[i];
             r.a.sw.stage_end[i] = sw.stage_end[i];
@@ -861,15 +881,19 @@ static cudaError_t plan_segment(Sim &s, AdjScratch &sc, const std::vector<GateDe
             key = fnv(key, &t, offsetof(TileGate, c));
             if (t.cls == TG_PI) key = fnv(key, &t.c[0], sizeof(double));
         }
+        // (merged signs are read from the program, not compiled in)
         key = fnv(key, "|", 1);
         // program (policy-packed constants) and gradient info into the staging bytes
         r.prog_off = progs.size();
-        progs.resize(progs.size() + sw.gates.size() * sizeof(TileGate));
+        progs.resize(progs.size() + (sw.gates.size() + sw.data.size()) * sizeof(TileGate));
         for (size_t i = 0; i < sw.gates.size(); i++) {
             TileGate t = sw.gates[i];
-            P::pack_host(t);
+            if (t.cls != TG_SIGN) P::pack_host(t);
             memcpy(progs.data() + r.prog_off + i * sizeof(TileGate), &t, sizeof t);
         }
+        if (!sw.data.empty())
+            memcpy(progs.data() + r.prog_off + sw.gates.size() * sizeof(TileGate), sw.data.data(),
+                   sw.data.size() * sizeof(TileGate));
         r.info_off = infos.size();
         const size_t nb = (meta.size() + gate_of_slot.size()) * sizeof(uint32_t);
         infos.resize(infos.size() + ((nb + 15) & ~(size_t)15));
@@ -1352,11 +1376,13 @@ static size_t check_adjoint_p(const Sim &s, const std::vector<GateDesc> &fwd, co
     const JitGeometry geo{AdjPolicyName<P>::s, K, R, AK::kThreads, 2};
     std::vector<std::string> srcs;
     for (PlannedSweep &sw : plan) {
+        merge_reverse<K, R>(sw);
         std::vector<double> mult;
         defer_sweep<P, R>(sw, &sw == &plan.back(), g, mult);
         std::vector<uint32_t> meta(sw.gates.size(), 0);
         uint32_t nslots = 0;
         for (size_t i = 0; i < sw.src.size(); i++) {
+            if (sw.src[i] == kNoSource) continue;
             const size_t j = rev_src[sw.src[i]];
             if (gtype[j] != GT_NONE) meta[i] = (uint32_t)gtype[j] | (nslots++ << 4);
         }

@@ -358,7 +358,7 @@ __device__ __forceinline__ void adjoint_sweep(typename P::Mem *__restrict__ phi,
     const uint32_t chunk_bytes = chunk * (uint32_t)sizeof(Mem);
     const uint64_t lowmask = chunk - 1;
 
-    for (uint32_t i = threadIdx.x; i < p.gate_count; i += blockDim.x) sg[i] = p.prog[i];
+    for (uint32_t i = threadIdx.x; i < p.gate_count + p.data_count; i += blockDim.x) sg[i] = p.prog[i];
     for (uint32_t i = threadIdx.x; i < (uint32_t)AK::kWarps * kMaxSweepGates; i += blockDim.x) acc[i] = Wacc{};
     for (uint32_t c = threadIdx.x; c < nchunks; c += blockDim.x) {
         uint64_t off = 0;

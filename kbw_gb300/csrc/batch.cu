@@ -44,7 +44,7 @@ namespace kbwg {
 
 struct BatchSweep {
     uint32_t l, m, nstages, gate_count;
-    uint32_t gate_off, pad;
+    uint32_t gate_off, data_count;
     uint8_t hq[16];
     uint8_t stage_layout[kMaxStages];
     uint16_t stage_end[kMaxStages];
@@ -117,7 +117,12 @@ struct BatchKernel {
     using Mem = typename P::Mem;
     static constexpr int kThreads = 32 << (K - kLaneBits - R);
     static constexpr size_t kTileBytes = sizeof(Mem) << K;
-    static constexpr size_t kSmem = 2 * kTileBytes + 256 * sizeof(uint64_t) + kMaxSweepGates * sizeof(TileGate) + 64 +
+    // complex64: three CTAs with one tile buffer each rather than two with two
+    // (24 warps hide the dispatch's latency better than the load ahead does:
+    // 1024 circuits 26.5 -> 23.3 ms; four CTAs spill, 28.2 ms).
+    static constexpr int kBuffers = sizeof(Mem) == 8 ? 1 : 2;
+    static constexpr int kCtas = sizeof(Mem) == 8 ? 3 : 2;
+    static constexpr size_t kSmem = kBuffers * kTileBytes + 256 * sizeof(uint64_t) + kMaxSweepGates * sizeof(TileGate) + 64 +
                                     32 * 8 + 64;
 };
 
@@ -224,9 +229,9 @@ __device__ __noinline__ bool batch_energy_pass(const BatchArgs &a, const BatchPa
     };
     const BatchTileTerm *tt = a.tterms + bp.term_off;
     issue_load(t0, 0);
-    if (t0 + 1 < t1) issue_load(t0 + 1, 1);
+    if (BK::kBuffers > 1 && t0 + 1 < t1) issue_load(t0 + 1, 1);
     for (uint64_t tau = t0; tau < t1; tau++) {
-        const uint32_t buf = (uint32_t)(tau - t0) & 1u;
+        const uint32_t buf = (uint32_t)(tau - t0) % (uint32_t)BK::kBuffers;
         const Mem *tile_mem = tiles_mem + ((size_t)buf << K);
         const uint64_t base = tile_base(tau);
         if (!tile_wait(bar + buf, phase[buf] & 1u, a.err)) return false;
@@ -270,14 +275,14 @@ __device__ __noinline__ bool batch_energy_pass(const BatchArgs &a, const BatchPa
             }
         }
         __syncthreads();  // the tile is read no more: a load may land in its buffer
-        if (tau + 2 < t1) issue_load(tau + 2, buf);
+        if (tau + BK::kBuffers < t1) issue_load(tau + BK::kBuffers, buf);
     }
     sum = acc.value();
     return true;
 }
 
 template <class P, int K, int R>
-__global__ void __launch_bounds__(BatchKernel<P, K, R>::kThreads, 2) k_batch_circuits(const __grid_constant__ BatchArgs a) {
+__global__ void __launch_bounds__(BatchKernel<P, K, R>::kThreads, BatchKernel<P, K, R>::kCtas) k_batch_circuits(const __grid_constant__ BatchArgs a) {
     using Amp = typename P::Amp;
     using Mem = typename P::Mem;
     using T = decltype(Mem{}.re);
@@ -287,7 +292,7 @@ __global__ void __launch_bounds__(BatchKernel<P, K, R>::kThreads, 2) k_batch_cir
     extern __shared__ __align__(128) unsigned char smem_raw[];
     Amp *tile = reinterpret_cast<Amp *>(smem_raw);  // two tile buffers
     Mem *tile_mem = reinterpret_cast<Mem *>(smem_raw);
-    unsigned char *q = smem_raw + 2 * BK::kTileBytes;
+    unsigned char *q = smem_raw + BK::kBuffers * BK::kTileBytes;
     uint64_t *chunk_off = reinterpret_cast<uint64_t *>(q);
     q += 256 * sizeof(uint64_t);
     TileGate *sg = reinterpret_cast<TileGate *>(q);
@@ -331,7 +336,8 @@ __global__ void __launch_bounds__(BatchKernel<P, K, R>::kThreads, 2) k_batch_cir
             for (uint32_t sw = s0; sw < s1; sw++) {
                 const BatchSweep &bs = a.sweeps[job.sweep_off + sw];
                 const uint32_t l = bs.l, m = bs.m, nst = bs.nstages;
-                for (uint32_t i = threadIdx.x; i < bs.gate_count; i += blockDim.x) sg[i] = a.prog[bs.gate_off + i];
+                for (uint32_t i = threadIdx.x; i < bs.gate_count + bs.data_count; i += blockDim.x)
+                    sg[i] = a.prog[bs.gate_off + i];
                 for (uint32_t c = threadIdx.x; c < (1u << m); c += blockDim.x) {
                     uint64_t off = 0;
                     for (uint32_t j = 0; j < m; j++) off |= (uint64_t)((c >> j) & 1u) << bs.hq[j];
@@ -359,10 +365,10 @@ __global__ void __launch_bounds__(BatchKernel<P, K, R>::kThreads, 2) k_batch_cir
                 const bool load = !whole && sw > 0;
                 if (load) {
                     issue_load(t0, 0);
-                    if (t0 + 1 < t1) issue_load(t0 + 1, 1);
+                    if (BK::kBuffers > 1 && t0 + 1 < t1) issue_load(t0 + 1, 1);
                 }
                 for (uint64_t tau = t0; tau < t1; tau++) {
-                    const uint32_t buf = whole ? 0u : (uint32_t)(tau - t0) & 1u;
+                    const uint32_t buf = whole ? 0u : (uint32_t)(tau - t0) % (uint32_t)BK::kBuffers;
                     Amp *tb = tile + ((size_t)buf << K);
                     const uint64_t base = tile_base(tau);
                     int layout = bs.stage_layout[0];
@@ -407,7 +413,7 @@ __global__ void __launch_bounds__(BatchKernel<P, K, R>::kThreads, 2) k_batch_cir
                         // the tile buffer is read no more (the load after next) once all threads pass here
                         fence_proxy_async();
                         __syncthreads();
-                        if (load && tau + 2 < t1) issue_load(tau + 2, buf);
+                        if (load && tau + BK::kBuffers < t1) issue_load(tau + BK::kBuffers, buf);
 #pragma unroll
                         for (int j = 0; j < NR; j++) {
                             const uint32_t u = F | ((uint32_t)j << R0);
@@ -639,15 +645,21 @@ static int32_t batch_run(int arith, std::vector<BatchCircuitIn> &circs, double *
         plan_of[c] = ins.first->second;
     }
     std::vector<std::vector<PlannedSweep>> plans(first.size());
+    std::vector<char> plan_ok(first.size());
     batch_parallel_for(first.size(), [&](size_t k) {
         const BatchCircuitIn &ci = circs[first[k]];
         const uint32_t nplan = std::max<uint32_t>(ci.n, (uint32_t)K);  // small registers padded with |0> qubits
         plans[k] = plan_sweeps(nplan, K, R, ci.gates.data(), ci.gates.size(), false, kMaxSweepGates);
+        size_t placed = 0;
+        for (PlannedSweep &sw : plans[k]) {
+            placed += sw.gates.size();
+            merge_signs(sw, K, R);
+        }
+        plan_ok[k] = placed == ci.gates.size() ? 1 : 0;
     });
     batch_parallel_for(circs.size(), [&](size_t c) {
         BatchCircuitIn &ci = circs[c];
         const std::vector<PlannedSweep> &plan = plans[plan_of[c]];
-        size_t placed = 0;
         for (const PlannedSweep &sw : plan) {
             BatchSweep b;
             memset(&b, 0, sizeof b);
@@ -656,6 +668,7 @@ static int32_t batch_run(int arith, std::vector<BatchCircuitIn> &circs, double *
             memcpy(b.hq, sw.hq, sizeof b.hq);
             b.nstages = (uint32_t)sw.stage_layout.size();
             b.gate_count = (uint32_t)sw.gates.size();
+            b.data_count = (uint32_t)sw.data.size();
             b.gate_off = (uint32_t)ci.prog.size();  // within the circuit; rebased below
             for (uint32_t i = 0; i < b.nstages; i++) {
                 b.stage_layout[i] = sw.stage_layout[i];
@@ -663,14 +676,16 @@ static int32_t batch_run(int arith, std::vector<BatchCircuitIn> &circs, double *
             }
             for (size_t i = 0; i < sw.gates.size(); i++) {
                 TileGate t = sw.gates[i];
-                memcpy(t.c, ci.gates[sw.src[i]].c, sizeof t.c);
-                P::pack_host(t);
+                if (sw.src[i] != kNoSource) {
+                    memcpy(t.c, ci.gates[sw.src[i]].c, sizeof t.c);
+                    P::pack_host(t);
+                }
                 ci.prog.push_back(t);
             }
-            placed += sw.gates.size();
+            ci.prog.insert(ci.prog.end(), sw.data.begin(), sw.data.end());
             ci.sweeps.push_back(b);
         }
-        ci.placed = placed == ci.gates.size();
+        ci.placed = plan_ok[plan_of[c]] != 0;
         if (ci.sweeps.empty() && ci.n > (uint32_t)K) {  // no gates: a sweep that writes |0...0>
             BatchSweep b;
             memset(&b, 0, sizeof b);

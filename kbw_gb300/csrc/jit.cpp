@@ -203,7 +203,7 @@ int env_int(const char *name, int dflt) {
     return atoi(v);
 }
 
-const char *kClassName[] = {"TG_X", "TG_Y", "TG_H", "TG_RX", "TG_RY", "TG_Z", "TG_P", "TG_RZ", "TG_PI", "TG_SCALE"};
+const char *kClassName[] = {"TG_X", "TG_Y", "TG_H", "TG_RX", "TG_RY", "TG_Z", "TG_P", "TG_RZ", "TG_PI", "TG_SCALE", "TG_SIGN"};
 
 // fn(w) for w in [0, count) on up to 32 threads.  An exception in an item
 // (an allocation failing) stops the remaining items and is rethrown on the
@@ -386,6 +386,13 @@ std::string jit_sweep_source(const JitGeometry &geo, const PlannedSweep &sw) {
         const size_t g1 = sw.stage_end[st];
         for (size_t i = g0; i < g1; i++) {
             const TileGate &t = sw.gates[i];
+            if (t.cls == TG_SIGN) {
+                snprintf(buf, sizeof buf,
+                         "    flip_registers<P, R>(v, jit::signs<P, K, R, %d>(sg[%zu], F, (uint64_t)base));\n",
+                         layout == LAYOUT_A ? kLaneBits : geo.K - geo.R, i);
+                s += buf;
+                continue;
+            }
             s += "    " + gate_stmt(t, "v", constants_of(t, i).c_str(), outer_cond(t, geo.wide)) + "\n";
         }
         g0 = g1;
@@ -433,6 +440,14 @@ std::string jit_adjoint_source(const JitGeometry &geo, const PlannedSweep &sw, c
         const size_t g1 = sw.stage_end[st];
         for (size_t i = g0; i < g1; i++) {
             const TileGate &t = sw.gates[i];
+            if (t.cls == TG_SIGN) {
+                snprintf(buf, sizeof buf,
+                         "    { const uint32_t S = jit::signs<P, K, R, %d>(sg[%zu], F, base); "
+                         "flip_registers<P, R>(vp, S); flip_registers<P, R>(vl, S); }\n",
+                         layout == LAYOUT_A ? kLaneBits : geo.K - geo.R, i);
+                s += buf;
+                continue;
+            }
             const int gt = (int)(ginfo[i] & 15u);
             const unsigned slot = ginfo[i] >> 4;
             std::string body;

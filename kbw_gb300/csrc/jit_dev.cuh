@@ -64,6 +64,12 @@ __device__ __forceinline__ void reg(typename P::Amp (&v)[1 << R], const typename
     }
 }
 
+// Many Z and CZ gates at once (TG_SIGN): the signs from the program's rows.
+template <class P, int K, int R, int R0>
+__device__ __forceinline__ uint32_t signs(const TileGate &g, uint32_t F, uint64_t base) {
+    return sign_mask<P, K, R>(g, R0, F, base);
+}
+
 template <class A>
 __device__ __forceinline__ A sel(bool c, const A &x, const A &y) {
     return c ? x : y;
@@ -209,7 +215,7 @@ __device__ __forceinline__ void sweep(typename P::Mem *__restrict__ st, const Sw
     const uint32_t chunk_bytes = chunk * (uint32_t)sizeof(Mem);
     const uint64_t lowmask = chunk - 1;
 
-    for (uint32_t i = threadIdx.x; i < p.gate_count; i += blockDim.x) sg[i] = p.prog[i];
+    for (uint32_t i = threadIdx.x; i < p.gate_count + p.data_count; i += blockDim.x) sg[i] = p.prog[i];
     for (uint32_t c = threadIdx.x; c < nchunks; c += blockDim.x) {
         uint64_t off = 0;
         for (uint32_t j = 0; j < m; j++) off |= (uint64_t)((c >> j) & 1u) << p.hq[j];

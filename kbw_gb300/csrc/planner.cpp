@@ -237,6 +237,110 @@ std::vector<PlannedSweep> plan_sweeps(uint32_t n, int K, int R, const GateDesc *
     return out;
 }
 
+// ---- merged signs -------------------------------------------------------------------
+void merge_signs(PlannedSweep &sw, int K, int R) {
+    std::vector<TileGate> out;
+    std::vector<uint32_t> src;
+    std::vector<uint16_t> ends;
+    size_t g0 = 0;
+    for (size_t st = 0; st < sw.stage_layout.size(); st++) {
+        const size_t g1 = sw.stage_end[st];
+        const int R0 = sw.stage_layout[st] == LAYOUT_A ? kLaneBits : K - R;
+        // groups: a gate joins the open one unless a gate since its first
+        // acts non-diagonally on one of its qubits
+        std::vector<int> group(g1 - g0, -1);
+        std::vector<std::vector<size_t>> members;
+        std::vector<int> outer_pairs;
+        uint32_t moved = 0;  // local targets of non-diagonal gates since the open group's first
+        for (size_t i = g0; i < g1; i++) {
+            const TileGate &t = sw.gates[i];
+            if (!tg_diagonal(t.cls)) {
+                moved |= 1u << t.tb;
+                continue;
+            }
+            if (t.cls != TG_Z) continue;
+            if (__builtin_popcount(t.cl) + __builtin_popcountll(t.co) > 1) continue;
+            const uint32_t local = t.cl | (t.tb == TG_OUTER ? 0u : 1u << t.tb);
+            const bool only_outer = local == 0;
+            if (members.empty() || (local & moved) || (only_outer && outer_pairs.back() == kSignPairs)) {
+                members.emplace_back();
+                outer_pairs.push_back(0);
+                moved = 0;
+            }
+            group[i - g0] = (int)members.size() - 1;
+            members.back().push_back(i);
+            outer_pairs.back() += only_outer ? 1 : 0;
+        }
+        for (size_t i = g0; i < g1; i++) {
+            const int gr = group[i - g0];
+            if (gr < 0 || members[(size_t)gr].size() < kSignMin) {
+                out.push_back(sw.gates[i]);
+                src.push_back(sw.src[i]);
+                continue;
+            }
+            if (members[(size_t)gr].front() != i) continue;
+            SignRow rows[kSignRows];
+            uint64_t pairs[kSignPairs];
+            memset(rows, 0, sizeof rows);
+            memset(pairs, 0, sizeof pairs);
+            uint32_t np = 0;
+            for (size_t k : members[(size_t)gr]) {
+                const TileGate &t = sw.gates[k];
+                uint32_t local = t.cl | (t.tb == TG_OUTER ? 0u : 1u << t.tb);
+                const uint64_t outer = t.co | (t.tb == TG_OUTER ? 1ull << t.tout : 0ull);
+                if (local == 0) {
+                    pairs[np++] = outer;
+                    continue;
+                }
+                const int a = __builtin_ctz(local);
+                local &= local - 1;
+                if (local) {
+                    const int b = __builtin_ctz(local);
+                    rows[a].up ^= (uint16_t)(1u << b);
+                    rows[a].sym ^= (uint16_t)(1u << b);
+                    rows[b].sym ^= (uint16_t)(1u << a);
+                } else if (outer) {
+                    rows[a].outer ^= outer;
+                } else {
+                    rows[a].lin ^= 1;
+                }
+            }
+            TileGate t;
+            memset(&t, 0, sizeof t);
+            t.cls = TG_SIGN;
+            t.op = OP_SIGN;
+            t.tb = TG_OUTER;
+            t.pad = np ? 1 : 0;
+            uint32_t q = 0;
+            for (uint32_t j = 0; j < (1u << R); j++) {
+                uint32_t par = 0;
+                for (int b = 0; b < R; b++)
+                    if (j >> b & 1) par += (uint32_t)__builtin_popcount(rows[R0 + b].up & (j << R0));
+                q |= (par & 1u) << j;
+            }
+            t.jm = (uint16_t)q;
+            t.creg = (uint32_t)sw.data.size();  // (made relative below)
+            const size_t at = sw.data.size();
+            sw.data.resize(at + 4 + (np ? 4 : 0));
+            memcpy((void *)&sw.data[at], rows, sizeof rows);
+            if (np) memcpy((void *)&sw.data[at + 4], pairs, sizeof pairs);
+            out.push_back(t);
+            src.push_back(kNoSource);
+        }
+        ends.push_back((uint16_t)out.size());
+        g0 = g1;
+    }
+    for (size_t i = 0; i < out.size(); i++)
+        if (out[i].cls == TG_SIGN && out[i].op == OP_SIGN) out[i].creg += (uint32_t)(out.size() - i);
+    if (out.size() + sw.data.size() > (size_t)kMaxSweepGates) {  // (no room behind a full program)
+        sw.data.clear();
+        return;
+    }
+    sw.gates.swap(out);
+    sw.src.swap(src);
+    sw.stage_end.swap(ends);
+}
+
 // ---- diagonal folding -------------------------------------------------------------
 static void diag_sides(const GateDesc &x, double s[4]) {  // |0> and |1> phases (re, im)
     s[0] = 1.0, s[1] = 0.0, s[2] = 1.0, s[3] = 0.0;

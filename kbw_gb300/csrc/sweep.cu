@@ -55,7 +55,9 @@ struct SweepKernel {
     static constexpr size_t kTileBytes = sizeof(Mem) << K;
     static constexpr size_t kChunkTable = 256 * sizeof(uint64_t);
     static constexpr size_t kSmem = kTileBytes + kChunkTable + kMaxSweepGates * sizeof(TileGate) + 16;
-    static constexpr int kCtasPerSm = (R == 3) ? 3 : 2;  // register budget: 80 resp. 128 (c128) / 64 (c64)
+    // register budget: 80 with 8 amplitudes per thread or complex64's 2^12
+    // tiles (24 warps per SM), else 128 (c128) / 64 (c64 on 2^13 tiles)
+    static constexpr int kCtasPerSm = (R == 3 || (sizeof(Mem) == 8 && K == 12)) ? 3 : 2;
     // register layouts A = bits [5, 5+R) and B = [K-R, K) must cover every
     // local bit above the lanes, or a gate on the gap could never run
     static_assert(K <= kLaneBits + 2 * R, "tile geometry leaves local bits no layout holds in registers");
@@ -85,7 +87,7 @@ __global__ void __launch_bounds__(SweepKernel<P, K, R>::kThreads, SweepKernel<P,
     const uint64_t lowmask = chunk - 1;
 
     // --- prologue: program, chunk table, barrier ---
-    for (uint32_t i = threadIdx.x; i < p.gate_count; i += blockDim.x) sg[i] = p.prog[i];
+    for (uint32_t i = threadIdx.x; i < p.gate_count + p.data_count; i += blockDim.x) sg[i] = p.prog[i];
     for (uint32_t c = threadIdx.x; c < nchunks; c += blockDim.x) {
         uint64_t off = 0;
         for (uint32_t j = 0; j < m; j++) off |= (uint64_t)((c >> j) & 1u) << p.hq[j];
@@ -249,12 +251,16 @@ static std::vector<uint64_t> structure_of(const GateDesc *gates, size_t count) {
     return sig;
 }
 
+// Z and CZ gates are merged unless every gate is to run as given.
+static bool merges(const Sim &s) { return !(s.flags & (KBWG_FLAG_EXACT_ORDER | KBWG_FLAG_NO_FOLD)); }
+
 // Pack the planned program with the constants of `gates` and upload it.
 template <class P>
 static cudaError_t upload_program(Sim &s, const std::vector<TileGate> &planned, const std::vector<uint32_t> &src,
                                   const GateDesc *gates, void *dst) {
     std::vector<TileGate> prog = planned;
     for (size_t i = 0; i < prog.size(); i++) {
+        if (src[i] == kNoSource) continue;  // (merged signs and their rows: nothing depends on angles)
         memcpy(prog[i].c, gates[src[i]].c, sizeof prog[i].c);
         P::pack_host(prog[i]);
     }
@@ -327,12 +333,17 @@ static cudaError_t run_fused_p(Sim &s, const GateDesc *gates, size_t count) {
         plan_sweeps(s.n, K, R, gates, count, (s.flags & KBWG_FLAG_EXACT_ORDER) != 0, depth);
     std::vector<TileGate> planned;
     std::vector<uint32_t> src;
-    for (const PlannedSweep &sw : plan) {
+    size_t placed = 0;
+    for (PlannedSweep &sw : plan) {
+        placed += sw.gates.size();
+        if (merges(s)) merge_signs(sw, K, R);
         planned.insert(planned.end(), sw.gates.begin(), sw.gates.end());
+        planned.insert(planned.end(), sw.data.begin(), sw.data.end());
         src.insert(src.end(), sw.src.begin(), sw.src.end());
+        src.insert(src.end(), sw.data.size(), kNoSource);
     }
+    if (placed != count) return cudaErrorInvalidValue;  // the planner could not place every gate
     const size_t total = planned.size();
-    if (total != count) return cudaErrorInvalidValue;  // the planner could not place every gate
     void *dbuf = nullptr;
     cudaError_t e;
     if (graphs) {
@@ -402,6 +413,7 @@ static cudaError_t run_fused_p(Sim &s, const GateDesc *gates, size_t count) {
         memcpy(p.hq, sw.hq, sizeof p.hq);
         p.nstages = (uint32_t)sw.stage_layout.size();
         p.gate_count = (uint32_t)sw.gates.size();
+        p.data_count = (uint32_t)sw.data.size();
         for (uint32_t i = 0; i < p.nstages; i++) {
             p.stage_layout[i] = sw.stage_layout[i];
             p.stage_end[i] = sw.stage_end[i];
@@ -409,7 +421,7 @@ static cudaError_t run_fused_p(Sim &s, const GateDesc *gates, size_t count) {
         p.prog = dprog + off;
         p.err = s.d_err;
         p.tiles = tiles;
-        off += sw.gates.size();
+        off += sw.gates.size() + sw.data.size();
         if (s.prof.on) s.prof.mark(s.stream);
         const void *spec = jk.empty() ? nullptr : jk[(size_t)(&sw - plan.data())];
         if (spec) {
@@ -498,13 +510,17 @@ uint32_t tile_register_bits(const Sim &s, uint32_t k) {
     return k == 11 ? 3u : 4u;  // the 2^11 tiles hold 8 amplitudes per thread, the larger ones 16
 }
 
-// Default tile by register size: below ~152 tiles of the largest geometry the
+// Default tile by register size.  Below ~152 tiles of the largest geometry the
 // chip has idle SMs, and a smaller tile spreads a gate over more of them at
-// the price of a few more sweeps.  Measured (interpreted sweeps, us per flush,
-// one GB300; HEA 4 layers / brickwork 8 layers):
-//   complex64  n = 16: K 13 153/161, 12 125/131, 11 117/120;  n = 19: 180/196,
-//   148/158, 145/150;  n = 20: 184/203, 173/189, 216/225;  n = 21: 261/291,
-//   282/315, 301/319
+// the price of a few more sweeps; on large registers complex64's 2^12 tiles
+// run three CTAs of 256 threads per SM where the 2^13 ones run two of 512 on
+// 64 registers.  At 21 qubits those 512 tiles are one wave and a bit of 456
+// CTAs, and 2^13 wins.  Measured (us per flush, one GB300; HEA / brickwork):
+//   complex64 interpreted  n = 16: K 13 120/138, 12 97/113, 11 87/96;  n = 19:
+//   143/167, 112/133, 111/120;  n = 20: 148/174, 141/166, 181/197;  n = 21:
+//   219/261, 242/293;  n = 24: 1477/1763, 1374/1734
+//   complex64 specialised  n = 22: 190/216, 177/169;  n = 28: 10456/11759,
+//   9953/10710
 //   binary64   n = 14: K 12 485/327, 11 278/201;  n = 19: 623/429, 620/401;
 //   specialised (from 20 qubits) K 12 is 3-5 % faster (n = 25: 46.5 against
 //   48.4 ms, HEA 6 layers)
@@ -513,7 +529,7 @@ uint32_t default_tile_k(const Sim &s) {
     const std::vector<uint32_t> ks = compiled_tiles(s);
     if (ks.size() > 1 && ks[0] <= s.n) {
         if (!s.prec && s.n <= 19) return 11;
-        if (!s.prec && s.n == 20) return 12;
+        if (!s.prec && s.n != 21 && s.n <= 32) return 12;
         if (s.prec && !ff_capable(s) && s.n <= 19) return 11;
     }
     if (ks[0] <= s.n) return ks[0];
@@ -784,8 +800,10 @@ template <class P, int K, int R>
 static size_t check_p(const Sim &s, const GateDesc *gates, size_t count, size_t &sweeps) {
     using SK = SweepKernel<P, K, R>;
     const size_t depth = s.fusion_depth ? s.fusion_depth : (size_t)kMaxSweepGates;
-    const std::vector<PlannedSweep> plan =
+    std::vector<PlannedSweep> plan =
         plan_sweeps(s.n, K, R, gates, count, (s.flags & KBWG_FLAG_EXACT_ORDER) != 0, depth);
+    if (merges(s))
+        for (PlannedSweep &sw : plan) merge_signs(sw, K, R);
     const JitGeometry geo{PolicyName<P>::s, K, R, SK::kThreads, SK::kCtasPerSm, s.n > 32};
     std::vector<std::string> srcs;
     for (const PlannedSweep &sw : plan) srcs.push_back(jit_sweep_source(geo, sw));

@@ -43,7 +43,8 @@ enum {
     TG_P = 6,      // |1> * (c0 + i c1)
     TG_RZ = 7,     // |0> * (c0 + i c1), |1> * (c2 + i c3)
     TG_PI = 8,     // |1> * i^q, q = c0
-    TG_SCALE = 9   // every amplitude * (c0 + i c1), the deferred factors (sub 1: * c0, real)
+    TG_SCALE = 9,  // every amplitude * (c0 + i c1), the deferred factors (sub 1: * c0, real)
+    TG_SIGN = 10   // many Z and CZ gates at once (SignRow)
 };
 __host__ __device__ inline bool tg_diagonal(uint32_t cls) { return cls >= TG_Z; }
 constexpr uint8_t TG_OUTER = 0xFF;  // tb value: diagonal gate whose target lies outside the tile
@@ -54,6 +55,7 @@ enum {
     OP_REG = 8,    // + class * 4 + register bit: target on a register bit, in-thread pairs
     OP_DREG = 32,  // + (class - TG_Z) * 4 + register bit: diagonal, target on a register bit
     OP_DFIX = 48,  // + (class - TG_Z): diagonal, side fixed per thread (lane/warp bit) or per tile
+    OP_SIGN = 60,  // TG_SIGN
     OP_ROT = 64    // + form * 4 + register bit: RX/RY with a deferred factor (form: 0 RX by tangent, 1 RX by
                    // cotangent, 2 and 3 RY), set when the constants are packed
 };
@@ -97,6 +99,20 @@ __host__ __device__ inline void tile_gate_dispatch(TileGate &g, int R0, int R) {
     else g.op = OP_DFIX + (g.cls - TG_Z);
 }
 
+// Z and CZ gates of one stage that nothing keeps apart, as one gate: their
+// product is (-1)^q(u) with a quadratic form q over the qubits.  Row i (local
+// bit i): the later local bits it pairs with (up), all of them (sym), the
+// qubits outside the tile it pairs with, and whether it has a Z of its own.
+// Pairs and single qubits outside the tile follow as masks (`pad` of the gate
+// set).  The rows stand behind the sweep's gates, `creg` entries after the
+// gate's own; jm bit j: q on register j's bits alone.
+struct alignas(16) SignRow {
+    uint64_t outer;
+    uint16_t up, sym;
+    uint16_t lin, pad;
+};
+constexpr int kSignRows = 16, kSignPairs = 32;  // 4 program entries each
+
 // A rotation with a deferred factor keeps one of its two coefficients: with
 // c = cos, s = sin of half the angle, |c| >= |s| leaves t = s / c and the
 // factor c ("tangent": a0 - t a1, a1 + t a0 for RY), else u = c / s and the
@@ -123,6 +139,7 @@ struct SweepParams {
     uint8_t hq[16];     // high qubit positions, ascending
     uint32_t nstages;
     uint32_t gate_count;
+    uint32_t data_count;  // program entries behind the gates (SignRow)
     uint8_t stage_layout[kMaxStages];
     uint16_t stage_end[kMaxStages];  // exclusive gate index at which each stage ends
     const TileGate *prog;           // gate_count gates of this sweep
@@ -138,8 +155,10 @@ struct PlannedSweep {
     std::vector<TileGate> gates;
     std::vector<uint8_t> stage_layout;
     std::vector<uint16_t> stage_end;
-    std::vector<uint32_t> src;  // index in the input list of each gate, in execution order
+    std::vector<uint32_t> src;  // index in the input list of each gate, in execution order (kNoSource: a merged one)
+    std::vector<TileGate> data;  // entries behind the gates in the sweep's program
 };
+constexpr uint32_t kNoSource = 0xFFFFFFFFu;
 
 // Greedy commutation-aware planner: groups the gate list into sweeps over
 // tiles of K qubits (targets of non-diagonal gates must lie in the tile;
@@ -149,6 +168,12 @@ struct PlannedSweep {
 // max_gates: fusion depth, the most gates one sweep may apply.
 std::vector<PlannedSweep> plan_sweeps(uint32_t n, int K, int R, const GateDesc *g, size_t count,
                                       bool keep_order = false, size_t max_gates = kMaxSweepGates);
+
+// Replace runs of Z and CZ gates (kSignMin or more that no gate in between
+// keeps apart) by one TG_SIGN gate each.  Signs are exact, so every
+// amplitude keeps its value bit for bit.
+constexpr size_t kSignMin = 3;
+void merge_signs(PlannedSweep &sw, int K, int R);
 
 bool is_diagonal(uint32_t kind);
 

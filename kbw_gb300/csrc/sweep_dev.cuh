@@ -162,6 +162,12 @@ struct Exact {
         return Amp{a.im, -a.re};
     }
     static __device__ __forceinline__ Amp smul(Amp a, T c) { return Amp{xmul(a.re, c), xmul(a.im, c)}; }
+    // negated where s (a sign bit) is set
+    static __device__ __forceinline__ T flip1(T x, uint32_t s) {
+        if constexpr (sizeof(T) == 4) return __uint_as_float(__float_as_uint(x) ^ s);
+        else return __hiloint2double(__double2hiint(x) ^ (int)s, __double2loint(x));
+    }
+    static __device__ __forceinline__ Amp flip(Amp a, uint32_t s) { return Amp{flip1(a.re, s), flip1(a.im, s)}; }
 };
 
 // Fast: the same gates with fused multiply-adds (RX/RY 8 FP operations per
@@ -341,6 +347,9 @@ struct FastP {
     }
     static __device__ __forceinline__ int power_of_i(const K4 &k) { return (int)k.c0; }
     static __device__ __forceinline__ Amp smul(Amp a, float c) { return mul_rn(a, c); }
+    static __device__ __forceinline__ Amp flip(Amp a, uint32_t s) {
+        return make_float2(__uint_as_float(__float_as_uint(a.x) ^ s), __uint_as_float(__float_as_uint(a.y) ^ s));
+    }
     // RX/RY with a deferred factor (pack_rot): one packed FMA per amplitude
     static constexpr bool kDefer = true;
     static __device__ __forceinline__ bool cot(const K4 &k) { return k.c1 != 0.f; }
@@ -479,6 +488,7 @@ struct FFPol {
     static constexpr bool kDefer = false;
     static __device__ __forceinline__ int power_of_i(const K4 &k) { return (int)k.c0.h; }
     static __device__ __forceinline__ Amp smul(Amp a, ff::f2 c) { return Amp{ff::mul(a.re, c), ff::mul(a.im, c)}; }
+    static __device__ __forceinline__ Amp flip(Amp a, uint32_t s) { return s ? neg(a) : a; }
     static __device__ __forceinline__ Amp pi_mul(Amp a, int q) {
         if (q == 1) return Amp{ff::neg(a.im), a.re};
         if (q == 2) return Amp{ff::neg(a.re), ff::neg(a.im)};
@@ -567,6 +577,12 @@ struct FF2 {
     }
     static __device__ __forceinline__ int power_of_i(const K4 &k) { return (int)k.c0.h; }
     static __device__ __forceinline__ Amp smul(Amp a, ff::f2 c) { return ff2::mul(a, ff2::konst(c)); }
+    static __device__ __forceinline__ Amp flip(Amp a, uint32_t s) {
+        auto f = [s](float2 x) {
+            return make_float2(__uint_as_float(__float_as_uint(x.x) ^ s), __uint_as_float(__float_as_uint(x.y) ^ s));
+        };
+        return Amp{f(a.h), f(a.l)};
+    }
     // RX/RY with a deferred factor (pack_rot): 15 packed operations per
     // amplitude (ff2::axpy) where the full form's dot product takes 19
     static constexpr bool kDefer = true;
@@ -763,6 +779,48 @@ __device__ __forceinline__ void diag_fixed(typename P::Amp (&v)[1 << R], const T
     }
 }
 
+// Signs of this thread's registers under a TG_SIGN gate (bit j: register j is
+// negated).  q(u) splits into the fixed bits F and the register bits j:
+// q(F) + q(j) + the pairs between them, which are linear in j.  The rows' share
+// of the qubits outside the tile is uniform over the warp (lane i takes row i).
+// About 100 instructions for any number of Z and CZ gates; one by one each
+// costs about 60 (16 amplitudes per thread, interpreted).  A ring of CZ gates
+// is one such gate: HEA layers in KBWG_SIGN_FIGURES
+template <class P, int K, int R>
+__device__ __forceinline__ uint32_t sign_mask(const TileGate &g, int R0, uint32_t F, uint64_t base) {
+    const SignRow *rows = reinterpret_cast<const SignRow *>(&g + g.creg);
+    const uint32_t lane = threadIdx.x & 31u;
+    bool lin = false;
+    if (lane < (uint32_t)K) lin = ((__popcll(base & rows[lane].outer) + rows[lane].lin) & 1) != 0;
+    const uint32_t L = __ballot_sync(0xffffffffu, lin);
+    uint32_t q = 0;
+    if (g.pad) {
+        const uint64_t m = reinterpret_cast<const uint64_t *>(rows + kSignRows)[lane];
+        q = (uint32_t)__popc(__ballot_sync(0xffffffffu, m != 0 && (base & m) == m));
+    }
+    uint32_t up = 0, sym = 0;
+#pragma unroll
+    for (int i = 0; i < K; i++) {  // (F has no register bits)
+        const uint32_t on = 0u - ((F >> i) & 1u);
+        up ^= on & rows[i].up;
+        sym ^= on & rows[i].sym;
+    }
+    q += (uint32_t)__popc(F & (up ^ L));
+    const uint32_t m = (sym ^ L) >> R0;
+    uint32_t S = g.jm;
+    S ^= 0u - (q & 1u);
+    S ^= (0u - (m & 1u)) & 0xAAAAu;
+    S ^= (0u - ((m >> 1) & 1u)) & 0xCCCCu;
+    S ^= (0u - ((m >> 2) & 1u)) & 0xF0F0u;
+    if constexpr (R > 3) S ^= (0u - ((m >> 3) & 1u)) & 0xFF00u;
+    return S;
+}
+template <class P, int R>
+__device__ __forceinline__ void flip_registers(typename P::Amp (&v)[1 << R], uint32_t S) {
+#pragma unroll
+    for (int j = 0; j < (1 << R); j++) v[j] = P::flip(v[j], (S << (31 - j)) & 0x80000000u);
+}
+
 // RX/RY with a deferred factor on register bit B (uncontrolled: every pair).
 template <class P, int R, int B, bool RYG, bool COT>
 __device__ __forceinline__ void rot_pairs(typename P::Amp (&v)[1 << R], const TileGate &g) {
@@ -806,7 +864,7 @@ template <class A, class C> struct pick_t<false, A, C> { using type = C; };
 // the program may hold rotations with deferred factors (their bodies cost
 // the adjoint's kernels, which never run them, registers).
 template <class P, int K, int R, class B = uint32_t, bool ROT = P::kDefer>
-__device__ __forceinline__ void tile_gate(const TileGate &g, typename P::Amp (&v)[1 << R], int /*R0*/, uint32_t F,
+__device__ __forceinline__ void tile_gate(const TileGate &g, typename P::Amp (&v)[1 << R], int R0, uint32_t F,
                                           typename ident<B>::type base) {
     static_assert(R >= 3 && R <= 4, "dispatch covers register bits 0..3");
     const uint32_t op = g.op;
@@ -833,6 +891,12 @@ __device__ __forceinline__ void tile_gate(const TileGate &g, typename P::Amp (&v
         } else if (op == OP_LANE + TG_RX) lane_gate<P, R, TG_RX>(v, g, fok, F);
         else lane_gate<P, R, TG_RY>(v, g, fok, F);
         return;
+    }
+    if constexpr (ROT) {
+        if (op == OP_SIGN) {  // (uniform: every lane joins the votes)
+            flip_registers<P, R>(v, sign_mask<P, K, R>(g, R0, F, (uint64_t)base));
+            return;
+        }
     }
     if (!fok) return;
     switch (op) {
