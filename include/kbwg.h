@@ -380,10 +380,10 @@ int32_t kbwg_wait_probe(kbwg_sim *sim, uint32_t spins);
  * kbwg_new creates (kbwg_new fails with KBWG_EINVAL on a value no kernel
  * exists for); a tile size larger than a handle's qubit count falls back to
  * the default on that handle.  The default tile is the arithmetic's
- * (complex64 12, complex128 12, float-float 11 qubits; 13 for complex64 at 21
- * and above 32 qubits); on registers of 13 to 19 qubits, which leave SMs
- * without such a tile, 11; for a register smaller than that the largest
- * compiled size that fits it.  They apply wherever gates are applied to a
+ * (complex64 13, complex128 12, float-float 11 qubits); on registers of 13 to
+ * 19 qubits, which leave SMs without such a tile, 11; 12 for complex64 at 20,
+ * 22, 24 and 25 qubits; for a register smaller than that the largest compiled
+ * size that fits it.  They apply wherever gates are applied to a
  * handle's state (gate calls, the forward pass of kbwg_adjoint_gradient, the
  * circuit runs of kbwg_param_shift_gradient), not to the adjoint's reverse
  * sweeps or to the batch and reduction kernels. */

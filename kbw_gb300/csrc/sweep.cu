@@ -512,15 +512,17 @@ uint32_t tile_register_bits(const Sim &s, uint32_t k) {
 
 // Default tile by register size.  Below ~152 tiles of the largest geometry the
 // chip has idle SMs, and a smaller tile spreads a gate over more of them at
-// the price of a few more sweeps; on large registers complex64's 2^12 tiles
-// run three CTAs of 256 threads per SM where the 2^13 ones run two of 512 on
-// 64 registers.  At 21 qubits those 512 tiles are one wave and a bit of 456
-// CTAs, and 2^13 wins.  Measured (us per flush, one GB300; HEA / brickwork):
-//   complex64 interpreted  n = 16: K 13 120/138, 12 97/113, 11 87/96;  n = 19:
-//   143/167, 112/133, 111/120;  n = 20: 148/174, 141/166, 181/197;  n = 21:
-//   219/261, 242/293;  n = 24: 1477/1763, 1374/1734
-//   complex64 specialised  n = 22: 190/216, 177/169;  n = 28: 10456/11759,
-//   9953/10710
+// the price of a few more sweeps; complex64's 2^12 tiles run three CTAs of 256
+// threads per SM on 80 registers, the 2^13 ones two of 512 on 64, and stay
+// ahead where they need hardly more sweeps.  At 21 and 23 qubits their last
+// wave of CTAs is nearly empty, or a random circuit takes a sweep more, and
+// from 26 on every sweep more costs a pass over HBM.  Measured (us per flush,
+// one GB300; HEA / brickwork, interpreted unless stated):
+//   complex64  n = 16: K 13 108/121, 12 88/100, 11 87/94;  n = 19: 128/145,
+//   105/118, 110/119;  n = 20: 131/152, 124/146, 173/188;  n = 21: 175/219,
+//   205/251;  n = 22: 318/412, 300/361 (specialised 191/220, 177/172);  n =
+//   24: 1136/1452, 1095/1455 (662/738, 612/683);  n = 26: 4357/5690, 4541/5895
+//   (2388/2725, 2446/2666)
 //   binary64   n = 14: K 12 485/327, 11 278/201;  n = 19: 623/429, 620/401;
 //   specialised (from 20 qubits) K 12 is 3-5 % faster (n = 25: 46.5 against
 //   48.4 ms, HEA 6 layers)
@@ -529,7 +531,7 @@ uint32_t default_tile_k(const Sim &s) {
     const std::vector<uint32_t> ks = compiled_tiles(s);
     if (ks.size() > 1 && ks[0] <= s.n) {
         if (!s.prec && s.n <= 19) return 11;
-        if (!s.prec && s.n != 21 && s.n <= 32) return 12;
+        if (!s.prec && (s.n == 20 || s.n == 22 || s.n == 24 || s.n == 25)) return 12;
         if (s.prec && !ff_capable(s) && s.n <= 19) return 11;
     }
     if (ks[0] <= s.n) return ks[0];
@@ -612,7 +614,7 @@ static cudaError_t run_fused_t(Sim &s, const GateDesc *gates, size_t count) {
 // Each H, RX or RY grows the state by at most sqrt(2), so kDeferRun of them
 // stay inside float's range before g is applied (a structural count: the
 // plan must not depend on the angles).  P(+-pi/2) and P(pi) become exact
-// multiplications by i^q.
+// multiplications by i^q (not in complex64).
 // A SCALE costs about two deferred rotations' savings, so lists with fewer
 // than kDeferMin such gates keep the full forms (float-float always drops H's
 // and RZ's factors: its multiplications cost most).
@@ -678,7 +680,7 @@ static std::vector<GateDesc> defer_scale(int arith, const GateDesc *gates, size_
             x.c[1] = r.cot ? 1.0 : 0.0;
             grew = true;
         }
-        if (x.kind == G_P) {
+        if (x.kind == G_P && arith != ARITH_C64) {
             const double c = x.c[0], sn = x.c[1], t = 1e-15;
             int q = 0;
             if (fabs(c) < t && fabs(sn - 1.0) < t) q = 1;

@@ -340,12 +340,10 @@ struct FastP {
     static __device__ __forceinline__ Amp cmul(Amp a, float c, float s) {
         return __ffma2_rn(a, bc(c), __fmul2_rn(swp(a), make_float2(-s, s)));
     }
-    static __device__ __forceinline__ Amp pi_mul(Amp a, int q) {
-        if (q == 1) return make_float2(-a.y, a.x);
-        if (q == 2) return make_float2(-a.x, -a.y);
-        return make_float2(a.y, -a.x);
-    }
-    static __device__ __forceinline__ int power_of_i(const K4 &k) { return (int)k.c0; }
+    // |1> * i^q stays a phase gate in complex64: bodies that pick q at run time
+    // made the interpreted 2^13 kernel spill (16 -> 112 bytes, up to 25 % slower)
+    static __device__ __forceinline__ Amp pi_mul(Amp a, int) { return a; }
+    static __device__ __forceinline__ int power_of_i(const K4 &) { return 0; }
     static __device__ __forceinline__ Amp smul(Amp a, float c) { return mul_rn(a, c); }
     static __device__ __forceinline__ Amp flip(Amp a, uint32_t s) {
         return make_float2(__uint_as_float(__float_as_uint(a.x) ^ s), __uint_as_float(__float_as_uint(a.y) ^ s));
@@ -892,12 +890,6 @@ __device__ __forceinline__ void tile_gate(const TileGate &g, typename P::Amp (&v
         else lane_gate<P, R, TG_RY>(v, g, fok, F);
         return;
     }
-    if constexpr (ROT) {
-        if (op == OP_SIGN) {  // (uniform: every lane joins the votes)
-            flip_registers<P, R>(v, sign_mask<P, K, R>(g, R0, F, (uint64_t)base));
-            return;
-        }
-    }
     if (!fok) return;
     switch (op) {
 #define KBWG_REG(C)                                                    \
@@ -930,6 +922,9 @@ __device__ __forceinline__ void tile_gate(const TileGate &g, typename P::Amp (&v
 #undef KBWG_ROT
 #undef KBWG_DREG
 #undef KBWG_DFIX
+    case OP_SIGN:  // (no controls: every lane of the warp is here and joins the votes)
+        if constexpr (ROT) flip_registers<P, R>(v, sign_mask<P, K, R>(g, R0, F, (uint64_t)base));
+        break;
     default: break;
     }
 }
