@@ -28,7 +28,9 @@
 
 #include <algorithm>
 #include <atomic>
+#include <condition_variable>
 #include <exception>
+#include <functional>
 #include <memory>
 #include <mutex>
 #include <thread>
@@ -508,33 +510,90 @@ struct BatchCircuitIn {
     const char *error = nullptr;
 };
 
-// fn(i) for i in [0, n) on all host cores (items taken one at a time).  An
-// exception in any item (an allocation failing) stops the remaining items and
-// is rethrown here, on the calling thread, after every worker has joined.
-template <class F>
-static void batch_parallel_for(size_t n, F &&fn) {
-    const size_t nt = std::min<size_t>(n, std::max(1u, std::thread::hardware_concurrency()));
-    std::atomic<size_t> next{0};
-    std::mutex mu;
-    std::exception_ptr first;
-    auto worker = [&]() {
+// Host threads of one call: its steps run fn(i) for i in [0, n), items taken
+// one at a time, on the calling thread and the workers.  Started once per call
+// and only for enough gates (starting one takes ~60 us here, planning 4,000
+// gates about as long; a set of 16 for every step cost 1 ms each time).  An
+// exception in any item (an allocation failing) stops the step's remaining
+// items and is rethrown by run(), on the calling thread, when no worker is in
+// it any more.
+class BatchWorkers {
+public:
+    explicit BatchWorkers(size_t gates) {
+        const size_t hw = std::max(1u, std::thread::hardware_concurrency());
+        const size_t nt = std::min(hw, 1 + gates / 4000);
         try {
-            for (size_t i; (i = next.fetch_add(1, std::memory_order_relaxed)) < n;) fn(i);
-        } catch (...) {
-            std::lock_guard<std::mutex> lk(mu);
-            if (!first) first = std::current_exception();
-            next.store(n);
+            for (size_t t = 1; t < nt; t++) threads_.emplace_back([this] { loop(); });
+        } catch (...) {  // fewer threads than asked: the ones started and the caller share the items
         }
-    };
-    std::vector<std::thread> pool;
-    try {
-        for (size_t t = 1; t < nt; t++) pool.emplace_back(worker);
-    } catch (...) {  // fewer threads than asked: the ones started and this one share the items
     }
-    worker();
-    for (std::thread &t : pool) t.join();
-    if (first) std::rethrow_exception(first);
-}
+    ~BatchWorkers() {
+        {
+            std::lock_guard<std::mutex> lk(mu_);
+            stop_ = true;
+        }
+        start_.notify_all();
+        for (std::thread &t : threads_) t.join();
+    }
+    void run(size_t n, const std::function<void(size_t)> &fn) {
+        if (threads_.empty() || n < 2) {
+            for (size_t i = 0; i < n; i++) fn(i);
+            return;
+        }
+        {
+            std::lock_guard<std::mutex> lk(mu_);
+            fn_ = &fn;
+            n_ = n;
+            next_.store(0);
+            busy_ = threads_.size();
+            step_++;
+        }
+        start_.notify_all();
+        items();
+        std::unique_lock<std::mutex> lk(mu_);
+        done_.wait(lk, [&] { return busy_ == 0; });
+        fn_ = nullptr;
+        if (first_) {
+            const std::exception_ptr e = first_;
+            first_ = nullptr;
+            std::rethrow_exception(e);
+        }
+    }
+
+private:
+    void items() {
+        try {
+            for (size_t i; (i = next_.fetch_add(1, std::memory_order_relaxed)) < n_;) (*fn_)(i);
+        } catch (...) {
+            std::lock_guard<std::mutex> lk(mu_);
+            if (!first_) first_ = std::current_exception();
+            next_.store(n_);
+        }
+    }
+    void loop() {
+        uint64_t seen = 0;
+        for (;;) {
+            {
+                std::unique_lock<std::mutex> lk(mu_);
+                start_.wait(lk, [&] { return stop_ || step_ != seen; });
+                if (stop_) return;
+                seen = step_;
+            }
+            items();
+            std::lock_guard<std::mutex> lk(mu_);
+            if (--busy_ == 0) done_.notify_one();
+        }
+    }
+    std::vector<std::thread> threads_;
+    std::mutex mu_;
+    std::condition_variable start_, done_;
+    const std::function<void(size_t)> *fn_ = nullptr;
+    size_t n_ = 0, busy_ = 0;
+    std::atomic<size_t> next_{0};
+    uint64_t step_ = 0;
+    std::exception_ptr first_;
+    bool stop_ = false;
+};
 
 // Device buffer of a call, kept for the next one (the largest up to
 // kBatchKeepBytes, one per process): allocating and freeing a gigabyte costs
@@ -601,7 +660,7 @@ void batch_release_workspace() {
 }
 
 template <class P, int K, int R>
-static int32_t batch_run(int arith, std::vector<BatchCircuitIn> &circs, double *energies) {
+static int32_t batch_run(int arith, BatchWorkers &workers, std::vector<BatchCircuitIn> &circs, double *energies) {
     using BK = BatchKernel<P, K, R>;
     using Mem = typename P::Mem;
     auto fail = [](cudaError_t e, const char *what) {
@@ -613,7 +672,7 @@ static int32_t batch_run(int arith, std::vector<BatchCircuitIn> &circs, double *
     // plan every circuit (in parallel: the circuits are independent), those of
     // one structure (register size, kinds, targets, controls) once
     std::vector<std::vector<uint64_t>> sigs(circs.size());
-    batch_parallel_for(circs.size(), [&](size_t c) {
+    workers.run(circs.size(), [&](size_t c) {
         BatchCircuitIn &ci = circs[c];
         ci.gates = defer_factors(arith, ci.gates.data(), ci.gates.size());
         std::vector<uint64_t> &sig = sigs[c];
@@ -646,7 +705,7 @@ static int32_t batch_run(int arith, std::vector<BatchCircuitIn> &circs, double *
     }
     std::vector<std::vector<PlannedSweep>> plans(first.size());
     std::vector<char> plan_ok(first.size());
-    batch_parallel_for(first.size(), [&](size_t k) {
+    workers.run(first.size(), [&](size_t k) {
         const BatchCircuitIn &ci = circs[first[k]];
         const uint32_t nplan = std::max<uint32_t>(ci.n, (uint32_t)K);  // small registers padded with |0> qubits
         plans[k] = plan_sweeps(nplan, K, R, ci.gates.data(), ci.gates.size(), false, kMaxSweepGates);
@@ -657,7 +716,7 @@ static int32_t batch_run(int arith, std::vector<BatchCircuitIn> &circs, double *
         }
         plan_ok[k] = placed == ci.gates.size() ? 1 : 0;
     });
-    batch_parallel_for(circs.size(), [&](size_t c) {
+    workers.run(circs.size(), [&](size_t c) {
         BatchCircuitIn &ci = circs[c];
         const std::vector<PlannedSweep> &plan = plans[plan_of[c]];
         for (const PlannedSweep &sw : plan) {
@@ -778,7 +837,7 @@ static int32_t batch_run(int arith, std::vector<BatchCircuitIn> &circs, double *
     std::unique_ptr<BatchTerm[]> terms(new BatchTerm[std::max<size_t>(nterms, 1)]);
     std::unique_ptr<BatchPass[]> passes(new BatchPass[std::max<size_t>(npass, 1)]);
     std::unique_ptr<BatchTileTerm[]> tterms(new BatchTileTerm[std::max<size_t>(ntt, 1)]);
-    batch_parallel_for(circs.size(), [&](size_t c) {
+    workers.run(circs.size(), [&](size_t c) {
         BatchCircuitIn &ci = circs[c];
         BatchJob &j = jobs[c];
         const uint32_t base = j.pad;
@@ -981,7 +1040,8 @@ int32_t batch_circuits(int precision, uint32_t flags, size_t ncirc, const uint32
                        const uintptr_t *term_offsets, const double *coefficients, const uintptr_t *ham_offsets,
                        double *energies) {
     std::vector<BatchCircuitIn> circs(ncirc);
-    batch_parallel_for(ncirc, [&](size_t c) {
+    BatchWorkers workers((size_t)(gate_offsets[ncirc] > gate_offsets[0] ? gate_offsets[ncirc] - gate_offsets[0] : 0));
+    workers.run(ncirc, [&](size_t c) {
         BatchCircuitIn &ci = circs[c];
         auto bad = [&](int32_t code, const char *msg) {
             ci.status = code;
@@ -1028,9 +1088,9 @@ int32_t batch_circuits(int precision, uint32_t flags, size_t ncirc, const uint32
             return ci.status;
         }
     if (ncirc == 0) return KBWG_OK;
-    if (precision == KBWG_C64) return batch_run<FastP, 12, 4>(ARITH_C64, circs, energies);
-    if (flags & KBWG_FLAG_FAST_C128) return batch_run<FF2B, 11, 3>(ARITH_FF, circs, energies);
-    return batch_run<Fast<double>, 11, 3>(ARITH_F64, circs, energies);
+    if (precision == KBWG_C64) return batch_run<FastP, 12, 4>(ARITH_C64, workers, circs, energies);
+    if (flags & KBWG_FLAG_FAST_C128) return batch_run<FF2B, 11, 3>(ARITH_FF, workers, circs, energies);
+    return batch_run<Fast<double>, 11, 3>(ARITH_F64, workers, circs, energies);
 }
 
 }  // namespace kbwg
