@@ -288,8 +288,12 @@ __global__ void __launch_bounds__(256) k_apply_group_ff(const ff2::v2 *__restric
 // The same runs for complex64 states (float arithmetic; the coefficients are
 // the high parts rh/ih): each thread keeps its 2^K/256 amplitudes u = tid +
 // 256 i in registers, the strings run in the outer loop (their fields read
-// once per tile), signs are counted per amplitude and partners summed per run.
-__global__ void __launch_bounds__(256) k_apply_tile_f32(const cx<float> *__restrict__ phi, cx<float> *__restrict__ lam,
+// once per tile) and partners are summed per run.  A sign splits into the
+// thread's bits (one parity per string) and the three bits of i: Z-type
+// strings are counted by their mask on those and the eight counts come from
+// one Walsh transform per run.  24 qubits, ring
+// TFIM, four passes: 1.10 -> 0.82 ms.
+__global__ void __launch_bounds__(256, 3) k_apply_tile_f32(const cx<float> *__restrict__ phi, cx<float> *__restrict__ lam,
                                                         uint32_t n, const __grid_constant__ ApplyTilePassFF p) {
     constexpr int K = kApplyTileBits, NA = (1 << K) / 256;
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -318,39 +322,72 @@ __global__ void __launch_bounds__(256) k_apply_tile_f32(const cx<float> *__restr
             tile[u] = self[i];
         }
         __syncthreads();
+        static_assert(NA == 8, "eight amplitudes per thread: their local bits above the thread's are three");
         float ar[NA], ai[NA], rr[NA], ri[NA];
-        int cnt[NA];
 #pragma unroll
-        for (int i = 0; i < NA; i++) ar[i] = ai[i] = rr[i] = ri[i] = 0.f, cnt[i] = 0;
+        for (int i = 0; i < NA; i++) ar[i] = ai[i] = rr[i] = ri[i] = 0.f;
+        long long count = 0;  // eight signed bytes: signed strings of the run by their mask on the three bits
         for (uint32_t k = 0; k < p.nterms; k++) {  // (branches depend on the string only: uniform)
             const ApplyTileTermFF t = p.t[k];
-            const uint32_t op = (uint32_t)__popcll(base & t.zo) & 1u;
+            const uint32_t xh = t.xl >> 8, zr = t.zl >> 8, lo = threadIdx.x ^ (t.xl & 255u);
+            const uint32_t par = ((uint32_t)__popc(lo & t.zl & 255u) + (uint32_t)__popcll(base & t.zo)) & 1u;
+            if (t.cat == 0u) {
+                count += (par ? -1ll : 1ll) << (8u * zr);
+                if (t.last) {
+                    // the bytes' Walsh transform: the signed count of every amplitude
+                    int w[NA];
 #pragma unroll
-            for (int i = 0; i < NA; i++) {
-                const uint32_t u = threadIdx.x + 256u * (uint32_t)i, src = u ^ t.xl;
-                const bool neg = (((uint32_t)__popc(src & t.zl) + op) & 1u) != 0u;
-                if (t.cat == 0u) {
-                    cnt[i] += neg ? -1 : 1;
-                    if (t.last) {
-                        const float w = (float)cnt[i] * t.rh;
-                        ar[i] += w * self[i].re;
-                        ai[i] += w * self[i].im;
-                        cnt[i] = 0;
+                    for (int i = 0; i < NA; i++) {
+                        w[i] = (int)(signed char)(count & 0xFF);
+                        count = (count - w[i]) >> 8;
                     }
-                } else if (t.cat == 1u) {
-                    const cx<float> a = tile[src];
-                    rr[i] += neg ? -a.re : a.re;
-                    ri[i] += neg ? -a.im : a.im;
-                    if (t.last) {
+                    count = 0;
+#pragma unroll
+                    for (int h = 1; h < NA; h <<= 1)
+#pragma unroll
+                        for (int i = 0; i < NA; i++)
+                            if (!(i & h)) {
+                                const int x = w[i], y = w[i | h];
+                                w[i] = x + y;
+                                w[i | h] = x - y;
+                            }
+#pragma unroll
+                    for (int i = 0; i < NA; i++) {
+                        const float f = (float)w[i] * t.rh;
+                        ar[i] += f * self[i].re;
+                        ai[i] += f * self[i].im;
+                    }
+                }
+                continue;
+            }
+            // bit i: the sign of amplitude i's partner (i ^ xh)
+            uint32_t neg = ((zr & 1u) ? 0xAAu : 0u) ^ ((zr & 2u) ? 0xCCu : 0u) ^ ((zr & 4u) ? 0xF0u : 0u);
+            if (((uint32_t)__popc(xh & zr) + par) & 1u) neg = ~neg;
+            const cx<float> *row = tile + lo;
+            if (t.cat == 1u) {
+#pragma unroll
+                for (int i = 0; i < NA; i++) {
+                    const cx<float> a = row[256u * ((uint32_t)i ^ xh)];
+                    const uint32_t sg = (neg << (31 - i)) & 0x80000000u;
+                    rr[i] += __uint_as_float(__float_as_uint(a.re) ^ sg);
+                    ri[i] += __uint_as_float(__float_as_uint(a.im) ^ sg);
+                }
+                if (t.last) {
+#pragma unroll
+                    for (int i = 0; i < NA; i++) {
                         ar[i] += t.rh * rr[i];
                         ai[i] += t.rh * ri[i];
                         rr[i] = ri[i] = 0.f;
                     }
-                } else {
-                    const cx<float> a = tile[src];
+                }
+            } else {
+#pragma unroll
+                for (int i = 0; i < NA; i++) {
+                    const cx<float> a = row[256u * ((uint32_t)i ^ xh)];
                     const float pr = t.rh * a.re - t.ih * a.im, pi = t.rh * a.im + t.ih * a.re;
-                    ar[i] += neg ? -pr : pr;
-                    ai[i] += neg ? -pi : pi;
+                    const bool m = ((neg >> i) & 1u) != 0u;
+                    ar[i] += m ? -pr : pr;
+                    ai[i] += m ? -pi : pi;
                 }
             }
         }

@@ -783,7 +783,7 @@ __device__ __forceinline__ void diag_fixed(typename P::Amp (&v)[1 << R], const T
 // of the qubits outside the tile is uniform over the warp (lane i takes row i).
 // About 100 instructions for any number of Z and CZ gates; one by one each
 // costs about 60 (16 amplitudes per thread, interpreted).  A ring of CZ gates
-// is one such gate: HEA layers in KBWG_SIGN_FIGURES
+// is a few such gates: 24 qubits, 10 layers, complex64 gradient 8.99 -> 8.61 ms.
 template <class P, int K, int R>
 __device__ __forceinline__ uint32_t sign_mask(const TileGate &g, int R0, uint32_t F, uint64_t base) {
     const SignRow *rows = reinterpret_cast<const SignRow *>(&g + g.creg);
