@@ -597,7 +597,8 @@ __global__ void __launch_bounds__(AdjKernel<P, K, R>::kThreads, 2)
                 const uint32_t info = sinfo[gi];
                 const int gt = (int)(info & 15u);
                 if (gt != GT_NONE) {
-                    const typename G::Acc w = G::warp_sum(grad_partial<P, K, R>(g, gt, vp, vl, R0, F, base));
+                    const typename G::Value w =
+                        G::warp_sum(G::finish(gt, grad_partial<P, K, R>(g, gt, vp, vl, R0, F, base)));
                     if (lane == 0) {
                         Wacc &slot = acc[warp * kMaxSweepGates + (info >> 4)];
                         slot = G::wadd(slot, w);

@@ -469,7 +469,7 @@ std::string jit_adjoint_source(const JitGeometry &geo, const PlannedSweep &sw, c
                     snprintf(buf, sizeof buf, "jit::grad_reg<P, R, %s, %d, 0x%xu>(vp, vl)", gn, (int)t.rb, t.creg);
                     expr = "if (" + fok_of(t) + ") part = " + std::string(buf) + ";";
                 }
-                snprintf(buf, sizeof buf, " jit::grad_store<P, %u>(acc, part);", slot);
+                snprintf(buf, sizeof buf, " jit::grad_store<P, %u, %s>(acc, part);", slot, gn);
                 body += "{ typename G::Acc part = G::zero(); " + expr + buf + " } ";
             }
             const std::string k = constants_of(t, i);
