@@ -15,7 +15,7 @@ constexpr int kLaneBits = 5;        // local bits 0..4 live across the 32 lanes 
 constexpr int kMaxStages = 48;      // register-layout stages per sweep
 constexpr int kMaxSweepGates = 256; // gates per sweep (the program is staged in shared memory)
 
-// Tile geometry per precision: 2^K amplitudes per tile (64 KiB), 2^R per
+// Largest tile geometry per precision: 2^K amplitudes per tile (64 KiB), 2^R per
 // thread, 32 * 2^(K-5-R) threads per CTA.
 template <class T> struct TileCfg;
 template <> struct TileCfg<float> {
