@@ -255,30 +255,51 @@ cudaError_t launch_masked_norm(const void *st, uint32_t n, uint64_t M, uint64_t 
     return cudaGetLastError();
 }
 
+// (re^2, im^2) of an amplitude as packed products and their errors.
+__device__ __forceinline__ ff2::v2 prob_square(float2 h, float2 l) {
+    const float2 p = ff2::mul(h, h);
+    return ff2::v2{p, ff2::fma(l, h, ff2::fma(h, l, ff2::fma(h, h, ff2::neg(p))))};
+}
+__device__ __forceinline__ ff2::v2 prob_square(float4 f) {  // re.hi, im.hi, re.lo, im.lo
+    return prob_square(make_float2(f.x, f.y), make_float2(f.z, f.w));
+}
+__device__ __forceinline__ ff2::v2 prob_square(cx<double> a) {
+    const ff::f2 re = ff::from_double(a.re), im = ff::from_double(a.im);
+    return prob_square(make_float2(re.h, im.h), make_float2(re.l, im.l));
+}
+__device__ __forceinline__ ff2::v2 prob_square(cx<float> a) {
+    const float2 h = make_float2(a.re, a.im), p = ff2::mul(h, h);
+    return ff2::v2{p, ff2::fma(h, h, ff2::neg(p))};
+}
+// (|a|^2, |b|^2) from their squares, in float-float.
+__device__ __forceinline__ ff2::v2 prob_pair(ff2::v2 a, ff2::v2 b) {
+    const ff2::v2 t = ff2::two_sum(make_float2(a.h.x, b.h.x), make_float2(a.h.y, b.h.y));
+    const float2 e = ff2::add(make_float2(a.l.x, b.l.x), make_float2(a.l.y, b.l.y));
+    return ff2::fast_two_sum(t.h, ff2::add(t.l, e));
+}
+
 // The same over the float-float resident form of a complex128 state
 // (re.hi, im.hi, re.lo, im.lo per amplitude): |a|^2 as a float-float dot
 // product, summed per thread in float-float (FP32-pipe work), then in binary64.
 __device__ __forceinline__ double masked_norm_body_ff(const float4 *__restrict__ st, uint64_t count, uint64_t M,
                                                       uint64_t V) {
-    // four loads in flight per thread and two independent sums: with one of
-    // each, a 24-qubit p1 (128 MiB read) took 41 us, two thirds of it waiting
-    ff::f2 acc{0.f, 0.f}, acc1{0.f, 0.f};
+    // four loads in flight per thread and two sums, packed; the last four
+    // guarded, where one by one they waited for memory up to three times
+    // (24-qubit p1, 128 MiB read: 32.1 -> 30.2 us, the bytes alone 20)
+    ff2::v2 acc{make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    auto prob = [](float4 f) {
-        const ff::f2 re{f.x, f.z}, im{f.y, f.w};
-        return ff::dot2(re, re, im, im);
-    };
-    for (; i + 3 * stride < count; i += 4 * stride) {
+    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < count; i += 4 * stride) {
         float4 f[4];
 #pragma unroll
-        for (int u = 0; u < 4; u++) f[u] = st[insert_zeros(i + u * stride, M) | V];
-        acc = ff::add(acc, ff::add(prob(f[0]), prob(f[1])));
-        acc1 = ff::add(acc1, ff::add(prob(f[2]), prob(f[3])));
+        for (int u = 0; u < 4; u++) {
+            const uint64_t x = i + u * stride;
+            f[u] = x < count ? st[insert_zeros(x, M) | V] : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+        acc = ff2::add(acc, ff2::add(prob_pair(prob_square(f[0]), prob_square(f[2])),
+                                     prob_pair(prob_square(f[1]), prob_square(f[3]))));
     }
-    for (; i < count; i += stride) acc = ff::add(acc, prob(st[insert_zeros(i, M) | V]));
-    acc = ff::add(acc, acc1);
-    return block_sum((double)acc.h + (double)acc.l);
+    const ff::f2 t = ff::add(ff::f2{acc.h.x, acc.l.x}, ff::f2{acc.h.y, acc.l.y});
+    return block_sum((double)t.h + (double)t.l);
 }
 
 __global__ void __launch_bounds__(kReduceThreads)
@@ -690,29 +711,6 @@ __global__ void __launch_bounds__(kReduceThreads)
 // a float-float dot product of the amplitude split into float-float (binary64
 // storage) or read as is (the float-float resident form) -- FP32-pipe work
 // instead of GB300's slow FP64 pipe, ~2^-48 relative per operation.
-// (re^2, im^2) of an amplitude as packed products and their errors.
-__device__ __forceinline__ ff2::v2 diag_square(float2 h, float2 l) {
-    const float2 p = ff2::mul(h, h);
-    return ff2::v2{p, ff2::fma(l, h, ff2::fma(h, l, ff2::fma(h, h, ff2::neg(p))))};
-}
-__device__ __forceinline__ ff2::v2 diag_square(float4 f) {  // re.hi, im.hi, re.lo, im.lo
-    return diag_square(make_float2(f.x, f.y), make_float2(f.z, f.w));
-}
-__device__ __forceinline__ ff2::v2 diag_square(cx<double> a) {
-    const ff::f2 re = ff::from_double(a.re), im = ff::from_double(a.im);
-    return diag_square(make_float2(re.h, im.h), make_float2(re.l, im.l));
-}
-__device__ __forceinline__ ff2::v2 diag_square(cx<float> a) {
-    const float2 h = make_float2(a.re, a.im), p = ff2::mul(h, h);
-    return ff2::v2{p, ff2::fma(h, h, ff2::neg(p))};
-}
-// (|a|^2, |b|^2) from their squares, in float-float.
-__device__ __forceinline__ ff2::v2 diag_probs(ff2::v2 a, ff2::v2 b) {
-    const ff2::v2 t = ff2::two_sum(make_float2(a.h.x, b.h.x), make_float2(a.h.y, b.h.y));
-    const float2 e = ff2::add(make_float2(a.l.x, b.l.x), make_float2(a.l.y, b.l.y));
-    return ff2::fast_two_sum(t.h, ff2::add(t.l, e));
-}
-
 constexpr int kDiagRun = 16;                   // amplitudes per thread per run
 constexpr int kDiagWarpSpan = 32 * kDiagRun;  // 512 consecutive amplitudes per warp
 
@@ -742,7 +740,7 @@ __global__ void __launch_bounds__(kReduceThreads, 2)
         const Load *src = reinterpret_cast<const Load *>(st) + b + lane;
         ff2::v2 p[H];  // amplitudes u and u + H
 #pragma unroll
-        for (int u = 0; u < H; u++) p[u] = diag_probs(diag_square(src[32 * u]), diag_square(src[32 * (u + H)]));
+        for (int u = 0; u < H; u++) p[u] = prob_pair(prob_square(src[32 * u]), prob_square(src[32 * (u + H)]));
 #pragma unroll
         for (int h = 1; h < H; h <<= 1) {
 #pragma unroll
