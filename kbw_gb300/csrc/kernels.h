@@ -114,10 +114,8 @@ struct PauliTilePass {
     uint8_t hq[16];
     PauliTileTerm t[kMaxTerms];  // window by window, then the rest; by flip mask and part (im)
 };
-// Largest tile of the pass kernel: two buffers of 32 KiB, three CTAs per SM.
-// Registers down to kPauliMinBits qubits are one tile of their own size.
+// Tile of the pass kernel: one buffer of 32 KiB, three CTAs per SM.
 template <class T> constexpr int pauli_tile_bits() { return sizeof(T) == 4 ? 12 : 11; }
-constexpr int kPauliMinBits = 9;
 template <class T>
 cudaError_t launch_pauli_tile(const void *st, uint32_t n, bool ff_resident, const PauliTilePass &p,
                               const ReduceScratch &rs, int *err, cudaStream_t s);
