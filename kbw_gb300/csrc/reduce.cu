@@ -123,23 +123,46 @@ __device__ double sum_partials(const double *partials, int nblocks, int stride, 
     return block_sum(v);
 }
 
-// Sums of up to 32 terms at once.  v[k]: this thread's share of term k; lane k
-// returns the warp's sum of term k.  Halving exchange: 31 float-float additions
-// instead of 5 per term, and no FP64 instruction: a double tree over 32 terms
-// took 19 us of a 25 us launch on GB300's FP64 pipe.
-__device__ __forceinline__ ff::f2 warp_sum_terms(ff::f2 (&v)[kMaxTerms]) {
+// A sum of floats in three parts: the errors of both upper additions are kept,
+// so a few dozen float-float shares add up without another rounding.
+struct f3 {
+    float h, m, l;
+};
+__device__ __forceinline__ f3 add(const f3 &a, const f3 &b) {
+    const ff::f2 h = ff::two_sum(a.h, b.h), t = ff::two_sum(a.m, b.m), m = ff::two_sum(t.h, h.l);
+    return f3{h.h, m.h, ff::add(ff::add(a.l, b.l), ff::add(t.l, m.l))};
+}
+__device__ __forceinline__ double to_double(const f3 &a) { return (double)a.h + ((double)a.m + (double)a.l); }
+
+// Sums of up to 32 terms at once.  share(k): this thread's of term k; lane k
+// returns the warp's sum of term k.  Halving exchange: 31 additions instead of
+// 5 per term, and no FP64 instruction: a double tree over 32 terms took 19 us
+// of a 25 us launch on GB300's FP64 pipe.  In three parts: a float-float tree
+// rounds to 48 bits where the warps' sums average out least (12 qubits, rms
+// error of a string without flips 3.5e-16 with a double tree, 6.9e-16 with
+// that one).
+template <class F>
+__device__ __forceinline__ f3 warp_sum_terms(F &&share) {
     const int lane = threadIdx.x & 31;
+    const bool top = (lane & 16) != 0;
+    f3 t[kMaxTerms / 2];
 #pragma unroll
-    for (int w = 16; w > 0; w >>= 1) {
+    for (int i = 0; i < kMaxTerms / 2; i++) {
+        const f3 a = share(i), b = share(i + 16), keep = top ? b : a, send = top ? a : b;
+        t[i] = add(keep, f3{__shfl_xor_sync(0xffffffffu, send.h, 16), __shfl_xor_sync(0xffffffffu, send.m, 16),
+                            __shfl_xor_sync(0xffffffffu, send.l, 16)});
+    }
+#pragma unroll
+    for (int w = 8; w > 0; w >>= 1) {
         const bool up = (lane & w) != 0;
 #pragma unroll
         for (int i = 0; i < w; i++) {
-            const ff::f2 keep = up ? v[i + w] : v[i], send = up ? v[i] : v[i + w];
-            const ff::f2 got{__shfl_xor_sync(0xffffffffu, send.h, w), __shfl_xor_sync(0xffffffffu, send.l, w)};
-            v[i] = ff::add(keep, got);
+            const f3 keep = up ? t[i + w] : t[i], send = up ? t[i] : t[i + w];
+            t[i] = add(keep, f3{__shfl_xor_sync(0xffffffffu, send.h, w), __shfl_xor_sync(0xffffffffu, send.m, w),
+                                __shfl_xor_sync(0xffffffffu, send.l, w)});
         }
     }
-    return v[0];
+    return t[0];
 }
 
 // The grid's sums of nt terms into rs.result: lane k of every warp holds its
@@ -775,12 +798,11 @@ __global__ void __launch_bounds__(kReduceThreads, 2)
         }
         __syncwarp();
     }
-    ff::f2 sums[kMaxTerms];
-#pragma unroll
-    for (int k = 0; k < kMaxTerms; k++)
-        sums[k] = (k & 1) ? ff::f2{acc[k / 2].h.y, acc[k / 2].l.y} : ff::f2{acc[k / 2].h.x, acc[k / 2].l.x};
-    const ff::f2 v = warp_sum_terms(sums);
-    finish_terms((double)v.h + (double)v.l, nt, rs);
+    const f3 sum = warp_sum_terms([&](int k) {
+        const ff2::v2 &a = acc[k / 2];
+        return (k & 1) ? f3{a.h.y, a.l.y, 0.f} : f3{a.h.x, a.l.x, 0.f};
+    });
+    finish_terms(to_double(sum), nt, rs);
 }
 
 template <class T>
@@ -816,8 +838,7 @@ cudaError_t launch_pauli_group(const void *st, uint32_t n, const PauliGroup &g, 
 // apart until the end, so 12 packed instructions form and add one pair.
 // A product is its rounded high part plus the exact error and the cross terms
 // (complex128: the tile holds float-float amplitudes, binary64 split once per
-// tile); it is added without normalising (TwoSum of the high parts, errors
-// into the low one).
+// tile); it is added without normalising (PauliSum).
 // Strings whose flips lie within three neighbouring tile bits run in windows:
 // a thread holds the 8 amplitudes of its window in registers, read once for
 // all strings of the window, and a pair is two registers.  Lane l takes the
@@ -826,11 +847,14 @@ cudaError_t launch_pauli_group(const void *st, uint32_t n, const PauliGroup &g, 
 // amplitudes of every pair.  Strings with one flip mask and part (Re or Im)
 // form a group: the products are formed once and every string adds them with
 // its signs.
-// Tile sums gather in float-float and go to binary64 every kPauliFlush tiles:
+// Tile sums gather in three floats and go to binary64 every kPauliFlush tiles:
 // a conversion per string and tile kept GB300's FP64 pipe busy half of the
 // time.
 // Measured, the 27 X strings of a ring TFIM on 27 qubits in float-float, four
-// passes: 5.8 -> 4.0 ms (a pass that only reads: 0.38 ms).
+// passes: 5.8 -> 4.2 ms (a pass that only reads: 0.38 ms).  With sums of two
+// floats it was 4.0 ms, and a string's value less exact than before (14
+// qubits, random states, rms: binary64 sums per tile 4.2e-17, two floats
+// 5.4e-17, three 2.5e-17; complex64 1.8e-17, 2.6e-17, 1.0e-17).
 __device__ __forceinline__ uint64_t tile_base_of(uint64_t tau, uint32_t l, uint32_t m, const uint8_t *hq) {
     uint64_t b = tau << l;
     for (uint32_t j = 0; j < m; j++) b = insert_zero(b, hq[j]);
@@ -867,24 +891,41 @@ __device__ __forceinline__ ff2::v2 pauli_product(const ff2::v2 &a, const ff2::v2
     if constexpr (FFV) lo = ff2::fma(a.l, b.h, ff2::fma(a.h, b.l, lo));
     return ff2::v2{p, lo};
 }
-__device__ __forceinline__ void pauli_add(ff2::v2 &S, float2 p, float2 lo) {
+// A sum over a tile, lane by lane: the products' high parts, their low parts
+// and the errors of adding the high ones, each in a sum of its own (joined
+// after every product they round where the start of this chain is longest:
+// rms error of a thread's sum 2.4e-15 -> 1.1e-15 of itself in complex64,
+// 3.7e-15 -> 2.7e-15 in float-float, at the same number of instructions).
+struct PauliSum {
+    float2 h, lo, er;
+};
+__device__ __forceinline__ void pauli_add(PauliSum &S, float2 p, float2 lo) {
     const ff2::v2 t = ff2::two_sum(S.h, p);
-    S = ff2::v2{t.h, ff2::add(S.l, ff2::add(t.l, lo))};
+    S = PauliSum{t.h, ff2::add(S.lo, lo), ff2::add(S.er, t.l)};
 }
-// a thread's sum over the tile, its lanes joined, into the string's running sum (both unnormalised)
-template <bool IM>
-__device__ __forceinline__ void pauli_tail(const ff2::v2 &S, bool neg, ff::f2 &acc) {
+// a thread's sum over the tile, its lanes joined, into the string's running
+// sum.  Float-float states keep the running sum's rounding errors too: the
+// sums of complex64 products have the bits to spare (32 tiles: 0.8e-14 of one
+// tile's sum; in plain float-float 2.5e-14).
+template <bool FFV, bool IM>
+__device__ __forceinline__ void pauli_tail(const PauliSum &S, bool neg, f3 &acc) {
     const float sn = neg ? -1.f : 1.f, sy = IM ? -sn : sn;
     const ff::f2 t = ff::two_sum(__fmul_rn(S.h.x, sn), __fmul_rn(S.h.y, sy)), r = ff::two_sum(acc.h, t.h);
-    const float l = __fmaf_rn(S.l.x, sn, __fmul_rn(S.l.y, sy));
-    acc = ff::f2{r.h, ff::add(acc.l, ff::add(ff::add(r.l, t.l), l))};
+    const float lo = __fmaf_rn(S.lo.x, sn, __fmul_rn(S.lo.y, sy));
+    const float er = ff::add(__fmaf_rn(S.er.x, sn, __fmaf_rn(S.er.y, sy, t.l)), r.l);
+    if constexpr (FFV) {
+        const ff::f2 g = ff::two_sum(acc.m, lo), k = ff::two_sum(g.h, er);
+        acc = f3{r.h, k.h, ff::add(acc.l, ff::add(g.l, k.l))};
+    } else {
+        acc = f3{r.h, ff::add(acc.m, lo), ff::add(acc.l, er)};
+    }
 }
 
 // The strings of one window with flip mask X and part IM: the four products,
 // then every string's signed sum.
 template <bool FFV, bool IM, int X>
 __device__ __forceinline__ void window_group(const PauliTilePass &p, const ff2::v2 (&a)[8], uint32_t &k, uint32_t w,
-                                             uint32_t F, uint32_t negs, uint32_t signs, ff::f2 *acc) {
+                                             uint32_t F, uint32_t negs, uint32_t signs, f3 *acc) {
     constexpr int hb = X >= 4 ? 2 : (X >= 2 ? 1 : 0);
     ff2::v2 c[4];
 #pragma unroll
@@ -895,7 +936,7 @@ __device__ __forceinline__ void window_group(const PauliTilePass &p, const ff2::
     const uint32_t end = p.t[k].group_end;
 #pragma unroll 1
     for (; k < end; k++) {
-        ff2::v2 S = c[0];
+        PauliSum S{c[0].h, c[0].l, make_float2(0.f, 0.f)};
         bool neg = ((negs >> k) & 1u) != 0;
         if ((signs >> k) & 1u) {
             const uint32_t zl = p.t[k].zl, zr = zl >> w;
@@ -910,7 +951,7 @@ __device__ __forceinline__ void window_group(const PauliTilePass &p, const ff2::
 #pragma unroll
             for (int i = 1; i < 4; i++) pauli_add(S, c[i].h, c[i].l);
         }
-        pauli_tail<IM>(S, neg, acc[k]);
+        pauli_tail<FFV, IM>(S, neg, acc[k]);
     }
 }
 
@@ -919,7 +960,7 @@ __device__ __forceinline__ void window_group(const PauliTilePass &p, const ff2::
 // inside the tile.
 template <bool FFV>
 __device__ __forceinline__ void pauli_window(const PauliTilePass &p, const void *tile, uint32_t k0, uint32_t negs,
-                                             uint32_t signs, ff::f2 *acc) {
+                                             uint32_t signs, f3 *acc) {
     const uint32_t w = p.t[k0].w, low = (1u << w) - 1u, groups = p.t[k0].groups;
     for (uint32_t q = threadIdx.x; q < (1u << (p.K - 3)); q += kPauliThreads) {
         const uint32_t sw = w < 3 ? ((threadIdx.x & 31u) >> w) & 7u : 0u;
@@ -939,14 +980,14 @@ __device__ __forceinline__ void pauli_window(const PauliTilePass &p, const void 
 // C strings k0.. of one group over the tile, both amplitudes of a pair read.
 template <bool FFV, bool IM, int C>
 __device__ __forceinline__ void pauli_group_terms(const PauliTilePass &p, const void *tile, uint32_t k0, uint32_t negs,
-                                                  ff::f2 *acc) {
+                                                  f3 *acc) {
     const uint32_t xl = p.t[k0].xl, pairs = 1u << (p.K - 1);
     const uint32_t keep = (1u << p.t[k0].hb) - 1u;
-    ff2::v2 S[C];
+    PauliSum S[C];
     uint32_t zl[C];
 #pragma unroll
     for (int c = 0; c < C; c++) {
-        S[c] = ff2::v2{make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+        S[c] = PauliSum{make_float2(0.f, 0.f), make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
         zl[c] = p.t[k0 + c].zl;
     }
 #pragma unroll 4
@@ -960,12 +1001,12 @@ __device__ __forceinline__ void pauli_group_terms(const PauliTilePass &p, const 
         }
     }
 #pragma unroll
-    for (int c = 0; c < C; c++) pauli_tail<IM>(S[c], ((negs >> (k0 + c)) & 1u) != 0, acc[k0 + c]);
+    for (int c = 0; c < C; c++) pauli_tail<FFV, IM>(S[c], ((negs >> (k0 + c)) & 1u) != 0, acc[k0 + c]);
 }
 
 template <bool FFV, bool IM>
 __device__ __forceinline__ void pauli_group(const PauliTilePass &p, const void *tile, uint32_t k0, uint32_t k1,
-                                            uint32_t negs, ff::f2 *acc) {
+                                            uint32_t negs, f3 *acc) {
     for (; k0 + 2 <= k1; k0 += 2) pauli_group_terms<FFV, IM, 2>(p, tile, k0, negs, acc);
     if (k0 < k1) pauli_group_terms<FFV, IM, 1>(p, tile, k0, negs, acc);
 }
@@ -991,10 +1032,10 @@ __global__ void __launch_bounds__(kPauliThreads, 3) k_pauli_tile(const void *__r
         fence_mbar_init();
     }
     const uint64_t tiles = 1ull << (n - K);
-    ff::f2 acc[kMaxTerms];  // (local memory, touched once per string and tile)
+    f3 acc[kMaxTerms];  // (local memory, touched once per string and tile)
     double wide[kMaxTerms];
     bool flushed = false;
-    for (int k = 0; k < kMaxTerms; k++) acc[k] = ff::f2{0.f, 0.f};
+    for (int k = 0; k < kMaxTerms; k++) acc[k] = f3{0.f, 0.f, 0.f};
     __syncthreads();
     auto issue_load = [&](uint64_t tau) {
         if (threadIdx.x < 32) {
@@ -1020,7 +1061,10 @@ __global__ void __launch_bounds__(kPauliThreads, 3) k_pauli_tile(const void *__r
         if constexpr (FFV && !kFF) {
             for (uint32_t u = threadIdx.x; u < N; u += kPauliThreads) {
                 const cx<double> a = reinterpret_cast<const cx<double> *>(tile)[u];
-                const ff::f2 r = ff::from_double(a.re), i = ff::from_double(a.im);
+                // (rounded, not cut: the low parts half as large and of both signs)
+                ff::f2 r = ff::from_double(a.re), i = ff::from_double(a.im);
+                r = ff::fast_two_sum(r.h, r.l);
+                i = ff::fast_two_sum(i.h, i.l);
                 reinterpret_cast<ff2::v2 *>(tile)[u] = ff2::v2{make_float2(r.h, i.h), make_float2(r.l, i.l)};
             }
             __syncthreads();
@@ -1042,8 +1086,8 @@ __global__ void __launch_bounds__(kPauliThreads, 3) k_pauli_tile(const void *__r
         if (tau + gridDim.x < tiles) issue_load(tau + gridDim.x);
         if ((it + 1) % (uint32_t)kPauliFlush == 0) {
             for (int k = 0; k < (int)nt; k++) {
-                wide[k] = (flushed ? wide[k] : 0.0) + ((double)acc[k].h + (double)acc[k].l);
-                acc[k] = ff::f2{0.f, 0.f};
+                wide[k] = (flushed ? wide[k] : 0.0) + to_double(acc[k]);
+                acc[k] = f3{0.f, 0.f, 0.f};
             }
             flushed = true;
         }
@@ -1055,10 +1099,10 @@ __global__ void __launch_bounds__(kPauliThreads, 3) k_pauli_tile(const void *__r
             const double v = warp_sum(wide[k]);
             if (lane == k) mine = v;
         }
-#pragma unroll 1
-    for (int k = 0; k < (int)nt; k++) acc[k] = ff::two_sum(acc[k].h, acc[k].l);
-    const ff::f2 r = warp_sum_terms(acc);
-    mine += (double)r.h + (double)r.l;
+    mine += to_double(warp_sum_terms([&](int k) {
+        const ff::f2 t = ff::two_sum(acc[k].m, acc[k].l);
+        return f3{acc[k].h, t.h, t.l};
+    }));
     finish_terms(lane < (int)nt ? mine * p.t[lane].factor : 0.0, nt, rs);
 }
 
