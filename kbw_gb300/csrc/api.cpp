@@ -526,20 +526,27 @@ int32_t kbwg_sample(kbwg_sim *s, const uintptr_t *qubits, uintptr_t n_qubits, ui
         return KBWG_ECAPACITY;
     }
     CUDA_TRY(flush_queue(*s));  // (a float-float resident state is sampled as is)
-    const bool ff = s->ff_resident;
+    bool ff = s->ff_resident;
     const int B = sample_blocks(s->n);
     CUDA_TRY(s->tmp0.ensure((size_t)B * 8));
     double *d_bs = (double *)s->tmp0.ptr;
-    CUDA_TRY(dispatch(s, [&](auto *tp) {
-        using T = std::remove_pointer_t<decltype(tp)>;
-        return launch_weight_blocksum<T>(s->state, s->n, ff, d_bs, s->stream);
-    }));
     std::vector<double> bs(B), pre(B + 1);
-    CUDA_TRY(copy_async(bs.data(), d_bs, (size_t)B * 8, cudaMemcpyDeviceToHost, s->stream));
-    CUDA_TRY(cudaStreamSynchronize(s->stream));
-    pre[0] = 0.0;
-    for (int b = 0; b < B; b++) pre[b + 1] = pre[b] + bs[b];
-    const double total = pre[B];
+    double total = 0.0;
+    for (;;) {
+        CUDA_TRY(dispatch(s, [&](auto *tp) {
+            using T = std::remove_pointer_t<decltype(tp)>;
+            return launch_weight_blocksum<T>(s->state, s->n, ff, d_bs, s->stream);
+        }));
+        CUDA_TRY(copy_async(bs.data(), d_bs, (size_t)B * 8, cudaMemcpyDeviceToHost, s->stream));
+        CUDA_TRY(cudaStreamSynchronize(s->stream));
+        pre[0] = 0.0;
+        for (int b = 0; b < B; b++) pre[b + 1] = pre[b] + bs[b];
+        total = pre[B];
+        // (a loaded state far from unit norm: squares outside float's range)
+        if (!ff || (total > 1e-6 && total < 1e30)) break;
+        ff = false;
+        CUDA_TRY(ensure_binary64(*s));
+    }
     if (!(total > 0.0)) return fail(KBWG_EWEIGHT, "all sampling weights are zero");
     if (shots == 0) return KBWG_OK;
     const double scale = host_uniform_scale(total);

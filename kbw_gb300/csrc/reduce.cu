@@ -1150,26 +1150,13 @@ __device__ __forceinline__ double weight(cx<T> a) {
     return __fma_rn(r, r, __dmul_rn(i, i));
 }
 
-// The same for the float-float resident form; kept as a float-float value.
-__device__ __forceinline__ ff::f2 weight_ff(float4 f) {
-    const ff::f2 re{f.x, f.z}, im{f.y, f.w}, w = ff::dot2(re, re, im, im);
-    if (w.h > 1.00001e-30f) return w;
-    if (w.h < 0.99999e-30f || !((double)w.h + (double)w.l > 1e-30)) return ff::f2{0.f, 0.f};
-    return w;
-}
-__device__ __forceinline__ ff::f2 weight_ff(cx<float> a) {  // exact products, summed in float-float
-    if (!above_eps(a)) return ff::f2{0.f, 0.f};
-    const float pr = __fmul_rn(a.re, a.re), pi = __fmul_rn(a.im, a.im);
-    const ff::f2 s = ff::two_sum(pr, pi);
-    const float e = __fadd_rn(__fmaf_rn(a.re, a.re, -pr), __fmaf_rn(a.im, a.im, -pi));
-    return ff::fast_two_sum(s.h, __fadd_rn(s.l, e));
-}
-// Weight of amplitude i of a state of either type or form.
+// Weight of amplitude i of a state of either type or form, in binary64: a
+// float-float amplitude is what ensure_binary64 would make of it.
 template <class T, bool kFF>
 __device__ __forceinline__ double weight_at(const void *st, uint64_t i) {
     if constexpr (kFF) {
-        const ff::f2 w = weight_ff(reinterpret_cast<const float4 *>(st)[i]);
-        return (double)w.h + (double)w.l;
+        const float4 f = reinterpret_cast<const float4 *>(st)[i];  // re.hi, im.hi, re.lo, im.lo
+        return weight(cx<double>{ff::to_double(ff::f2{f.x, f.z}), ff::to_double(ff::f2{f.y, f.w})});
     } else {
         return weight(reinterpret_cast<const cx<T> *>(st)[i]);
     }
@@ -1254,25 +1241,43 @@ cudaError_t launch_dump_write(const void *st, uint32_t n, const uint64_t *offset
 }
 
 // ---- sampling -------------------------------------------------------------------
-// Both kernels walk a block's range in chunks of blockDim with the same scan,
-// so the in-block running sums of the pick kernel end exactly at the block
-// sums the host prefixes.
-// (Sums only: the picks scan the few blocks that hold a shot.  Scanning every
-// block here too kept the FP64 pipe busy for 372 us on 24 qubits.)
+// The block sums only say which block a shot falls into; the picks scan the few
+// blocks that hold one.  (Scanning every block here too kept the FP64 pipe busy
+// for 372 us on 24 qubits.)  The scan's total may differ from the sum in the
+// last bits: a shot between the two takes the block's last amplitude with a
+// weight.  The sums are no less exact than in binary64, which float-float ones
+// are not (they move the border between two blocks by up to 2^-49 of it):
+// complex64 and binary64 states on the FP64 pipe, float-float states as three
+// floats per part, whose roundings stay below 2^-60 (24 qubits, a whole
+// experiment: on the FP64 pipe, after ensure_binary64's conversion of every
+// amplitude, 0.39 ms more).
 template <class T, bool kFF>
 __global__ void __launch_bounds__(256) k_weight_blocksum(const void *__restrict__ st, uint64_t R, double *blocksum) {
     const uint64_t base = (uint64_t)blockIdx.x * R;
     double sum = 0.0;
-    if constexpr (sizeof(T) == 8 && !kFF) {
+    if constexpr (!kFF) {
 #pragma unroll 4
         for (uint64_t i = threadIdx.x; i < R; i += 256) sum += weight_at<T, kFF>(st, base + i);
     } else {
-        using Mem = typename std::conditional<kFF, float4, cx<float>>::type;
-        ff::f2 acc{0.f, 0.f};
+        const float4 *amp = reinterpret_cast<const float4 *>(st) + base;  // re.hi, im.hi, re.lo, im.lo
+        float2 ah = make_float2(0.f, 0.f), am = ah, al = ah;
 #pragma unroll 4
-        for (uint64_t i = threadIdx.x; i < R; i += 256)
-            acc = ff::add(acc, weight_ff(reinterpret_cast<const Mem *>(st)[base + i]));
-        sum = (double)acc.h + (double)acc.l;
+        for (uint64_t i = threadIdx.x; i < R; i += 256) {
+            const float4 f = amp[i];
+            float2 h = make_float2(f.x, f.y), l = make_float2(f.z, f.w);
+            float2 p = ff2::mul(h, h);
+            const float q = __fadd_rn(p.x, p.y);
+            if (!(q > 1.00001e-30f) && !(q > 0.99999e-30f && weight_at<T, true>(st, base + i) > 0.0))
+                h = l = p = make_float2(0.f, 0.f);  // (no weight: see weight())
+            const float2 e = ff2::fma(h, h, ff2::neg(p)), l2 = ff2::add(l, l), c = ff2::mul(h, l2);
+            const float2 ec = ff2::fma(h, l2, ff2::neg(c));  // p + e + c + ec + l l: the squares
+            const ff2::v2 t = ff2::two_sum(ah, p), u = ff2::two_sum(am, t.l), v = ff2::two_sum(u.h, e),
+                          w = ff2::two_sum(v.h, c);
+            ah = t.h;
+            am = w.h;
+            al = ff2::add(al, ff2::fma(l, l, ff2::add(ff2::add(u.l, v.l), ff2::add(w.l, ec))));
+        }
+        sum = to_double(add(f3{ah.x, am.x, al.x}, f3{ah.y, am.y, al.y}));
     }
     const double t = block_sum(sum);
     if (threadIdx.x == 0) blocksum[blockIdx.x] = t;

@@ -62,3 +62,50 @@ def test_shares_of_a_warp(prec, n, string):
         if odd:  # (i^ny of one Y)
             got = -got if abs(got + want) < abs(got - want) else got
         assert abs(got - want) <= 3 * U * np.abs(parts).sum()
+
+
+def _pick(sim, n, draw):
+    states, counts = sim.sample(list(range(n))[::-1], 1, [draw])
+    return int(states[0])
+
+
+@pytest.mark.parametrize("arith", ["c64", "c128", "ff"])
+def test_border_between_two_samples(arith):
+    """Two weights in blocks of their own, and draws a few last places around
+    their border: weights, total and the drawn weight as binary64 rounds them
+    (re^2 of a float is exact there, re^2 + im^2 rounded once)."""
+    n, rng = 14, np.random.default_rng(4)
+    sim = DenseGB300(n, "c64" if arith == "c64" else "c128", fast_c128=arith == "ff")
+    for _ in range(40):
+        a = np.zeros(1 << n, np.complex64)
+        a[0], a[-1] = (rng.uniform(0.3, 1.0, 2) + 1j * rng.uniform(0.3, 1.0, 2)).astype(np.complex64)
+        sim.set_state(a)
+        if arith == "ff":
+            sim.apply([(C.X, 3, (), 0.0)])  # (exact: the two states swap bit 3)
+        w = (np.longdouble(a.real) ** 2 + np.longdouble(a.imag) ** 2).astype(np.float64)
+        total = w[0] + w[-1]
+        scale = total
+        while scale * (1.0 - np.finfo(np.float64).eps) >= total:
+            scale = np.nextafter(scale, 0.0)
+        first, last = (8, (1 << n) - 9) if arith == "ff" else (0, (1 << n) - 1)
+        draw = w[0] / scale
+        for _ in range(4):
+            draw = np.nextafter(draw, 0.0)
+        for _ in range(9):
+            assert _pick(sim, n, draw) == (first if draw * scale < w[0] else last)
+            draw = np.nextafter(draw, 1.0)
+
+
+@pytest.mark.parametrize("arith", ["c64", "ff"])
+@pytest.mark.parametrize("size", [1e25, 1e-13])
+def test_samples_far_from_unit_norm(arith, size):
+    """Weights beyond float's range."""
+    n = 12
+    if arith == "c64" and size < 1:
+        size = 1e-4  # (complex64 drops amplitudes below 1e-6)
+    a = np.zeros(1 << n, np.complex128)
+    a[5], a[4000] = 3 * size, 4j * size
+    sim = DenseGB300(n, "c64" if arith == "c64" else "c128", fast_c128=arith == "ff")
+    sim.set_state(a)
+    sim.apply([(C.X, 0, (), 0.0)])
+    assert [_pick(sim, n, d) for d in (0.1, 0.35, 0.37, 0.9)] == [4, 4, 4001, 4001]
