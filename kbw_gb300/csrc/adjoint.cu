@@ -763,10 +763,11 @@ static void defer_sweep(PlannedSweep &sw, bool last, DdFactor &g, std::vector<do
         mult[i] = mag.h * mag.h;
         if (!defer || t.cl || t.co) continue;
         if (t.cls == TG_RZ) {
-            const double u[4] = {t.c[0], t.c[1], t.c[2], t.c[3]};
-            defer_diagonal(u, t.c[0], t.c[1]);
+            const DeferredDiagonal d = defer_diagonal(t.c);
+            g.times(d.f);
+            t.c[0] = d.c;
+            t.c[1] = d.s;
             t.c[2] = t.c[3] = 0.0;
-            g.times(u[0], u[1]);
             t.cls = TG_P;
             t.op = (uint8_t)(t.op - (TG_RZ - TG_P) * (t.op < OP_DFIX ? 4 : 1));
         } else if (t.cls == TG_H && grown < kAdjDeferRun) {

@@ -664,13 +664,12 @@ static std::vector<GateDesc> defer_scale(int arith, const GateDesc *gates, size_
             grew = true;
         } else if (defer && x.kind == G_RZ && x.ctrl == 0) {
             // u0 diag(1, u1 conj(u0)) (for RZ(t): u1 conj(u0) = e^{it}; also a folded general diagonal)
-            double c, sn;
-            defer_diagonal(x.c, c, sn);
-            g.times(x.c[0], x.c[1]);
+            const DeferredDiagonal d = defer_diagonal(x.c);
+            g.times(d.f);
             complex_g = pending = true;
             x.kind = G_P;
-            x.c[0] = c;
-            x.c[1] = sn;
+            x.c[0] = d.c;
+            x.c[1] = d.s;
             x.c[2] = x.c[3] = 0.0;
         } else if (drot && (x.kind == G_RX || x.kind == G_RY) && x.ctrl == 0) {
             const DeferredRotation r = defer_rotation(arith, x.c[0], x.c[1]);
