@@ -613,8 +613,9 @@ static cudaError_t run_fused_t(Sim &s, const GateDesc *gates, size_t count) {
 //     float-float 15 packed operations instead of 19 per amplitude.
 // Each H, RX or RY grows the state by at most sqrt(2), so kDeferRun of them
 // stay inside float's range before g is applied (a structural count: the
-// plan must not depend on the angles).  P(+-pi/2) and P(pi) become exact
-// multiplications by i^q (not in complex64).
+// plan must not depend on the angles).  In float-float P(+-pi/2) and P(pi)
+// become exact multiplications by i^q (1e-15 is below its 48 bits; binary64
+// and complex64 keep the phase they are given).
 // A SCALE costs about two deferred rotations' savings, so lists with fewer
 // than kDeferMin such gates keep the full forms (float-float always drops H's
 // and RZ's factors: its multiplications cost most).
@@ -679,7 +680,7 @@ static std::vector<GateDesc> defer_scale(int arith, const GateDesc *gates, size_
             x.c[1] = r.cot ? 1.0 : 0.0;
             grew = true;
         }
-        if (x.kind == G_P && arith != ARITH_C64) {
+        if (x.kind == G_P && arith == ARITH_FF) {
             const double c = x.c[0], sn = x.c[1], t = 1e-15;
             int q = 0;
             if (fabs(c) < t && fabs(sn - 1.0) < t) q = 1;

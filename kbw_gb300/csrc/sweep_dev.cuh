@@ -153,14 +153,10 @@ struct Exact {
         return Amp{xadd(xmul(k.c0, self.re), xmul(ss, o.re)), xadd(xmul(k.c0, self.im), xmul(ss, o.im))};
     }
     static __device__ __forceinline__ Amp cmul(Amp a, T c, T s) { return cmul_exact(a, c, s); }
-    // |1> * i^q and the deferred forms never run in program order
+    // |1> * i^q is a float-float gate, the deferred forms never run in program order
     static constexpr bool kDefer = false;
-    static __device__ __forceinline__ int power_of_i(const K4 &k) { return (int)k.c0; }
-    static __device__ __forceinline__ Amp pi_mul(Amp a, int q) {
-        if (q == 1) return Amp{-a.im, a.re};
-        if (q == 2) return Amp{-a.re, -a.im};
-        return Amp{a.im, -a.re};
-    }
+    static __device__ __forceinline__ Amp pi_mul(Amp a, int) { return a; }
+    static __device__ __forceinline__ int power_of_i(const K4 &) { return 0; }
     static __device__ __forceinline__ Amp smul(Amp a, T c) { return Amp{xmul(a.re, c), xmul(a.im, c)}; }
     // negated where s (a sign bit) is set
     static __device__ __forceinline__ T flip1(T x, uint32_t s) {
@@ -340,8 +336,8 @@ struct FastP {
     static __device__ __forceinline__ Amp cmul(Amp a, float c, float s) {
         return __ffma2_rn(a, bc(c), __fmul2_rn(swp(a), make_float2(-s, s)));
     }
-    // |1> * i^q stays a phase gate in complex64: bodies that pick q at run time
-    // made the interpreted 2^13 kernel spill (16 -> 112 bytes, up to 25 % slower)
+    // |1> * i^q is a float-float gate (bodies that pick q at run time made the
+    // interpreted 2^13 kernel spill, 16 -> 112 bytes, up to 25 % slower)
     static __device__ __forceinline__ Amp pi_mul(Amp a, int) { return a; }
     static __device__ __forceinline__ int power_of_i(const K4 &) { return 0; }
     static __device__ __forceinline__ Amp smul(Amp a, float c) { return mul_rn(a, c); }
