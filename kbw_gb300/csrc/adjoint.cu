@@ -712,7 +712,7 @@ static cudaError_t adj_grow(B *&p, size_t &cap, size_t want) {
     if (p) cudaFree(p);
     p = nullptr;
     cap = 0;
-    const cudaError_t e = cudaMalloc((void **)&p, want);
+    const cudaError_t e = device_malloc((void **)&p, want);
     if (e == cudaSuccess) cap = want;
     return e;
 }
@@ -1240,7 +1240,7 @@ static int32_t adjoint_run(Sim &s, const std::vector<GateDesc> &fwd, const std::
     // scratch (kept from an earlier call when it is there)
     if (sc.sb != sb) sc.release_states();
     if (!sc.lam) {
-        e = cudaMalloc(&sc.lam, sb);
+        e = device_malloc(&sc.lam, sb);
         if (e != cudaSuccess) return fail_cuda(e, "lambda buffer");
         sc.sb = sb;
     }
@@ -1257,13 +1257,11 @@ static int32_t adjoint_run(Sim &s, const std::vector<GateDesc> &fwd, const std::
     if (sc.ckpt.size() < want || sb > kSmallState) {
         e = cudaMemGetInfo(&free_b, &total_b);
         if (e != cudaSuccess) return fail_cuda(e, "memory query");
+        free_b += batch_kept_bytes();  // (device_malloc gets it back)
     }
     while (sc.ckpt.size() < want && sb <= (size_t)(0.8 * (double)free_b)) {
         void *c = nullptr;
-        if (cudaMalloc(&c, sb) != cudaSuccess) {
-            cudaGetLastError();
-            break;
-        }
+        if (device_malloc(&c, sb) != cudaSuccess) break;
         sc.ckpt.push_back(c);
         free_b -= std::min(free_b, sb);
     }

@@ -36,7 +36,7 @@ cudaError_t DevBuf::ensure(size_t bytes) {
     ptr = nullptr;
     cap = 0;
     size_t want = std::max(bytes, (size_t)4096);
-    cudaError_t e = cudaMalloc(&ptr, want);
+    cudaError_t e = device_malloc(&ptr, want);
     if (e == cudaSuccess) cap = want;
     return e;
 }
@@ -242,14 +242,11 @@ int32_t kbwg_new(uintptr_t num_qubits, int32_t precision, uint32_t flags, kbwg_s
     };
     cudaError_t e = cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking);
     if (e != cudaSuccess) return cleanup(KBWG_ECUDA, cudaGetErrorString(e));
-    e = cudaMalloc(&s->state, s->ns * s->elem);
-    if (e != cudaSuccess) {
-        cudaGetLastError();
-        return cleanup(KBWG_ENOMEM, std::string("state allocation: ") + cudaGetErrorString(e));
-    }
+    e = device_malloc(&s->state, s->ns * s->elem);
+    if (e != cudaSuccess) return cleanup(KBWG_ENOMEM, std::string("state allocation: ") + cudaGetErrorString(e));
     const size_t part = (size_t)kReduceBlocks * kMaxTerms * sizeof(double);
     const size_t scratch_bytes = part + 256 + 256 + sizeof(MeasureCtl) + 256;
-    e = cudaMalloc(&s->scratch, scratch_bytes);
+    e = device_malloc(&s->scratch, scratch_bytes);
     if (e != cudaSuccess) return cleanup(KBWG_ENOMEM, "scratch allocation");
     char *p = (char *)s->scratch;
     s->rs.partials = (double *)p;

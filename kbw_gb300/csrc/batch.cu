@@ -38,6 +38,7 @@
 #include <vector>
 
 #include "../../include/kbwg.h"
+#include "retry.h"
 #include "kernels.h"
 #include "sim.h"
 #include "sweep_dev.cuh"
@@ -615,34 +616,41 @@ static cudaError_t batch_take(int dev, size_t bytes, char **buf, size_t *cap) {
             return cudaSuccess;
         }
     }
-    cudaError_t e = cudaMalloc((void **)buf, bytes);
-    if (e == cudaErrorMemoryAllocation) {  // the kept buffer may be what is missing
-        cudaGetLastError();
-        batch_release_workspace();
-        e = cudaMalloc((void **)buf, bytes);
-    }
     *cap = bytes;
-    return e;
+    return device_malloc((void **)buf, bytes);  // (a kept buffer that is too small may be what is missing)
 }
 
 static void batch_give(int dev, char *buf, size_t cap) {
-    void *drop = buf;
-    int drop_dev = dev;
+    void *drop = buf;  // (the one kept before is on this device too)
     if (cap <= kBatchKeepBytes) {
         std::lock_guard<std::mutex> lk(g_batch_mu);
         if (!g_batch_buf || (g_batch_dev == dev && g_batch_cap < cap)) {
             drop = g_batch_buf;
-            drop_dev = g_batch_dev;
             g_batch_buf = buf;
             g_batch_cap = cap;
             g_batch_dev = dev;
         }
     }
-    (void)drop_dev;  // (the dropped buffer is on this device or null)
     if (drop) cudaFree(drop);
 }
 
-void batch_release_workspace() {
+size_t batch_kept_bytes() {
+    std::lock_guard<std::mutex> lk(g_batch_mu);
+    return g_batch_buf ? g_batch_cap : 0;
+}
+
+cudaError_t device_malloc(void **p, size_t bytes) {
+    return alloc_or_release(
+        cudaErrorMemoryAllocation,
+        [&] {
+            const cudaError_t e = cudaMalloc(p, bytes);
+            if (e != cudaSuccess) cudaGetLastError();
+            return e;
+        },
+        batch_release_workspace);
+}
+
+bool batch_release_workspace() {
     void *buf = nullptr;
     int dev = -1, cur = -1;
     {
@@ -652,11 +660,12 @@ void batch_release_workspace() {
         g_batch_buf = nullptr;
         g_batch_cap = 0;
     }
-    if (!buf) return;
+    if (!buf) return false;
     cudaGetDevice(&cur);
     if (cur != dev) cudaSetDevice(dev);
     cudaFree(buf);
     if (cur != dev && cur >= 0) cudaSetDevice(cur);
+    return true;
 }
 
 template <class P, int K, int R>

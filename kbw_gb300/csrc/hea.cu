@@ -559,7 +559,7 @@ static int32_t hea_run(const std::vector<HeaJob> &jobs, const std::vector<double
                  eb = jobs.size() * sizeof(double), sb = (size_t)grid * slot_elems * sizeof(Mem);
     const size_t off_p = (jb + 255) & ~(size_t)255, off_e = (off_p + pb + 255) & ~(size_t)255,
                  off_c = (off_e + eb + 255) & ~(size_t)255, off_err = off_c + 256, off_s = off_err + 256;
-    e = cudaMalloc(&dbuf, off_s + sb);
+    e = device_malloc((void **)&dbuf, off_s + sb);
     if (e != cudaSuccess) {
         cudaStreamDestroy(st);
         return fail(e, "buffers");

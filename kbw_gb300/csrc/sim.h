@@ -179,8 +179,14 @@ int32_t batch_circuits(int precision, uint32_t flags, size_t ncirc, const uint32
                        const uintptr_t *qubits, const uintptr_t *term_offsets, const double *coefficients,
                        const uintptr_t *ham_offsets, double *energies);
 
-// Free the buffer batch_circuits keeps between calls.
-void batch_release_workspace();
+// Free the buffer batch_circuits keeps between calls; true if there was one.
+bool batch_release_workspace();
+// Its size (0 while a call uses it).
+size_t batch_kept_bytes();
+
+// cudaMalloc of a handle's own memory: where it is short, the buffer kept
+// between batch calls goes first.
+cudaError_t device_malloc(void **p, size_t bytes);
 
 // Adjoint gradient (adjoint.cu).  fwd: the circuit; angles: each gate's
 // angle; gtype: GT_* per gate (GT_NONE if not differentiated).  Writes E and

@@ -347,7 +347,7 @@ static cudaError_t run_fused_p(Sim &s, const GateDesc *gates, size_t count) {
     void *dbuf = nullptr;
     cudaError_t e;
     if (graphs) {
-        e = cudaMalloc(&dbuf, std::max<size_t>(total, 1) * sizeof(TileGate));
+        e = device_malloc(&dbuf, std::max<size_t>(total, 1) * sizeof(TileGate));
         if (e != cudaSuccess) return e;
     } else {
         e = s.tmp4.ensure(total * sizeof(TileGate));

@@ -119,8 +119,7 @@ int32_t autotune(Sim &s, const std::vector<GateDesc> &gates, uint32_t reps, Tune
     }
     const size_t bytes = (size_t)s.ns * s.elem;
     void *saved = nullptr;
-    if (cudaMalloc(&saved, bytes) != cudaSuccess) {
-        cudaGetLastError();
+    if (device_malloc(&saved, bytes) != cudaSuccess) {
         err = "not enough device memory for a copy of the state while tuning";
         return KBWG_ENOMEM;
     }
