@@ -653,6 +653,7 @@ __global__ void k_sum_slots(const double *partials, uint32_t nblocks, uint32_t n
 // kernels of each segment structure seen.
 struct AdjScratch {
     size_t sb = 0;  // state bytes lam/ckpt were made for
+    size_t device_bytes = 0;
     void *lam = nullptr;
     std::vector<void *> ckpt;
     double *partials = nullptr;
@@ -1208,7 +1209,6 @@ static std::vector<ApplyGroup> make_groups(const std::vector<PauliString> &H) {
 }
 
 constexpr size_t kDriftGates = 256;           // most gates uncomputed between two checkpoints
-constexpr size_t kSmallState = 64ull << 20;  // scratch of states up to this size stays with the handle unasked
 
 template <class P, class T, int K, int R>
 static int32_t adjoint_run(Sim &s, const std::vector<GateDesc> &fwd, const std::vector<double> &angles,
@@ -1253,9 +1253,9 @@ static int32_t adjoint_run(Sim &s, const std::vector<GateDesc> &fwd, const std::
     // could give, while every segment boundary costs sweeps: 24 qubits, 720
     // gates, 17 segments 33 + 36 sweeps and 32 copies, 3 segments 10 + 12 and 4.)
     const size_t want = std::min<size_t>(max_ckpt, M ? (M - 1) / kDriftGates : 0);
-    size_t free_b = 0, total_b = 0;
-    if (sc.ckpt.size() < want || sb > kSmallState) {
-        e = cudaMemGetInfo(&free_b, &total_b);
+    size_t free_b = 0;
+    if (sc.ckpt.size() < want || !sc.device_bytes) {
+        e = cudaMemGetInfo(&free_b, &sc.device_bytes);
         if (e != cudaSuccess) return fail_cuda(e, "memory query");
         free_b += batch_kept_bytes();  // (device_malloc gets it back)
     }
@@ -1393,7 +1393,7 @@ static int32_t adjoint_run(Sim &s, const std::vector<GateDesc> &fwd, const std::
     for (size_t j = 0; j < M; j++) grad_per_gate[j] *= gate_mult[j];
     // lambda and the checkpoints stay for the next call while they are small
     // against the device (a sixteenth of its memory); larger ones go now
-    if (sb > kSmallState && sb * (1 + sc.ckpt.size()) > total_b / 16) sc.release_states();
+    if (sb * (1 + sc.ckpt.size()) > sc.device_bytes / 16) sc.release_states();
     return KBWG_OK;
 }
 
