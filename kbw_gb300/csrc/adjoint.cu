@@ -1444,9 +1444,20 @@ size_t jit_check_adjoint(const Sim &s, const std::vector<GateDesc> &fwd, const s
     return check_adjoint_p<Fast<double>, AdjCfg<double>::K, AdjCfg<double>::R>(s, fwd, gtype, sweeps);
 }
 
-int32_t adjoint_gradient(Sim &s, const std::vector<GateDesc> &fwd, const std::vector<double> &angles,
-                         const std::vector<int> &gtype, const std::vector<PauliString> &H, double *energy,
-                         std::vector<double> &grad_per_gate, uint32_t max_ckpt) {
+// A power of two H is divided by for the run: lambda and the deferred factors
+// of the reverse sweeps (up to 2^40 on either state, so 2^80 in a product) stay
+// inside float's range for coefficients that sum up to 2^32; larger ones are
+// scaled to one, exactly, and the results back.
+static int hamiltonian_scale(const std::vector<PauliString> &H) {
+    double sum = 0.0;
+    for (const PauliString &t : H) sum += fabs(t.coef);
+    if (!(sum > 4294967296.0) || !isfinite(sum)) return 0;
+    return ilogb(sum);
+}
+
+static int32_t adjoint_dispatch(Sim &s, const std::vector<GateDesc> &fwd, const std::vector<double> &angles,
+                                const std::vector<int> &gtype, const std::vector<PauliString> &H, double *energy,
+                                std::vector<double> &grad_per_gate, uint32_t max_ckpt) {
     // (above 32 qubits the reverse sweeps read gate bits of a 64-bit tile
     // base; memory decides how far: the state, lambda and the checkpoints)
     if (s.n < (uint32_t)AdjCfg<float>::K || (s.prec && s.n < (uint32_t)AdjCfg<double>::K)) {
@@ -1464,6 +1475,20 @@ int32_t adjoint_gradient(Sim &s, const std::vector<GateDesc> &fwd, const std::ve
                                                                              grad_per_gate, max_ckpt);
     return adjoint_run<Fast<double>, double, AdjCfg<double>::K, AdjCfg<double>::R>(s, fwd, angles, gtype, H, energy,
                                                                                 grad_per_gate, max_ckpt);
+}
+
+int32_t adjoint_gradient(Sim &s, const std::vector<GateDesc> &fwd, const std::vector<double> &angles,
+                         const std::vector<int> &gtype, const std::vector<PauliString> &H, double *energy,
+                         std::vector<double> &grad_per_gate, uint32_t max_ckpt) {
+    const int scale = hamiltonian_scale(H);
+    if (!scale) return adjoint_dispatch(s, fwd, angles, gtype, H, energy, grad_per_gate, max_ckpt);
+    std::vector<PauliString> h = H;
+    for (PauliString &t : h) t.coef = ldexp(t.coef, -scale);
+    const int32_t rc = adjoint_dispatch(s, fwd, angles, gtype, h, energy, grad_per_gate, max_ckpt);
+    if (rc != KBWG_OK) return rc;
+    *energy = ldexp(*energy, scale);
+    for (double &g : grad_per_gate) g = ldexp(g, scale);
+    return KBWG_OK;
 }
 
 }  // namespace kbwg
