@@ -400,6 +400,7 @@ int32_t kbwg_measure_collapse(kbwg_sim *s, uintptr_t target, bool result, double
     if (target >= s->n) return fail(KBWG_EINVAL, "target qubit out of range");
     CUDA_TRY(flush_queue(*s));  // (a float-float resident state is collapsed as is)
     const uint64_t bit = 1ull << target;
+    s->norm_bound *= std::max(1.0, fabs(p));
     if (s->ff_resident) {
         CUDA_TRY(launch_collapse_ff(s->state, s->n, nullptr, bit, result ? bit : 0ull, p, s->stream));
     } else {
@@ -970,6 +971,7 @@ int32_t kbwg_set_state(kbwg_sim *s, const void *host_src, uintptr_t bytes) {
     if (!host_src || bytes != s->ns * s->elem) return fail(KBWG_EINVAL, "buffer size must equal 2^n * element size");
     s->queue.clear();
     s->ff_resident = false;
+    s->norm_bound = HUGE_VAL;
     CUDA_TRY(copy_async(s->state, host_src, bytes, cudaMemcpyHostToDevice, s->stream));
     CUDA_TRY(cudaStreamSynchronize(s->stream));
     return KBWG_OK;
@@ -984,7 +986,10 @@ int32_t kbwg_state_info(kbwg_sim *s, uintptr_t *num_qubits, int32_t *precision, 
     CUDA_TRY(cudaStreamSynchronize(s->stream));
     if (num_qubits) *num_qubits = s->n;
     if (precision) *precision = s->prec;
-    if (device_ptr) *device_ptr = s->state;
+    if (device_ptr) {
+        *device_ptr = s->state;
+        s->norm_bound = HUGE_VAL;  // (the caller may write through it)
+    }
     if (bytes) *bytes = s->ns * s->elem;
     return KBWG_OK;
     GUARD_END

@@ -63,6 +63,9 @@ struct Sim {
     // complex128 fast path: the buffer holds float-float pairs (hi, lo of the
     // real part, then of the imaginary part) instead of binary64 while true
     bool ff_resident = false;
+    // at most the state's norm as far as it is known: one from |0...0> on,
+    // infinite for amplitudes the caller wrote (see within_range in sweep.cu)
+    double norm_bound = 1.0;
 
     std::vector<GateDesc> queue;  // gates waiting for the next flush
 

@@ -629,8 +629,10 @@ static cudaError_t run_fused_t(Sim &s, const GateDesc *gates, size_t count) {
 // factor is that of the coefficient as rounded to the program's type, so
 // each gate with its share of g is a rotation to binary64 accuracy.
 constexpr int kDeferRun = 192, kDeferMin = 3;
+constexpr int kDeferRunH = 100;  // of float-float's H alone (states of any norm float can hold, see within_range)
 
 static std::vector<GateDesc> defer_scale(int arith, const GateDesc *gates, size_t count, bool rotations) {
+    const int run = rotations ? kDeferRun : kDeferRunH;
     std::vector<GateDesc> out;
     out.reserve(count + 2);
     size_t rots = 0, any = 0;
@@ -694,7 +696,7 @@ static std::vector<GateDesc> defer_scale(int arith, const GateDesc *gates, size_
         }
         out.push_back(x);
         pending = pending || grew;
-        if (grew && ++unscaled >= kDeferRun) emit_scale();
+        if (grew && ++unscaled >= run) emit_scale();
     }
     if (pending) emit_scale();
     return out;
@@ -712,10 +714,43 @@ std::vector<GateDesc> defer_factors(int arith, const GateDesc *gates, size_t cou
     return defer_scale(arith, f.data(), f.size(), true);
 }
 
+// Whether the state's norm leaves room for a run of deferred factors (2^96) in
+// float's range: below kNormRoom, as after |0...0> or a loaded state of unit
+// norm.  Where it is not known (amplitudes written by the caller, collapses
+// with factors of the caller's) it is measured, once, before the gates run.
+constexpr double kNormRoom = 1048576.0;
+
+static cudaError_t within_range(Sim &s, bool &ok) {
+    ok = true;
+    if (s.norm_bound <= kNormRoom || (s.flags & (KBWG_FLAG_EXACT_ORDER | KBWG_FLAG_NO_FOLD))) return cudaSuccess;
+    if (s.prec && !ff_capable(s)) return cudaSuccess;  // (binary64 sweeps)
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    cudaError_t e = cudaStreamIsCapturing(s.stream, &capture);
+    if (e != cudaSuccess || capture != cudaStreamCaptureStatusNone) {  // (nothing can be read back now)
+        ok = false;
+        return e;
+    }
+    if (s.ff_resident) e = launch_masked_norm_ff(s.state, s.n, 0, 0, s.rs, s.stream);
+    else if (s.prec) e = launch_masked_norm<double>(s.state, s.n, 0, 0, s.rs, s.stream);
+    else e = launch_masked_norm<float>(s.state, s.n, 0, 0, s.rs, s.stream);
+    if (e == cudaSuccess) e = copy_async(s.h_result, s.rs.result, sizeof(double), cudaMemcpyDeviceToHost, s.stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s.stream);
+    if (e != cudaSuccess) return e;
+    const double norm = sqrt(s.h_result[0]);
+    s.norm_bound = norm <= kNormRoom ? std::max(1.0, norm) : HUGE_VAL;  // (also for a NaN)
+    ok = s.norm_bound <= kNormRoom;
+    return cudaSuccess;
+}
+
 // The gate list as the fused sweeps of a handle run it (folded, factors
-// deferred); the handle's state is at least one tile.
-static std::vector<GateDesc> rewritten(const Sim &s, const GateDesc *gates, size_t count) {
+// deferred where the state's norm allows); the handle's state is at least one
+// tile.
+static std::vector<GateDesc> rewritten(const Sim &s, const GateDesc *gates, size_t count, bool in_range) {
     if (s.flags & KBWG_FLAG_EXACT_ORDER) return std::vector<GateDesc>(gates, gates + count);
+    if (!in_range) {
+        const std::vector<GateDesc> f = fold_diagonals(gates, count);
+        return ff_capable(s) ? defer_scale(ARITH_FF, f.data(), f.size(), false) : f;
+    }
     if (s.flags & KBWG_FLAG_NO_FOLD) {  // every gate applied as given, but for float-float's H and RZ
         if (ff_capable(s)) return defer_scale(ARITH_FF, gates, count, false);
         return std::vector<GateDesc>(gates, gates + count);
@@ -789,6 +824,7 @@ cudaError_t ensure_binary64(Sim &s) {
 }
 
 cudaError_t init_state(Sim &s) {
+    s.norm_bound = 1.0;
     if (ff_capable(s)) {
         s.ff_resident = true;
         return launch_init_ff(s.state, s.n, s.stream);
@@ -833,7 +869,7 @@ static size_t check_t(const Sim &s, const GateDesc *gates, size_t count, size_t 
 }
 
 size_t jit_check(const Sim &s, const GateDesc *gates, size_t count, size_t &sweeps) {
-    const std::vector<GateDesc> g = rewritten(s, gates, count);
+    const std::vector<GateDesc> g = rewritten(s, gates, count, true);
     if (ff_capable(s)) {
         if (chosen_tile(s) == 12) return check_p<FF2, 12, 4>(s, g.data(), g.size(), sweeps);
         return check_p<FF2, TileCfgFF::K, TileCfgFF::R>(s, g.data(), g.size(), sweeps);
@@ -851,7 +887,10 @@ cudaError_t run_fused(Sim &s, const GateDesc *gates, size_t count) {
         }
         return s.prec ? run_fused_t<double>(s, gates, count) : run_fused_t<float>(s, gates, count);
     }
-    const std::vector<GateDesc> g = rewritten(s, gates, count);
+    bool in_range = true;
+    const cudaError_t er = within_range(s, in_range);
+    if (er != cudaSuccess) return er;
+    const std::vector<GateDesc> g = rewritten(s, gates, count, in_range);
     if (ff_capable(s)) {
         // float-float sweeps read and write the float-float form; the state
         // stays in it until an operation needs binary64
