@@ -175,8 +175,9 @@ int32_t kbwg_exp_value(kbwg_sim *sim, const uint8_t *paulis, const uintptr_t *qu
  * param_index[i] in [0, n_params) marks gate i (P/RX/RY/RZ only) as depending
  * on parameter param_index[i] (shared parameters add up); -1 = constant.  The
  * Hamiltonian is given as in kbwg_exp_value.  Up to max_checkpoints copies of
- * the forward state (one per 256 gates, as memory allows) bound the uncompute
- * drift.  Writes E
+ * the forward state (as memory allows) bound the uncompute drift: one per 256
+ * gates, or for max_checkpoints > 16 as many as asked for, evenly spaced and
+ * at most one per gate.  Writes E
  * and gradient[n_params]; the handle is left in |0...0>.  Needs >= 12 qubits
  * (complex64) or >= 11 (complex128).  The call's scratch (lambda and the
  * checkpoints) stays with the handle for the next call while it takes at most
