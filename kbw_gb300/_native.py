@@ -162,8 +162,9 @@ def _packer():
     global _pack, _pack_tried
     if not _pack_tried:
         _pack_tried = True
-        path = os.path.join(os.path.dirname(LIB_PATH), "_kbwgpack.so")
-        if os.path.exists(path):
+        from .build import PACK_NAME
+        path = os.path.join(os.path.dirname(LIB_PATH), PACK_NAME or "")
+        if PACK_NAME and os.path.exists(path):
             try:
                 lib = ctypes.PyDLL(path)  # the functions walk Python objects: the interpreter lock stays held
             except OSError:

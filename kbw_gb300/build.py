@@ -70,7 +70,11 @@ def write_jit_sources():
 
 
 PACK_SRC = os.path.join(HERE, "native", "pack.c")
-PACK_LIB = os.path.join(HERE, "_kbwgpack.so")
+# The packers' file carries the interpreter's ABI tag (their macros read object
+# layouts); an interpreter without a global lock has none.
+PACK_NAME = None
+if sysconfig.get_config_var("EXT_SUFFIX") and not sysconfig.get_config_var("Py_GIL_DISABLED"):
+    PACK_NAME = "_kbwgpack" + sysconfig.get_config_var("EXT_SUFFIX")
 
 
 def build_pack():
@@ -78,17 +82,18 @@ def build_pack():
     headers or a C compiler are missing the binding packs in Python."""
     inc = sysconfig.get_paths()["include"]
     cc = shutil.which("gcc") or shutil.which("cc")
-    if cc is None or not os.path.exists(os.path.join(inc, "Python.h")):
+    if cc is None or PACK_NAME is None or not os.path.exists(os.path.join(inc, "Python.h")):
         return None
-    if os.path.exists(PACK_LIB) and os.path.getmtime(PACK_LIB) >= os.path.getmtime(PACK_SRC):
-        return PACK_LIB
-    tmp = PACK_LIB + ".tmp%d" % os.getpid()
+    lib = os.path.join(HERE, PACK_NAME)
+    if os.path.exists(lib) and os.path.getmtime(lib) >= os.path.getmtime(PACK_SRC):
+        return lib
+    tmp = lib + ".tmp%d" % os.getpid()
     r = subprocess.run([cc, "-std=c11", "-O2", "-fPIC", "-shared", "-I", inc, PACK_SRC, "-o", tmp],
                        capture_output=True, text=True)
     if r.returncode != 0:
         raise RuntimeError("building %s failed:\n%s" % (PACK_SRC, r.stderr))
-    os.replace(tmp, PACK_LIB)
-    return PACK_LIB
+    os.replace(tmp, lib)
+    return lib
 
 
 def _compile(src, verbose):
