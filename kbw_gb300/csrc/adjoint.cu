@@ -406,16 +406,38 @@ __global__ void __launch_bounds__(256, 3) k_apply_tile_f32(const cx<float> *__re
     }
 }
 
-// Share of Re<a|b> of one amplitude pair: float-float (exact products of the
-// complex64 parts), or added in binary64 for binary64 states.
-__device__ __forceinline__ ff::f2 re_product(const ff2::v2 &x, const ff2::v2 &y) {
-    return ff::dot2(ff::f2{x.h.x, x.l.x}, ff::f2{y.h.x, y.l.x}, ff::f2{x.h.y, x.l.y}, ff::f2{y.h.y, y.l.y});
-}
-__device__ __forceinline__ ff::f2 re_product(const cx<float> &x, const cx<float> &y) {
-    const float p = __fmul_rn(x.re, y.re), q = __fmul_rn(x.im, y.im);
-    const ff::f2 t = ff::two_sum(p, q);
-    return ff::fast_two_sum(t.h, ff::add(t.l, ff::add(__fmaf_rn(x.re, y.re, -p), __fmaf_rn(x.im, y.im, -q))));
-}
+// A thread's share of Re<a|b>.  Binary64 states: in binary64.  Float-float
+// states: float-float.  complex64 states: the products are exact in two floats,
+// and their sum keeps every rounding error in a third (parts apart, packed), so
+// it is no less exact than in binary64.
+template <class Mem>
+struct ReSum {
+    double acc = 0.0;
+    __device__ __forceinline__ void add(const Mem &x, const Mem &y) { acc = fma(x.re, y.re, fma(x.im, y.im, acc)); }
+    __device__ __forceinline__ double value() const { return acc; }
+};
+template <>
+struct ReSum<ff2::v2> {
+    ff::f2 t{0.f, 0.f};
+    __device__ __forceinline__ void add(const ff2::v2 &x, const ff2::v2 &y) {
+        t = ff::add(t, ff::dot2(ff::f2{x.h.x, x.l.x}, ff::f2{y.h.x, y.l.x}, ff::f2{x.h.y, x.l.y}, ff::f2{y.h.y, y.l.y}));
+    }
+    __device__ __forceinline__ double value() const { return (double)t.h + (double)t.l; }
+};
+template <>
+struct ReSum<cx<float>> {
+    float2 h = make_float2(0.f, 0.f), m = h, l = h;
+    __device__ __forceinline__ void add(const cx<float> &x, const cx<float> &y) {
+        const float2 a = make_float2(x.re, x.im), b = make_float2(y.re, y.im), p = ff2::mul(a, b);
+        const ff2::v2 t = ff2::two_sum(h, p), u = ff2::two_sum(m, ff2::fma(a, b, ff2::neg(p))), v = ff2::two_sum(u.h, t.l);
+        h = t.h;
+        m = v.h;
+        l = ff2::add(l, ff2::add(u.l, v.l));
+    }
+    __device__ __forceinline__ double value() const {
+        return ((double)h.x + (double)h.y) + (((double)m.x + (double)m.y) + ((double)l.x + (double)l.y));
+    }
+};
 
 // Re<a|b> (FP64-grade) into result[0].  Four pairs in flight per thread; the
 // last block adds the partials with all its threads (one thread read 608 of
@@ -424,11 +446,9 @@ __device__ __forceinline__ ff::f2 re_product(const cx<float> &x, const cx<float>
 template <class Mem>
 __global__ void __launch_bounds__(256) k_inner_re(const Mem *__restrict__ a, const Mem *__restrict__ b, uint64_t ns,
                                                   double *partials, unsigned *ticket, double *result) {
-    constexpr bool kWide = std::is_same<Mem, cx<double>>::value;
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
     uint64_t s = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    double acc = 0.0;
-    ff::f2 t0{0.f, 0.f}, t1{0.f, 0.f};
+    ReSum<Mem> t0, t1;
     for (; s + 3 * stride < ns; s += 4 * stride) {
         Mem x[4], y[4];
 #pragma unroll
@@ -436,23 +456,12 @@ __global__ void __launch_bounds__(256) k_inner_re(const Mem *__restrict__ a, con
             x[u] = a[s + u * stride];
             y[u] = b[s + u * stride];
         }
-        if constexpr (kWide) {
-#pragma unroll
-            for (int u = 0; u < 4; u++) acc = fma(x[u].re, y[u].re, fma(x[u].im, y[u].im, acc));
-        } else {
-            t0 = ff::add(t0, ff::add(re_product(x[0], y[0]), re_product(x[1], y[1])));
-            t1 = ff::add(t1, ff::add(re_product(x[2], y[2]), re_product(x[3], y[3])));
-        }
+        t0.add(x[0], y[0]);
+        t1.add(x[1], y[1]);
+        t0.add(x[2], y[2]);
+        t1.add(x[3], y[3]);
     }
-    for (; s < ns; s += stride) {
-        const Mem x = a[s], y = b[s];
-        if constexpr (kWide) acc = fma(x.re, y.re, fma(x.im, y.im, acc));
-        else t0 = ff::add(t0, re_product(x, y));
-    }
-    if constexpr (!kWide) {
-        t0 = ff::add(t0, t1);
-        acc = (double)t0.h + (double)t0.l;
-    }
+    for (; s < ns; s += stride) t0.add(a[s], b[s]);
     __shared__ double sh[8];
     __shared__ bool is_last;
     auto block_total = [&](double v) {  // valid in thread 0
@@ -465,7 +474,7 @@ __global__ void __launch_bounds__(256) k_inner_re(const Mem *__restrict__ a, con
             for (int w = 0; w < (int)(blockDim.x >> 5); w++) t += sh[w];
         return t;
     };
-    const double mine = block_total(acc);
+    const double mine = block_total(t0.value() + t1.value());
     if (threadIdx.x == 0) {
         partials[blockIdx.x] = mine;
         __threadfence();

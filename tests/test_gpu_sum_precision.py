@@ -109,3 +109,17 @@ def test_samples_far_from_unit_norm(arith, size):
     sim.set_state(a)
     sim.apply([(C.X, 0, (), 0.0)])
     assert [_pick(sim, n, d) for d in (0.1, 0.35, 0.37, 0.9)] == [4, 4, 4001, 4001]
+
+
+def test_energy_of_a_gradient_of_two_amplitudes():
+    """lambda = Z psi is exact, and psi one rotation's two amplitudes: squares
+    (exact in binary64), their sum, and the zeros around it."""
+    n, rng = 12, np.random.default_rng(8)
+    sim = DenseGB300(n, "c64")
+    for _ in range(50):
+        gates = [(C.RY, 0, (), float(rng.uniform(0.5, 1.0)))]
+        sim.clear()
+        sim.apply(gates)
+        a = np.longdouble(sim.state().real)
+        e, _ = sim.adjoint_gradient(gates, [0], 1, [(1.0, [(Z, 0)])])
+        assert abs(e - (a[0] ** 2 - a[1] ** 2)) <= 3 * U * (a[0] ** 2 + a[1] ** 2)
