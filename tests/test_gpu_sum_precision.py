@@ -112,14 +112,15 @@ def test_samples_far_from_unit_norm(arith, size):
 
 
 def test_energy_of_a_gradient_of_two_amplitudes():
-    """lambda = Z psi is exact, and psi one rotation's two amplitudes: squares
-    (exact in binary64), their sum, and the zeros around it."""
+    """lambda = Z psi is exact, and psi two complex amplitudes: their squares
+    (exact in binary64), the sum of each pair, and the difference."""
     n, rng = 12, np.random.default_rng(8)
     sim = DenseGB300(n, "c64")
     for _ in range(50):
-        gates = [(C.RY, 0, (), float(rng.uniform(0.5, 1.0)))]
+        gates = [(C.RY, 0, (), float(rng.uniform(0.5, 1.0))), (C.RZ, 0, (), float(rng.uniform(0.5, 1.0)))]
         sim.clear()
         sim.apply(gates)
-        a = np.longdouble(sim.state().real)
-        e, _ = sim.adjoint_gradient(gates, [0], 1, [(1.0, [(Z, 0)])])
-        assert abs(e - (a[0] ** 2 - a[1] ** 2)) <= 3 * U * (a[0] ** 2 + a[1] ** 2)
+        a = sim.state()
+        w = np.longdouble(a.real) ** 2 + np.longdouble(a.imag) ** 2
+        e, _ = sim.adjoint_gradient(gates, [0, 1], 2, [(1.0, [(Z, 0)])])
+        assert abs(e - (w[0] - w[1])) <= 3 * U * (w[0] + w[1])
