@@ -381,10 +381,12 @@ int32_t kbwg_wait_probe(kbwg_sim *sim, uint32_t spins);
  * kbwg_new creates (kbwg_new fails with KBWG_EINVAL on a value no kernel
  * exists for); a tile size larger than a handle's qubit count falls back to
  * the default on that handle.  The default tile is the arithmetic's
- * (complex64 13, complex128 12, float-float 11 qubits); on registers of 13 to
- * 19 qubits, which leave SMs without such a tile, 11; 12 for complex64 at 20,
- * 22, 24 and 25 qubits; for a register smaller than that the largest compiled
- * size that fits it.  They apply wherever gates are applied to a
+ * (complex64 13, complex128 12, float-float 11 qubits); on registers up to 19
+ * qubits that hold such a tile (complex64 from 13, complex128 from 12 on), which
+ * leave SMs without one, 11; 12 for complex64 at 20, 22, 24 and 25 qubits (25:
+ * gate lists of mostly controlled gates on handles with KBWG_JIT_OFF run on
+ * 13); for a register smaller than that the largest compiled size that fits
+ * it.  They apply wherever gates are applied to a
  * handle's state (gate calls, the forward pass of kbwg_adjoint_gradient, the
  * circuit runs of kbwg_param_shift_gradient), not to the adjoint's reverse
  * sweeps or to the batch and reduction kernels. */

@@ -65,7 +65,8 @@ struct SweepKernel {
 
 // W: 64-bit state indices (registers above 32 qubits); the 32-bit form keeps
 // registers free for the amplitudes.
-template <class P, int K, int R, bool W>
+// ROT: the program may hold rotations with deferred factors or merged signs.
+template <class P, int K, int R, bool W, bool ROT>
 __global__ void __launch_bounds__(SweepKernel<P, K, R>::kThreads, SweepKernel<P, K, R>::kCtasPerSm)
     k_sweep(typename P::Mem *__restrict__ st, const __grid_constant__ SweepParams p) {
     using Amp = typename P::Amp;
@@ -143,7 +144,7 @@ __global__ void __launch_bounds__(SweepKernel<P, K, R>::kThreads, SweepKernel<P,
                 for (int j = 0; j < NR; j++) v[j] = tile[F | ((uint32_t)j << R0)];
             }
             const uint32_t g1 = p.stage_end[s];
-            for (uint32_t gi = g0; gi < g1; gi++) tile_gate<P, K, R, B>(sg[gi], v, R0, F, base);
+            for (uint32_t gi = g0; gi < g1; gi++) tile_gate<P, K, R, B, ROT>(sg[gi], v, R0, F, base);
             g0 = g1;
         }
         // the tile buffer is free: start the next tile's load, then store this one
@@ -251,9 +252,6 @@ static std::vector<uint64_t> structure_of(const GateDesc *gates, size_t count) {
     return sig;
 }
 
-// Z and CZ gates are merged unless every gate is to run as given.
-static bool merges(const Sim &s) { return !(s.flags & (KBWG_FLAG_EXACT_ORDER | KBWG_FLAG_NO_FOLD)); }
-
 // Pack the planned program with the constants of `gates` and upload it.
 template <class P>
 static cudaError_t upload_program(Sim &s, const std::vector<TileGate> &planned, const std::vector<uint32_t> &src,
@@ -268,17 +266,34 @@ static cudaError_t upload_program(Sim &s, const std::vector<TileGate> &planned, 
     return copy_async(dst, prog.data(), prog.size() * sizeof(TileGate), cudaMemcpyHostToDevice, s.stream);
 }
 
+// Policy of the kernel that runs a complex64 or float-float sweep without
+// deferred factors and merged signs.
+template <class P> struct PlainPolicy { using type = void; };
+template <> struct PlainPolicy<FastP> { using type = FastPPlain; };
+template <> struct PlainPolicy<FF2> { using type = FF2; };
+template <class P>
+static bool runs_plain(const PlannedSweep &sw) {
+    for (const TileGate &t : sw.gates)
+        if (t.cls == TG_SIGN || (t.sub == 1 && (t.cls == TG_RX || t.cls == TG_RY || !PlainPolicy<P>::type::kSub)))
+            return false;
+    return true;
+}
+
 template <class P, int K, int R, bool W = false>
-static cudaError_t run_fused_p(Sim &s, const GateDesc *gates, size_t count) {
+static cudaError_t run_fused_p(Sim &s, const GateDesc *gates, size_t count, bool merge) {
     using SK = SweepKernel<P, K, R>;
     using Mem = typename P::Mem;
+    using Plain = typename PlainPolicy<P>::type;
+    constexpr bool kPlain = !std::is_same<Plain, void>::value;
     int num_sms = 0;
     {
-        cudaError_t e = ensure_smem_limit((const void *)k_sweep<P, K, R, W>, SK::kSmem);
+        cudaError_t e = ensure_smem_limit((const void *)k_sweep<P, K, R, W, P::kDefer>, SK::kSmem);
+        if constexpr (kPlain)
+            if (e == cudaSuccess) e = ensure_smem_limit((const void *)k_sweep<Plain, K, R, W, false>, SK::kSmem);
         if (e == cudaSuccess) e = current_sm_count(num_sms);
         if (e != cudaSuccess) return e;
     }
-    const void *kid = (const void *)k_sweep<P, K, R, W>;
+    const void *kid = (const void *)k_sweep<P, K, R, W, P::kDefer>;
     const size_t depth = s.fusion_depth ? s.fusion_depth : (size_t)kMaxSweepGates;
     // timed profiling marks every launch with events, which a graph replay cannot
     const bool graphs_ok = !s.prof.on && !(s.flags & KBWG_FLAG_NO_GRAPHS);
@@ -295,6 +310,7 @@ static cudaError_t run_fused_p(Sim &s, const GateDesc *gates, size_t count) {
         if (!s.graphs) s.graphs = new GraphCache();
         GraphCache &gc = *(GraphCache *)s.graphs;
         sig = structure_of(gates, count);
+        sig.push_back(merge);
         sig.push_back((uint64_t)(uintptr_t)kid);
         sig.push_back(depth);
         h = hash_of(sig);
@@ -336,7 +352,7 @@ static cudaError_t run_fused_p(Sim &s, const GateDesc *gates, size_t count) {
     size_t placed = 0;
     for (PlannedSweep &sw : plan) {
         placed += sw.gates.size();
-        if (merges(s)) merge_signs(sw, K, R);
+        if (merge) merge_signs(sw, K, R);
         planned.insert(planned.end(), sw.gates.begin(), sw.gates.end());
         planned.insert(planned.end(), sw.data.begin(), sw.data.end());
         src.insert(src.end(), sw.src.begin(), sw.src.end());
@@ -430,7 +446,10 @@ static cudaError_t run_fused_p(Sim &s, const GateDesc *gates, size_t count) {
             cudaLaunchKernel(spec, dim3((unsigned)grid), dim3(SK::kThreads), args, SK::kSmem, s.stream);
             specialised++;
         } else {
-            k_sweep<P, K, R, W><<<(unsigned)grid, SK::kThreads, SK::kSmem, s.stream>>>((Mem *)s.state, p);
+            auto kern = k_sweep<P, K, R, W, P::kDefer>;
+            if constexpr (kPlain)
+                if (runs_plain<P>(sw)) kern = k_sweep<Plain, K, R, W, false>;
+            kern<<<(unsigned)grid, SK::kThreads, SK::kSmem, s.stream>>>((Mem *)s.state, p);
         }
         if (!graphs) count_launch();
         e = cudaGetLastError();
@@ -510,23 +529,31 @@ uint32_t tile_register_bits(const Sim &s, uint32_t k) {
     return k == 11 ? 3u : 4u;  // the 2^11 tiles hold 8 amplitudes per thread, the larger ones 16
 }
 
-// Default tile by register size.  Below ~152 tiles of the largest geometry the
-// chip has idle SMs, and a smaller tile spreads a gate over more of them at
-// the price of a few more sweeps; complex64's 2^12 tiles run three CTAs of 256
-// threads per SM on 80 registers, the 2^13 ones two of 512 on 64, and stay
-// ahead where they need hardly more sweeps.  At 21 and 23 qubits their last
-// wave of CTAs is nearly empty, or a random circuit takes a sweep more, and
-// from 26 on every sweep more costs a pass over HBM.  Measured (us per flush,
-// one GB300; HEA / brickwork, interpreted unless stated):
-//   complex64  n = 16: K 13 108/121, 12 88/100, 11 87/94;  n = 19: 128/145,
-//   105/118, 110/119;  n = 20: 131/152, 124/146, 173/188;  n = 21: 175/219,
-//   205/251;  n = 22: 318/412, 300/361 (specialised 191/220, 177/172);  n =
-//   24: 1136/1452, 1095/1455 (662/738, 612/683);  n = 26: 4357/5690, 4541/5895
-//   (2388/2725, 2446/2666)
+// Default tile by register size: a table of what measured faster on one GB300
+// (152 SMs), not a model.  Below ~152 tiles of the largest geometry the chip
+// has idle SMs, and a smaller tile spreads a gate over more of them at the price
+// of a few more sweeps; complex64's 2^12 tiles run three CTAs of 256 threads per
+// SM on 80 registers, the 2^13 ones two of 512 on 64.  Measured (us, clear,
+// apply and flush; HEA of 6 layers / brickwork of 8):
+//   complex64, tiles of 2^13, 2^12, 2^11
+//     n    interpreted                          specialised
+//     16   108/121    88/100    87/94           (HEA of 4 layers)
+//     19   128/145   105/118   110/119
+//     20   181/153   174/147   244/187          116/97    117/93    133/102
+//     21   251/223   290/247   357/281          170/138   180/138   184/140
+//     22   449/410   431/353   614/510          269/224   255/180   280/236
+//     23   731/669   788/671  1203/970          422/352   447/321   520/417
+//     24  1551/1431 1598/1406 2446/1941         882/742   909/684  1037/824
+//     25  3165/2933 3229/2853 5030/3984        1793/1428 1750/1252 2018/1593
+//     26  6252/5601 6537/5665 10377/8109       3401/2726 3415/2679 4123/3330
+//     28  27.2/25.1 28.2/24.6 44.5/36.4 ms     15.0/12.0 14.9/11.0 18.2/15.3 ms
+//   2^12 where both kernels gain or the specialised one gains more than the
+//   interpreted one loses, up to 25 qubits (from 26 on a first flush loses most);
 //   binary64   n = 14: K 12 485/327, 11 278/201;  n = 19: 623/429, 620/401;
 //   specialised (from 20 qubits) K 12 is 3-5 % faster (n = 25: 46.5 against
 //   48.4 ms, HEA 6 layers)
-//   float-float: K 11 is the faster one up to 24 qubits.
+//   float-float: K 11 is the faster one interpreted at every size (27 qubits
+//   30 %), specialised K 12 from 27 qubits on (3-8 %).
 uint32_t default_tile_k(const Sim &s) {
     const std::vector<uint32_t> ks = compiled_tiles(s);
     if (ks.size() > 1 && ks[0] <= s.n) {
@@ -566,21 +593,31 @@ uint32_t effective_tile_k(const Sim &s) {
     return k <= s.n ? k : 0;
 }
 
+// Complex64 lists of 25 qubits with few gates to defer (`merge` unset: see
+// keeps_full_forms) run on 2^13 tiles where they stay interpreted: they need
+// the most sweeps more on the default 2^12 ones (200 controlled gates, 11
+// against 8: 2.53 against 2.31 ms; 24 qubits, 10 against 8: 1.18 and 1.19).
+static uint32_t tile_of_list(const Sim &s, bool merge) {
+    const uint32_t k = chosen_tile(s);
+    const bool exact = (s.flags & (KBWG_FLAG_EXACT_ORDER | KBWG_FLAG_NO_FOLD)) != 0;
+    return !s.prec && !exact && !merge && s.n == 25 && !s.tile_k ? (uint32_t)TileCfg<float>::K : k;
+}
+
 template <class T>
-static cudaError_t run_fused_t(Sim &s, const GateDesc *gates, size_t count) {
+static cudaError_t run_fused_t(Sim &s, const GateDesc *gates, size_t count, bool merge) {
     constexpr int K = TileCfg<T>::K, R = TileCfg<T>::R;
     if (s.n > 32) {  // 64-bit state indices, default geometry
-        if (s.flags & KBWG_FLAG_EXACT_ORDER) return run_fused_p<Exact<T>, K, R, true>(s, gates, count);
-        if constexpr (std::is_same<T, float>::value) return run_fused_p<FastP, K, R, true>(s, gates, count);
-        else return run_fused_p<Fast<T>, K, R, true>(s, gates, count);
+        if (s.flags & KBWG_FLAG_EXACT_ORDER) return run_fused_p<Exact<T>, K, R, true>(s, gates, count, merge);
+        if constexpr (std::is_same<T, float>::value) return run_fused_p<FastP, K, R, true>(s, gates, count, merge);
+        else return run_fused_p<Fast<T>, K, R, true>(s, gates, count, merge);
     }
-    const uint32_t tk = chosen_tile(s);
+    const uint32_t tk = tile_of_list(s, merge);
     if (tk != (uint32_t)K && !(s.flags & KBWG_FLAG_EXACT_ORDER)) {
         if constexpr (std::is_same<T, float>::value) {
-            if (tk == 12) return run_fused_p<FastP, 12, 4>(s, gates, count);
-            if (tk == 11) return run_fused_p<FastP, 11, 3>(s, gates, count);
+            if (tk == 12) return run_fused_p<FastP, 12, 4>(s, gates, count, merge);
+            if (tk == 11) return run_fused_p<FastP, 11, 3>(s, gates, count, merge);
         } else {
-            if (tk == 11) return run_fused_p<Fast<T>, 11, 3>(s, gates, count);
+            if (tk == 11) return run_fused_p<Fast<T>, 11, 3>(s, gates, count, merge);
         }
     }
     if (s.n < (uint32_t)K) {
@@ -596,9 +633,9 @@ static cudaError_t run_fused_t(Sim &s, const GateDesc *gates, size_t count) {
         s.last_passes = count;
         return cudaSuccess;
     }
-    if (s.flags & KBWG_FLAG_EXACT_ORDER) return run_fused_p<Exact<T>, K, R>(s, gates, count);
-    if constexpr (std::is_same<T, float>::value) return run_fused_p<FastP, K, R>(s, gates, count);
-    else return run_fused_p<Fast<T>, K, R>(s, gates, count);
+    if (s.flags & KBWG_FLAG_EXACT_ORDER) return run_fused_p<Exact<T>, K, R>(s, gates, count, merge);
+    if constexpr (std::is_same<T, float>::value) return run_fused_p<FastP, K, R>(s, gates, count, merge);
+    else return run_fused_p<Fast<T>, K, R>(s, gates, count, merge);
 }
 
 // Rewrite of the queue before planning, in every arithmetic that need not keep
@@ -702,15 +739,20 @@ static std::vector<GateDesc> defer_scale(int arith, const GateDesc *gates, size_
     return out;
 }
 
-std::vector<GateDesc> defer_factors(int arith, const GateDesc *gates, size_t count) {
+// Diagonal runs folded, complex64's constants in binary64 from the angles.
+static std::vector<GateDesc> folded(int arith, const GateDesc *gates, size_t count) {
     std::vector<GateDesc> r;
-    if (arith == ARITH_C64) {  // constants in binary64 from the angles
+    if (arith == ARITH_C64) {
         r.assign(gates, gates + count);
         for (GateDesc &x : r)
             if (x.kind <= G_RZ) x = make_gate_desc(1, x.kind, x.target, x.ctrl, x.angle);
         gates = r.data();
     }
-    const std::vector<GateDesc> f = fold_diagonals(gates, count);
+    return fold_diagonals(gates, count);
+}
+
+std::vector<GateDesc> defer_factors(int arith, const GateDesc *gates, size_t count) {
+    const std::vector<GateDesc> f = folded(arith, gates, count);
     return defer_scale(arith, f.data(), f.size(), true);
 }
 
@@ -742,20 +784,42 @@ static cudaError_t within_range(Sim &s, bool &ok) {
     return cudaSuccess;
 }
 
+// Large complex64 and float-float lists with few gates to defer keep the full
+// forms (and their Z and CZ gates apart): the bodies of the deferred rotations
+// and merged signs cost an interpreted sweep more than a sixth of its gates
+// gives back, and the complex64 specialised ones too.  300 random gates, up to
+// two controls, us, full forms / deferred: complex64 26 qubits 5946 / 6099
+// (specialised 4179 / 4195), 28 qubits 25417 / 26136 (18369 / 18812), 25 qubits
+// 3264 / 3281 (2023 / 1992); float-float 25 qubits 10220 / 10414 (6871 / 6682),
+// 26 qubits 19633 / 20241 (13266 / 12731), so 25 qubits and float-float only on
+// handles that never specialise.
+static bool keeps_full_forms(const Sim &s, const std::vector<GateDesc> &gates) {
+    if ((s.prec && !ff_capable(s)) || s.n < 25) return false;
+    if ((s.prec || s.n == 25) && s.jit_mode != KBWG_JIT_OFF) return false;
+    size_t any = 0;
+    for (const GateDesc &x : gates)
+        if (!x.ctrl && (x.kind == G_H || x.kind == G_RX || x.kind == G_RY || x.kind == G_RZ)) any++;
+    return 4 * any < gates.size();
+}
+
 // The gate list as the fused sweeps of a handle run it (folded, factors
-// deferred where the state's norm allows); the handle's state is at least one
-// tile.
-static std::vector<GateDesc> rewritten(const Sim &s, const GateDesc *gates, size_t count, bool in_range) {
-    if (s.flags & KBWG_FLAG_EXACT_ORDER) return std::vector<GateDesc>(gates, gates + count);
-    if (!in_range) {
-        const std::vector<GateDesc> f = fold_diagonals(gates, count);
-        return ff_capable(s) ? defer_scale(ARITH_FF, f.data(), f.size(), false) : f;
-    }
+// deferred where the state's norm allows and they pay), and whether its Z and
+// CZ gates are merged; the handle's state is at least one tile.
+struct Rewritten {
+    std::vector<GateDesc> gates;
+    bool merge;
+};
+static Rewritten rewritten(const Sim &s, const GateDesc *gates, size_t count, bool in_range) {
+    if (s.flags & KBWG_FLAG_EXACT_ORDER) return {std::vector<GateDesc>(gates, gates + count), false};
     if (s.flags & KBWG_FLAG_NO_FOLD) {  // every gate applied as given, but for float-float's H and RZ
-        if (ff_capable(s)) return defer_scale(ARITH_FF, gates, count, false);
-        return std::vector<GateDesc>(gates, gates + count);
+        if (ff_capable(s)) return {defer_scale(ARITH_FF, gates, count, false), false};
+        return {std::vector<GateDesc>(gates, gates + count), false};
     }
-    return defer_factors(ff_capable(s) ? ARITH_FF : (s.prec ? ARITH_F64 : ARITH_C64), gates, count);
+    const int arith = ff_capable(s) ? ARITH_FF : (s.prec ? ARITH_F64 : ARITH_C64);
+    const std::vector<GateDesc> f = folded(arith, gates, count);
+    const bool full = keeps_full_forms(s, f);
+    if ((full || !in_range) && arith != ARITH_FF) return {f, !full};
+    return {defer_scale(arith, f.data(), f.size(), !full && in_range), !full};
 }
 
 std::vector<const void *> specialised_kernels(Sim &s, const std::vector<std::string> &srcs, const char *entry,
@@ -835,12 +899,12 @@ cudaError_t init_state(Sim &s) {
 
 // ---- compile-only check of the specialised kernels (no GPU) --------------------
 template <class P, int K, int R>
-static size_t check_p(const Sim &s, const GateDesc *gates, size_t count, size_t &sweeps) {
+static size_t check_p(const Sim &s, const GateDesc *gates, size_t count, bool merge, size_t &sweeps) {
     using SK = SweepKernel<P, K, R>;
     const size_t depth = s.fusion_depth ? s.fusion_depth : (size_t)kMaxSweepGates;
     std::vector<PlannedSweep> plan =
         plan_sweeps(s.n, K, R, gates, count, (s.flags & KBWG_FLAG_EXACT_ORDER) != 0, depth);
-    if (merges(s))
+    if (merge)
         for (PlannedSweep &sw : plan) merge_signs(sw, K, R);
     const JitGeometry geo{PolicyName<P>::s, K, R, SK::kThreads, SK::kCtasPerSm, s.n > 32};
     std::vector<std::string> srcs;
@@ -850,31 +914,32 @@ static size_t check_p(const Sim &s, const GateDesc *gates, size_t count, size_t 
 }
 
 template <class T>
-static size_t check_t(const Sim &s, const GateDesc *gates, size_t count, size_t &sweeps) {
+static size_t check_t(const Sim &s, const GateDesc *gates, size_t count, bool merge, size_t &sweeps) {
     constexpr int K = TileCfg<T>::K, R = TileCfg<T>::R;
-    const uint32_t tk = chosen_tile(s);
+    const uint32_t tk = tile_of_list(s, merge);
     if (tk != (uint32_t)K && !(s.flags & KBWG_FLAG_EXACT_ORDER)) {
         if constexpr (std::is_same<T, float>::value) {
-            if (tk == 12) return check_p<FastP, 12, 4>(s, gates, count, sweeps);
-            if (tk == 11) return check_p<FastP, 11, 3>(s, gates, count, sweeps);
+            if (tk == 12) return check_p<FastP, 12, 4>(s, gates, count, merge, sweeps);
+            if (tk == 11) return check_p<FastP, 11, 3>(s, gates, count, merge, sweeps);
         } else {
-            if (tk == 11) return check_p<Fast<T>, 11, 3>(s, gates, count, sweeps);
+            if (tk == 11) return check_p<Fast<T>, 11, 3>(s, gates, count, merge, sweeps);
         }
     }
     sweeps = 0;
     if (s.n < (uint32_t)K) return 0;
-    if (s.flags & KBWG_FLAG_EXACT_ORDER) return check_p<Exact<T>, K, R>(s, gates, count, sweeps);
-    if constexpr (std::is_same<T, float>::value) return check_p<FastP, K, R>(s, gates, count, sweeps);
-    else return check_p<Fast<T>, K, R>(s, gates, count, sweeps);
+    if (s.flags & KBWG_FLAG_EXACT_ORDER) return check_p<Exact<T>, K, R>(s, gates, count, merge, sweeps);
+    if constexpr (std::is_same<T, float>::value) return check_p<FastP, K, R>(s, gates, count, merge, sweeps);
+    else return check_p<Fast<T>, K, R>(s, gates, count, merge, sweeps);
 }
 
 size_t jit_check(const Sim &s, const GateDesc *gates, size_t count, size_t &sweeps) {
-    const std::vector<GateDesc> g = rewritten(s, gates, count, true);
+    const Rewritten g = rewritten(s, gates, count, true);
     if (ff_capable(s)) {
-        if (chosen_tile(s) == 12) return check_p<FF2, 12, 4>(s, g.data(), g.size(), sweeps);
-        return check_p<FF2, TileCfgFF::K, TileCfgFF::R>(s, g.data(), g.size(), sweeps);
+        if (chosen_tile(s) == 12) return check_p<FF2, 12, 4>(s, g.gates.data(), g.gates.size(), g.merge, sweeps);
+        return check_p<FF2, TileCfgFF::K, TileCfgFF::R>(s, g.gates.data(), g.gates.size(), g.merge, sweeps);
     }
-    return s.prec ? check_t<double>(s, g.data(), g.size(), sweeps) : check_t<float>(s, g.data(), g.size(), sweeps);
+    return s.prec ? check_t<double>(s, g.gates.data(), g.gates.size(), g.merge, sweeps)
+                  : check_t<float>(s, g.gates.data(), g.gates.size(), g.merge, sweeps);
 }
 
 cudaError_t run_fused(Sim &s, const GateDesc *gates, size_t count) {
@@ -885,12 +950,12 @@ cudaError_t run_fused(Sim &s, const GateDesc *gates, size_t count) {
             gates = folded.data();
             count = folded.size();
         }
-        return s.prec ? run_fused_t<double>(s, gates, count) : run_fused_t<float>(s, gates, count);
+        return s.prec ? run_fused_t<double>(s, gates, count, false) : run_fused_t<float>(s, gates, count, false);
     }
     bool in_range = true;
     const cudaError_t er = within_range(s, in_range);
     if (er != cudaSuccess) return er;
-    const std::vector<GateDesc> g = rewritten(s, gates, count, in_range);
+    const Rewritten g = rewritten(s, gates, count, in_range);
     if (ff_capable(s)) {
         // float-float sweeps read and write the float-float form; the state
         // stays in it until an operation needs binary64
@@ -899,11 +964,12 @@ cudaError_t run_fused(Sim &s, const GateDesc *gates, size_t count) {
             if (e != cudaSuccess) return e;
             s.ff_resident = true;
         }
-        if (s.n > 32) return run_fused_p<FF2, TileCfgFF::K, TileCfgFF::R, true>(s, g.data(), g.size());
-        if (chosen_tile(s) == 12) return run_fused_p<FF2, 12, 4>(s, g.data(), g.size());
-        return run_fused_p<FF2, TileCfgFF::K, TileCfgFF::R>(s, g.data(), g.size());
+        if (s.n > 32) return run_fused_p<FF2, TileCfgFF::K, TileCfgFF::R, true>(s, g.gates.data(), g.gates.size(), g.merge);
+        if (chosen_tile(s) == 12) return run_fused_p<FF2, 12, 4>(s, g.gates.data(), g.gates.size(), g.merge);
+        return run_fused_p<FF2, TileCfgFF::K, TileCfgFF::R>(s, g.gates.data(), g.gates.size(), g.merge);
     }
-    return s.prec ? run_fused_t<double>(s, g.data(), g.size()) : run_fused_t<float>(s, g.data(), g.size());
+    return s.prec ? run_fused_t<double>(s, g.gates.data(), g.gates.size(), g.merge)
+                  : run_fused_t<float>(s, g.gates.data(), g.gates.size(), g.merge);
 }
 
 }  // namespace kbwg

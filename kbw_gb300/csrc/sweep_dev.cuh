@@ -154,7 +154,7 @@ struct Exact {
     }
     static __device__ __forceinline__ Amp cmul(Amp a, T c, T s) { return cmul_exact(a, c, s); }
     // |1> * i^q is a float-float gate, the deferred forms never run in program order
-    static constexpr bool kDefer = false;
+    static constexpr bool kDefer = false, kSub = true;
     static __device__ __forceinline__ Amp pi_mul(Amp a, int) { return a; }
     static __device__ __forceinline__ int power_of_i(const K4 &) { return 0; }
     static __device__ __forceinline__ Amp smul(Amp a, T c) { return Amp{xmul(a.re, c), xmul(a.im, c)}; }
@@ -214,7 +214,7 @@ struct Fast : Exact<T> {
     }
     // RX/RY with a deferred factor (pack_rot): one FMA per real part where
     // the full form takes a product and an FMA
-    static constexpr bool kDefer = true;
+    static constexpr bool kDefer = true, kSub = true;
     static __device__ __forceinline__ bool cot(const K4 &k) { return k.c1 != (T)0; }
     template <bool COT>
     static __device__ __forceinline__ void rxd_pair(const K4 &k, Amp &a0, Amp &a1) {
@@ -345,7 +345,7 @@ struct FastP {
         return make_float2(__uint_as_float(__float_as_uint(a.x) ^ s), __uint_as_float(__float_as_uint(a.y) ^ s));
     }
     // RX/RY with a deferred factor (pack_rot): one packed FMA per amplitude
-    static constexpr bool kDefer = true;
+    static constexpr bool kDefer = true, kSub = true;
     static __device__ __forceinline__ bool cot(const K4 &k) { return k.c1 != 0.f; }
     template <bool COT>
     static __device__ __forceinline__ Amp rxd_half(const K4 &k, Amp self, Amp o) {
@@ -380,6 +380,15 @@ struct FastP {
     static __device__ __forceinline__ Amp ryd_half(const K4 &k, Amp self, Amp o, float w) {
         if constexpr (COT) return __ffma2_rn(bc(k.c0), self, __fmul2_rn(bc(w), o));
         return __ffma2_rn(bc(w), o, self);
+    }
+};
+
+// FastP for programs without deferred factors.
+struct FastPPlain : FastP {
+    static constexpr bool kDefer = false, kSub = false;
+    static __device__ __forceinline__ void h_pair(int, const K4 &k, Amp &a0, Amp &a1) { FastP::h_pair(0, k, a0, a1); }
+    static __device__ __forceinline__ Amp h_half(int, const K4 &k, Amp self, Amp o, float sgn) {
+        return FastP::h_half(0, k, self, o, sgn);
     }
 };
 
@@ -479,7 +488,7 @@ struct FFPol {
     static __device__ __forceinline__ Amp cmul(Amp a, ff::f2 c, ff::f2 s) {
         return Amp{ff::dot2(c, a.re, ff::neg(s), a.im), ff::dot2(c, a.im, s, a.re)};
     }
-    static constexpr bool kDefer = false;
+    static constexpr bool kDefer = false, kSub = true;
     static __device__ __forceinline__ int power_of_i(const K4 &k) { return (int)k.c0.h; }
     static __device__ __forceinline__ Amp smul(Amp a, ff::f2 c) { return Amp{ff::mul(a.re, c), ff::mul(a.im, c)}; }
     static __device__ __forceinline__ Amp flip(Amp a, uint32_t s) { return s ? neg(a) : a; }
@@ -579,7 +588,7 @@ struct FF2 {
     }
     // RX/RY with a deferred factor (pack_rot): 15 packed operations per
     // amplitude (ff2::axpy) where the full form's dot product takes 19
-    static constexpr bool kDefer = true;
+    static constexpr bool kDefer = true, kSub = true;
     static __device__ __forceinline__ bool cot(const K4 &k) { return k.c1.h != 0.f; }
     template <bool COT>
     static __device__ __forceinline__ Amp rxd_half(const K4 &k, Amp self, Amp o) {
@@ -762,7 +771,7 @@ __device__ __forceinline__ void diag_fixed(typename P::Amp (&v)[1 << R], const T
         // P: |1> * (c0, c1); SCALE: all * (c0, c1); RZ: (c0, c1) or (c2, c3)
         const auto c = (CLS == TG_RZ && one) ? k.c2 : k.c0;
         const auto s = (CLS == TG_RZ && one) ? k.c3 : k.c1;
-        if (CLS == TG_SCALE && g.sub != 0) {  // real factor
+        if (P::kSub && CLS == TG_SCALE && g.sub != 0) {  // real factor
 #pragma unroll
             for (int j = 0; j < NR; j++) v[j] = P::smul(v[j], c);
             return;
