@@ -326,6 +326,7 @@ __global__ void __launch_bounds__(256, 3) k_apply_tile_f32(const cx<float> *__re
         float ar[NA], ai[NA], rr[NA], ri[NA];
 #pragma unroll
         for (int i = 0; i < NA; i++) ar[i] = ai[i] = rr[i] = ri[i] = 0.f;
+        static_assert(kMaxTerms <= 127, "a byte holds the count of a pass's strings");
         long long count = 0;  // eight signed bytes: signed strings of the run by their mask on the three bits
         for (uint32_t k = 0; k < p.nterms; k++) {  // (branches depend on the string only: uniform)
             const ApplyTileTermFF t = p.t[k];

@@ -89,12 +89,12 @@ struct BatchPass {
 // A string of a pass: flip and phase masks on the tile's local bits, phase
 // mask on the qubits outside it; `last` closes a run of strings with the
 // same flip mask and coefficient (their signs are counted, the coefficient
-// applied once); `newx`: the first string of a flip mask.
+// applied once).
 struct BatchTileTerm {
     uint32_t xl, zl;
     uint64_t zo;
     double cr, ci;
-    uint32_t last, newx;
+    uint32_t last, pad;
 };
 
 struct BatchArgs {
@@ -293,7 +293,7 @@ __global__ void __launch_bounds__(BatchKernel<P, K, R>::kThreads, BatchKernel<P,
     static_assert(sizeof(Amp) == sizeof(Mem), "register and memory amplitudes share the tile buffers");
     constexpr int NR = 1 << R;
     extern __shared__ __align__(128) unsigned char smem_raw[];
-    Amp *tile = reinterpret_cast<Amp *>(smem_raw);  // two tile buffers
+    Amp *tile = reinterpret_cast<Amp *>(smem_raw);  // kBuffers tiles
     Mem *tile_mem = reinterpret_cast<Mem *>(smem_raw);
     unsigned char *q = smem_raw + BK::kBuffers * BK::kTileBytes;
     uint64_t *chunk_off = reinterpret_cast<uint64_t *>(q);
@@ -792,7 +792,6 @@ static int32_t batch_run(int arith, BatchWorkers &workers, std::vector<BatchCirc
                     return x.ci < y.ci;
                 });
                 for (size_t j = 0; j < ts.size(); j++) {
-                    ts[j].newx = (j == 0 || ts[j - 1].xl != ts[j].xl) ? 1u : 0u;
                     const bool end = j + 1 == ts.size() || ts[j + 1].xl != ts[j].xl || ts[j + 1].cr != ts[j].cr ||
                                      ts[j + 1].ci != ts[j].ci;
                     ts[j].last = end ? 1u : 0u;

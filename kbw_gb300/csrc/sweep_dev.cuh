@@ -866,8 +866,8 @@ template <class A, class C> struct pick_t<false, A, C> { using type = C; };
 
 // B: type of the state index (32 bits up to 32 qubits, 64 bits above; not
 // deduced from the argument, so a caller names 64 bits explicitly).  ROT:
-// the program may hold rotations with deferred factors (their bodies cost
-// the adjoint's kernels, which never run them, registers).
+// the program may hold rotations with deferred factors and merged signs (their
+// bodies cost registers where it never does: k_hea_batch, plain sweeps).
 template <class P, int K, int R, class B = uint32_t, bool ROT = P::kDefer>
 __device__ __forceinline__ void tile_gate(const TileGate &g, typename P::Amp (&v)[1 << R], int R0, uint32_t F,
                                           typename ident<B>::type base) {
