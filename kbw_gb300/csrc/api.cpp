@@ -680,7 +680,7 @@ static int32_t exp_strings(kbwg_sim *s, const std::vector<PauliString> &strs, st
     };
     // strings with a flip mask: tiled passes, each covering every string whose
     // flip mask fits one tile (ring TFIM, 30 qubits: 4 passes instead of 30)
-    // (smaller registers: k_pauli_group, in complex128 on binary64 products, as
+    // (smaller registers: k_pauli_small, in complex128 on binary64 products, as
     // few pairs average the tile kernel's 48-bit products out less: 9 qubits, rms
     // error of a string's value 1.9e-17 against 6.0e-16)
     const int K = s->prec ? pauli_tile_bits<double>() : pauli_tile_bits<float>();
@@ -763,6 +763,27 @@ static int32_t exp_strings(kbwg_sim *s, const std::vector<PauliString> &strs, st
     while (i < n_strings) {
         if (by_tile[order[i]]) {  // done by the tiled passes
             i++;
+            continue;
+        }
+        if (!tiled && strs[order[i]].x != 0) {  // (the strings without flips come first)
+            PauliSmall p;
+            memset(&p, 0, sizeof p);
+            const size_t first = i;
+            for (; i < n_strings && i - first < (size_t)kMaxTerms; i++) {
+                const PauliString &t = strs[order[i]];
+                const size_t k = i - first;
+                p.x[k] = t.x;
+                p.z[k] = t.z;
+                pair_term(t, p.factor[k], p.use_im[k]);
+            }
+            p.nterms = (uint32_t)(i - first);
+            ReduceScratch rs = s->rs;
+            rs.result = d_vals + slot_of.size();
+            CUDA_TRY(dispatch(s, [&](auto *tp) {
+                using T = std::remove_pointer_t<decltype(tp)>;
+                return launch_pauli_small<T>(s->state, s->n, p, rs, s->stream);
+            }));
+            slot_of.insert(slot_of.end(), order.begin() + (long)first, order.begin() + (long)i);
             continue;
         }
         PauliGroup g;

@@ -92,6 +92,16 @@ template <class T>
 cudaError_t launch_pauli_group(const void *st, uint32_t n, const PauliGroup &g, const ReduceScratch &rs,
                                cudaStream_t s, bool ff_resident = false);
 
+// Pair-form Pauli strings of any flip masks on a register below one tile.
+struct PauliSmall {
+    uint32_t nterms, pad;
+    uint64_t x[kMaxTerms], z[kMaxTerms];
+    double factor[kMaxTerms];
+    uint32_t use_im[kMaxTerms];
+};
+template <class T>
+cudaError_t launch_pauli_small(const void *st, uint32_t n, const PauliSmall &p, const ReduceScratch &rs, cudaStream_t s);
+
 // Pair-form Pauli strings with different flip masks in one pass: a tile of
 // 2^K amplitudes (local bits 0..l-1 = qubits 0..l-1, l..K-1 = qubits hq[])
 // holds both members of every pair of every string whose flip mask lies in
