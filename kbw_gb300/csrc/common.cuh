@@ -76,7 +76,7 @@ struct GateDesc {
 
 enum { G_X = 0, G_Y = 1, G_Z = 2, G_H = 3, G_P = 4, G_RX = 5, G_RY = 6, G_RZ = 7 };
 // Internal kinds of the reordering paths (never seen at the ABI): H without its
-// 1/sqrt(2), |1> times i^q (c[0] = q), multiply every amplitude by c[0] + i c[1]
+// 1/sqrt(2), |1> times i^q (c[0] = q; see TG_PI), multiply every amplitude by c[0] + i c[1]
 // (G_SCALER: by the real c[0]), RX and RY without the larger of their
 // coefficients (c[0], c[1]: see pack_rot in sweep.h).
 enum { G_HN = 8, G_PI = 9, G_SCALE = 10, G_SCALER = 11, G_RXD = 12, G_RYD = 13 };

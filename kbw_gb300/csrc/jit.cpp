@@ -265,7 +265,7 @@ namespace {
 // The constants expression of gate i (a load of its program entry, or the
 // zero constants for a gate that needs none).
 std::string constants_of(const TileGate &t, size_t i) {
-    const bool needs_k = !(t.cls == TG_X || t.cls == TG_Y || t.cls == TG_Z || t.cls == TG_PI ||
+    const bool needs_k = !(t.cls == TG_X || t.cls == TG_Y || t.cls == TG_Z ||
                            (t.cls == TG_H && t.sub == 1));
     if (!needs_k) return "kz";
     char buf[64];

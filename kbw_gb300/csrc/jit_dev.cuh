@@ -138,7 +138,7 @@ __device__ __forceinline__ void dreg(typename P::Amp (&v)[1 << R], const typenam
         } else if constexpr (CLS == TG_RZ) {
             v[j] = sel(c, hi ? P::cmul(v[j], k.c2, k.c3) : P::cmul(v[j], k.c0, k.c1), v[j]);
         } else {  // TG_PI
-            if (hi) v[j] = sel(c, P::pi_mul(v[j], Q), v[j]);
+            if (hi) v[j] = sel(c, P::pi_mul(v[j], Q, k), v[j]);
         }
     }
 }
@@ -164,7 +164,7 @@ __device__ __forceinline__ void dfix(typename P::Amp (&v)[1 << R], const typenam
             if constexpr (CLS == TG_Z) {
                 v[j] = sel(on, P::neg(v[j]), v[j]);
             } else if constexpr (CLS == TG_PI) {
-                v[j] = sel(on, P::pi_mul(v[j], Q), v[j]);
+                v[j] = sel(on, P::pi_mul(v[j], Q, k), v[j]);
             } else if constexpr (CLS == TG_SCALE && Q != 0) {  // real factor
                 v[j] = P::smul(v[j], k.c0);
             } else {  // P (|1> side only) and SCALE

@@ -651,8 +651,8 @@ static cudaError_t run_fused_t(Sim &s, const GateDesc *gates, size_t count, bool
 // Each H, RX or RY grows the state by at most sqrt(2), so kDeferRun of them
 // stay inside float's range before g is applied (a structural count: the
 // plan must not depend on the angles).  In float-float P(+-pi/2) and P(pi)
-// become exact multiplications by i^q (1e-15 is below its 48 bits; binary64
-// and complex64 keep the phase they are given).
+// become exact multiplications by i^q (1e-15 is below its 48 bits); in binary64
+// a phase whose sine is +-1 drops the two products with it and keeps its cosine.
 // A SCALE costs about two deferred rotations' savings, so lists with fewer
 // than kDeferMin such gates keep the full forms (float-float always drops H's
 // and RZ's factors: its multiplications cost most).
@@ -730,6 +730,12 @@ static std::vector<GateDesc> defer_scale(int arith, const GateDesc *gates, size_
                 x.c[0] = (double)q;
                 x.c[1] = 0.0;
             }
+        }
+        if (x.kind == G_P && arith == ARITH_F64 && fabs(x.c[1]) == 1.0) {
+            const double q = x.c[1] > 0.0 ? 1.0 : 3.0;
+            x.kind = G_PI;
+            x.c[1] = x.c[0];
+            x.c[0] = q;
         }
         out.push_back(x);
         pending = pending || grew;

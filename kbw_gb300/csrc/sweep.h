@@ -42,7 +42,7 @@ enum {
     TG_Z = 5,      // |1> negated (first diagonal class)
     TG_P = 6,      // |1> * (c0 + i c1)
     TG_RZ = 7,     // |0> * (c0 + i c1), |1> * (c2 + i c3)
-    TG_PI = 8,     // |1> * i^q, q = c0
+    TG_PI = 8,     // |1> * i^q, q = c0 (float-float), or (c1 + i s), s = +-1 by q = 1, 3 (binary64)
     TG_SCALE = 9,  // every amplitude * (c0 + i c1), the deferred factors (sub 1: * c0, real)
     TG_SIGN = 10   // many Z and CZ gates at once (SignRow)
 };

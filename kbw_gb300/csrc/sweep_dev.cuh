@@ -153,10 +153,15 @@ struct Exact {
         return Amp{xadd(xmul(k.c0, self.re), xmul(ss, o.re)), xadd(xmul(k.c0, self.im), xmul(ss, o.im))};
     }
     static __device__ __forceinline__ Amp cmul(Amp a, T c, T s) { return cmul_exact(a, c, s); }
-    // |1> * i^q is a float-float gate, the deferred forms never run in program order
+    // |1> * (c + i s) with s = +-1 in binary64 (q 1 or 3; c, a rest below 1.5e-8,
+    // in c1): the products with s need no instruction.  Neither this nor the
+    // deferred forms run in program order.
     static constexpr bool kDefer = false, kSub = true;
-    static __device__ __forceinline__ Amp pi_mul(Amp a, int) { return a; }
-    static __device__ __forceinline__ int power_of_i(const K4 &) { return 0; }
+    static __device__ __forceinline__ int power_of_i(const K4 &k) { return (int)k.c0; }
+    static __device__ __forceinline__ Amp pi_mul(Amp a, int q, const K4 &k) {
+        if (q == 1) return Amp{fma(a.re, k.c1, -a.im), fma(a.im, k.c1, a.re)};
+        return Amp{fma(a.re, k.c1, a.im), fma(a.im, k.c1, -a.re)};
+    }
     static __device__ __forceinline__ Amp smul(Amp a, T c) { return Amp{xmul(a.re, c), xmul(a.im, c)}; }
     // negated where s (a sign bit) is set
     static __device__ __forceinline__ T flip1(T x, uint32_t s) {
@@ -336,9 +341,9 @@ struct FastP {
     static __device__ __forceinline__ Amp cmul(Amp a, float c, float s) {
         return __ffma2_rn(a, bc(c), __fmul2_rn(swp(a), make_float2(-s, s)));
     }
-    // |1> * i^q is a float-float gate (bodies that pick q at run time made the
+    // |1> * i^q is no complex64 gate (bodies that pick q at run time made the
     // interpreted 2^13 kernel spill, 16 -> 112 bytes, up to 25 % slower)
-    static __device__ __forceinline__ Amp pi_mul(Amp a, int) { return a; }
+    static __device__ __forceinline__ Amp pi_mul(Amp a, int, const K4 &) { return a; }
     static __device__ __forceinline__ int power_of_i(const K4 &) { return 0; }
     static __device__ __forceinline__ Amp smul(Amp a, float c) { return mul_rn(a, c); }
     static __device__ __forceinline__ Amp flip(Amp a, uint32_t s) {
@@ -492,7 +497,7 @@ struct FFPol {
     static __device__ __forceinline__ int power_of_i(const K4 &k) { return (int)k.c0.h; }
     static __device__ __forceinline__ Amp smul(Amp a, ff::f2 c) { return Amp{ff::mul(a.re, c), ff::mul(a.im, c)}; }
     static __device__ __forceinline__ Amp flip(Amp a, uint32_t s) { return s ? neg(a) : a; }
-    static __device__ __forceinline__ Amp pi_mul(Amp a, int q) {
+    static __device__ __forceinline__ Amp pi_mul(Amp a, int q, const K4 &) {
         if (q == 1) return Amp{ff::neg(a.im), a.re};
         if (q == 2) return Amp{ff::neg(a.re), ff::neg(a.im)};
         return Amp{a.im, ff::neg(a.re)};
@@ -573,7 +578,7 @@ struct FF2 {
     static __device__ __forceinline__ Amp cmul(Amp a, ff::f2 c, ff::f2 s) {
         return ff2::dot2(ff2::konst(c), a, ff2::konst(ff::neg(s), s), ff2::swap(a));
     }
-    static __device__ __forceinline__ Amp pi_mul(Amp a, int q) {
+    static __device__ __forceinline__ Amp pi_mul(Amp a, int q, const K4 &) {
         if (q == 1) return ff2::mul_i(a);
         if (q == 2) return ff2::neg(a);
         return ff2::mul_minus_i(a);
@@ -744,7 +749,7 @@ __device__ __forceinline__ void diag_reg(typename P::Amp (&v)[1 << R], const Til
             } else if constexpr (CLS == TG_RZ) {
                 v[j] = hi ? P::cmul(v[j], k.c2, k.c3) : P::cmul(v[j], k.c0, k.c1);
             } else {  // TG_PI
-                if (hi) v[j] = P::pi_mul(v[j], P::power_of_i(k));
+                if (hi) v[j] = P::pi_mul(v[j], P::power_of_i(k), k);
             }
         }
     }
@@ -766,7 +771,7 @@ __device__ __forceinline__ void diag_fixed(typename P::Amp (&v)[1 << R], const T
         const int q = P::power_of_i(k);
 #pragma unroll
         for (int j = 0; j < NR; j++)
-            if (KBWG_JM(j)) v[j] = P::pi_mul(v[j], q);
+            if (KBWG_JM(j)) v[j] = P::pi_mul(v[j], q, k);
     } else {
         // P: |1> * (c0, c1); SCALE: all * (c0, c1); RZ: (c0, c1) or (c2, c3)
         const auto c = (CLS == TG_RZ && one) ? k.c2 : k.c0;
