@@ -443,7 +443,7 @@ struct ReSum<cx<float>> {
 // Re<a|b> (FP64-grade) into result[0].  Four pairs in flight per thread; the
 // last block adds the partials with all its threads (one thread read 608 of
 // them in a row: most of a 35 us launch on 17 qubits), and complex64 products
-// stay off the FP64 pipe (24 qubits: 227 us there, 40 us of reads).
+// stay off the FP64 pipe (24 qubits: 227 us there, 68 us so, 40 us of reads).
 template <class Mem>
 __global__ void __launch_bounds__(256) k_inner_re(const Mem *__restrict__ a, const Mem *__restrict__ b, uint64_t ns,
                                                   double *partials, unsigned *ticket, double *result) {

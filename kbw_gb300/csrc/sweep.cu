@@ -657,10 +657,11 @@ static cudaError_t run_fused_t(Sim &s, const GateDesc *gates, size_t count, bool
 // than kDeferMin such gates keep the full forms (float-float always drops H's
 // and RZ's factors: its multiplications cost most).
 // Measured (one GB300, specialised kernels): 25q 8-layer brickwork in binary64
-// 28.6 -> 16.3 ms (FP64-bound: half the products), 28q 20-layer complex64 27.3
-// -> 25.3 ms, 30q float-float 424 -> 395 ms.  Error of a 13q 12-layer
-// brickwork against 80-bit arithmetic: binary64 1.1-1.8e-15 -> 4.9-7.5e-16,
-// float-float 1.4-1.8e-14 -> 1.2-1.4e-14, complex64 6.9-8.6e-7 -> 2.3-2.7e-7.
+// 28.6 -> 17.1 ms (FP64-bound: half the products), 28q 20-layer complex64 27.3
+// -> 25.5 ms, 30q float-float 424 -> 394 ms.  Error of a 13q 12-layer
+// brickwork against 80-bit arithmetic, six seeds: binary64 1.1-1.8e-15 ->
+// 4.1-6.1e-16, float-float 1.3-1.8e-14 -> 1.1-1.4e-14, complex64 6.2-10.1e-7 ->
+// 2.1-2.5e-7.
 // Constants are recomputed in binary64 from the angles, also for complex64
 // (whose program-order constants are rounded like Dense<f32>'s); the deferred
 // factor is that of the coefficient as rounded to the program's type, so
