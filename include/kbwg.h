@@ -282,7 +282,11 @@ int32_t kbwg_clear(kbwg_sim *sim);
 /* Execute queued gates now and wait for the device. */
 int32_t kbwg_flush(kbwg_sim *sim);
 
-/* Raw amplitude access (interleaved re,im in the handle's precision). */
+/* Raw amplitude access (interleaved re,im in the handle's precision).  A state
+ * written through device_ptr should have a norm below 1e9 in complex64 and
+ * float-float handles (gates leave factors of up to 2^96 to a later
+ * multiplication, and a look at the norm before each flush would cost those
+ * who only read there); kbwg_set_state takes any. */
 int32_t kbwg_get_state(kbwg_sim *sim, void *host_dst, uintptr_t bytes);
 int32_t kbwg_set_state(kbwg_sim *sim, const void *host_src, uintptr_t bytes);
 int32_t kbwg_state_info(kbwg_sim *sim, uintptr_t *num_qubits, int32_t *precision,

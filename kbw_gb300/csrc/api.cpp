@@ -1007,10 +1007,7 @@ int32_t kbwg_state_info(kbwg_sim *s, uintptr_t *num_qubits, int32_t *precision, 
     CUDA_TRY(cudaStreamSynchronize(s->stream));
     if (num_qubits) *num_qubits = s->n;
     if (precision) *precision = s->prec;
-    if (device_ptr) {
-        *device_ptr = s->state;
-        s->norm_bound = HUGE_VAL;  // (the caller may write through it)
-    }
+    if (device_ptr) *device_ptr = s->state;
     if (bytes) *bytes = s->ns * s->elem;
     return KBWG_OK;
     GUARD_END

@@ -64,7 +64,7 @@ struct Sim {
     // real part, then of the imaginary part) instead of binary64 while true
     bool ff_resident = false;
     // at most the state's norm as far as it is known: one from |0...0> on,
-    // infinite for amplitudes the caller wrote (see within_range in sweep.cu)
+    // infinite for amplitudes the caller loaded (see within_range in sweep.cu)
     double norm_bound = 1.0;
 
     std::vector<GateDesc> queue;  // gates waiting for the next flush

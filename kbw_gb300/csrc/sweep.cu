@@ -765,7 +765,7 @@ std::vector<GateDesc> defer_factors(int arith, const GateDesc *gates, size_t cou
 
 // Whether the state's norm leaves room for a run of deferred factors (2^96) in
 // float's range: below kNormRoom, as after |0...0> or a loaded state of unit
-// norm.  Where it is not known (amplitudes written by the caller, collapses
+// norm.  Where it is not known (amplitudes loaded by the caller, collapses
 // with factors of the caller's) it is measured, once, before the gates run.
 constexpr double kNormRoom = 1048576.0;
 
